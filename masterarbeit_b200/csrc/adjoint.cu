@@ -39,9 +39,7 @@ __device__ __forceinline__ Q<float> ldq(const float* p, size_t i)
 }
 __device__ __forceinline__ Q<double> ldq(const double* p, size_t i)
 {
-    const double2* a = reinterpret_cast<const double2*>(p) + 2 * i;
-    double2 x = a[0], y = a[1];
-    return q_make<double>(x.x, x.y, y.x, y.y);
+    return ldnc_256(reinterpret_cast<const Vec4d*>(p) + i);
 }
 __device__ __forceinline__ void stq(float* p, size_t i, const Q<float>& q)
 {
@@ -49,9 +47,7 @@ __device__ __forceinline__ void stq(float* p, size_t i, const Q<float>& q)
 }
 __device__ __forceinline__ void stq(double* p, size_t i, const Q<double>& q)
 {
-    double2* a = reinterpret_cast<double2*>(p) + 2 * i;
-    a[0] = make_double2(q.c0, q.c1);
-    a[1] = make_double2(q.c2, q.c3);
+    st_256(reinterpret_cast<Vec4d*>(p) + i, q);
 }
 
 // Atomic accumulation into a link of a gradient field.
@@ -62,7 +58,7 @@ __device__ __forceinline__ void atomic_add_link(const Field<float>& G, int mu, i
 }
 __device__ __forceinline__ void atomic_add_link(const Field<double>& G, int mu, int par, int n, const Q<double>& v)
 {
-    double* a = reinterpret_cast<double*>(G.p[mu] + 2u * (unsigned)(par * G.Vh + (int)((unsigned)n >> 1)));
+    double* a = reinterpret_cast<double*>(G.p[mu] + (unsigned)(par * G.Vh + (int)((unsigned)n >> 1)));
     atomicAdd(a + 0, v.c0);
     atomicAdd(a + 1, v.c1);
     atomicAdd(a + 2, v.c2);

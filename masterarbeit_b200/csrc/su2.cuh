@@ -9,7 +9,7 @@
 // where n = ((t*L1 + x)*L2 + y)*L3 + z is the reference's lexicographic site index
 // (LGT_Code/modules/admin/init.c:741-829) and parity = (t+x+y+z) & 1.  Because L3 is even,
 // the two sites n = 2h and 2h+1 have opposite parity, so h enumerates each parity exactly once.
-// One link is 16 B in FP32 (one float4, one 128-bit load) and 32 B in FP64 (two double2).
+// One link is 16 B in FP32 (one 128-bit access) and 32 B in FP64 (one 256-bit access).
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -326,23 +326,48 @@ struct Field<float> {
     }
 };
 
+// 256-bit accesses to four consecutive doubles at a 32-byte boundary (sm_100).  An FP64 link moves in
+// one instruction whose lanes' bytes are contiguous; as two 128-bit accesses each instruction touched
+// every line of the warp's 1 KB and used half of each sector.  The read-only load is a pure function
+// of its address (the kernels that use it never read what the launch writes); the others order with
+// the memory accesses around them.
+struct __align__(32) Vec4d {
+    double x, y, z, w;
+};
+__device__ __forceinline__ Q<double> ldnc_256(const Vec4d* a)
+{
+    Q<double> q;
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(q.c0), "=d"(q.c1), "=d"(q.c2), "=d"(q.c3) : "l"(a));
+    return q;
+}
+__device__ __forceinline__ Q<double> ldcg_256(const Vec4d* a)
+{
+    Q<double> q;
+    asm volatile("ld.global.cg.v4.f64 {%0, %1, %2, %3}, [%4];"
+                 : "=d"(q.c0), "=d"(q.c1), "=d"(q.c2), "=d"(q.c3)
+                 : "l"(a)
+                 : "memory");
+    return q;
+}
+__device__ __forceinline__ void st_256(Vec4d* a, const Q<double>& q)
+{
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(a), "d"(q.c0), "d"(q.c1), "d"(q.c2), "d"(q.c3)
+                 : "memory");
+}
+
 template <>
 struct Field<double> {
-    using ptr_t = double2*;
-    double2* p[4];   // two double2 per link
+    using ptr_t = Vec4d*;
+    Vec4d* p[4];   // 32-byte aligned: every field starts at an allocation or a whole number of links into one
     int Vh;
     __device__ __forceinline__ Q<double> ld(int mu, int par, int n) const { return ldh(mu, par, (int)((unsigned)n >> 1)); }
     __device__ __forceinline__ Q<double> ldh(int mu, int par, int h) const
     {
-        const double2* a = p[mu] + 2u * (unsigned)(par * Vh + h);
-        double2 x = __ldg(a), y = __ldg(a + 1);
-        return q_make<double>(x.x, x.y, y.x, y.y);
+        return ldnc_256(p[mu] + (unsigned)(par * Vh + h));
     }
     __device__ __forceinline__ void sth(int mu, int par, int h, const Q<double>& q) const
     {
-        double2* a = p[mu] + 2u * (unsigned)(par * Vh + h);
-        a[0] = make_double2(q.c0, q.c1);
-        a[1] = make_double2(q.c2, q.c3);
+        st_256(p[mu] + (unsigned)(par * Vh + h), q);
     }
 };
 
@@ -367,9 +392,7 @@ struct FieldCG<double> : Field<double> {
     __device__ __forceinline__ Q<double> ld(int mu, int par, int n) const { return ldh(mu, par, (int)((unsigned)n >> 1)); }
     __device__ __forceinline__ Q<double> ldh(int mu, int par, int h) const
     {
-        const double2* a = p[mu] + 2u * (unsigned)(par * Vh + h);
-        double2 x = __ldcg(a), y = __ldcg(a + 1);
-        return q_make<double>(x.x, x.y, y.x, y.y);
+        return ldcg_256(p[mu] + (unsigned)(par * Vh + h));
     }
 };
 
