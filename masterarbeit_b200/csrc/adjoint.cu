@@ -12,8 +12,9 @@
 //
 // Passes.
 //  1. Forward with sqrt(N) checkpointing: U_0 and every c-th level are kept (c = ckpt or ceil(sqrt N)).
-//  2. G_N = dQ/dU_N: F-bar per site and plane (k_qgrad_fbar), then every link of every clover leaf
-//     receives prefix^dag F-bar suffix^dag (k_qgrad_scatter, atomic adds).
+//  2. G_N = dQ/dU_N: the charge kernel leaves F-bar = dQ/dF per site and plane; the gradient with
+//     respect to every 1-, 2- and 3-link line is gathered from the loops it is an edge of
+//     (k_line_gradient), and a link's from the lines it is part of (k_line_chain).
 //  3. Per segment, recompute its levels from the checkpoint; per level, backwards:
 //     v-bar = (G_{k+1} - u' <u', G_{k+1}>) / |v|, the Jacobian of u' = v/|v| (k_ape_vbar), then
 //     G_k = v-bar + alpha * (the 18 staple terms in which a link appears) (k_ape_gather).
@@ -22,166 +23,132 @@
 #include <vector>
 
 #include "ape.cuh"
-#include "clover.cuh"
 #include "internal.cuh"
 
 using namespace su2g;
 
 namespace {
 
-constexpr double kPi = 3.14159265358979323846;
-
-// Plain quaternion arrays (F-bar per plane and site).
-__device__ __forceinline__ Q<float> ldq(const float* p, size_t i)
-{
-    float4 v = reinterpret_cast<const float4*>(p)[i];
-    return q_make<float>(v.x, v.y, v.z, v.w);
-}
-__device__ __forceinline__ Q<double> ldq(const double* p, size_t i)
-{
-    return ldnc_256(reinterpret_cast<const Vec4d*>(p) + i);
-}
-__device__ __forceinline__ void stq(float* p, size_t i, const Q<float>& q)
-{
-    reinterpret_cast<float4*>(p)[i] = make_float4(q.c0, q.c1, q.c2, q.c3);
-}
-__device__ __forceinline__ void stq(double* p, size_t i, const Q<double>& q)
-{
-    st_256(reinterpret_cast<Vec4d*>(p) + i, q);
-}
-
-// Atomic accumulation into a link of a gradient field.
-__device__ __forceinline__ void atomic_add_link(const Field<float>& G, int mu, int par, int n, const Q<float>& v)
-{
-    // one 16-byte vector atomic per link
-    atomicAdd(G.p[mu] + (unsigned)(par * G.Vh + (int)((unsigned)n >> 1)), make_float4(v.c0, v.c1, v.c2, v.c3));
-}
-__device__ __forceinline__ void atomic_add_link(const Field<double>& G, int mu, int par, int n, const Q<double>& v)
-{
-    double* a = reinterpret_cast<double*>(G.p[mu] + (unsigned)(par * G.Vh + (int)((unsigned)n >> 1)));
-    atomicAdd(a + 0, v.c0);
-    atomicAdd(a + 1, v.c1);
-    atomicAdd(a + 2, v.c2);
-    atomicAdd(a + 3, v.c3);
-}
-
 // ----------------------------------------------------------- dQ / dU_N ---
 
-// Planes in the order of the charge's three products: (01)(23), (02)(31), (03)(12).
-__host__ __device__ constexpr int plane_a(int p) { return p == 0 ? 0 : p == 1 ? 2 : p == 2 ? 0 : p == 3 ? 3 : p == 4 ? 0 : 1; }
-__host__ __device__ constexpr int plane_b(int p) { return p == 0 ? 1 : p == 1 ? 3 : p == 2 ? 2 : p == 3 ? 1 : p == 4 ? 3 : 2; }
-
-// F-bar(x, plane) = dQ/dF(x, plane).  With F pure, c0(F_a F_b) = -<F_a, F_b>, and
-// q = 16 sum_pairs c0(F_a F_b)  =>  dQ/dF_a = -16 s F_b, dQ/dF_b = -16 s F_a, s = 1/(32 pi^2).
+// r + a b for a pure quaternion a (a.c0 is not read), and for a pure b.
 template <typename R>
-__global__ void __launch_bounds__(kBlock) k_qgrad_fbar(Field<R> U, Geom g, R* __restrict__ fbar, R scale)
+__device__ __forceinline__ Q<R> q_pure_mul_add(const Q<R>& r, const Q<R>& a, const Q<R>& b)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= g.V) return;
-    int par;
-    const Site s = site_lex(g, i, par);
-    const size_t V = (size_t)g.V, n = (size_t)s.n;
-    Q<R> f0 = clover_F<R, 0, 1>(U, g, s, par), f1 = clover_F<R, 2, 3>(U, g, s, par);
-    stq(fbar, 0 * V + n, q_scale(f1, -scale));
-    stq(fbar, 1 * V + n, q_scale(f0, -scale));
-    f0 = clover_F<R, 0, 2>(U, g, s, par);
-    f1 = clover_F<R, 3, 1>(U, g, s, par);
-    stq(fbar, 2 * V + n, q_scale(f1, -scale));
-    stq(fbar, 3 * V + n, q_scale(f0, -scale));
-    f0 = clover_F<R, 0, 3>(U, g, s, par);
-    f1 = clover_F<R, 1, 2>(U, g, s, par);
-    stq(fbar, 4 * V + n, q_scale(f1, -scale));
-    stq(fbar, 5 * V + n, q_scale(f0, -scale));
+    return q_make<R>(r.c0 - a.c1 * b.c1 - a.c2 * b.c2 - a.c3 * b.c3, r.c1 + a.c1 * b.c0 - a.c2 * b.c3 + a.c3 * b.c2,
+                     r.c2 + a.c1 * b.c3 + a.c2 * b.c0 - a.c3 * b.c1, r.c3 - a.c1 * b.c2 + a.c2 * b.c1 + a.c3 * b.c0);
+}
+template <typename R>
+__device__ __forceinline__ Q<R> q_mul_pure_add(const Q<R>& r, const Q<R>& a, const Q<R>& b)
+{
+    return q_make<R>(r.c0 - a.c1 * b.c1 - a.c2 * b.c2 - a.c3 * b.c3, r.c1 + a.c0 * b.c1 - a.c2 * b.c3 + a.c3 * b.c2,
+                     r.c2 + a.c0 * b.c2 + a.c1 * b.c3 - a.c3 * b.c1, r.c3 + a.c0 * b.c3 - a.c1 * b.c2 + a.c2 * b.c1);
 }
 
-// Leaf step tables: leaf l, segment k -> (direction A or B, sign); the four leaves of
-// computeCloverAverages (topologicalcharge.c:70-100): +A+B-A-B, -B+A+B-A, +B-A-B+A, -A-B+A+B.
-__host__ __device__ constexpr bool leaf_on_a(int l, int k)
+// The plane of directions (d, v) among clover_plane's six, and whether d is its first direction.
+__host__ __device__ constexpr int plane_of(int d, int v)
 {
-    return (l == 0 || l == 3) ? (k == 0 || k == 2) : (k == 1 || k == 3);
+    for (int p = 0; p < 6; ++p)
+        if ((clover_plane_a(p) == d && clover_plane_b(p) == v) || (clover_plane_a(p) == v && clover_plane_b(p) == d)) return p;
+    return -1;
 }
-__host__ __device__ constexpr int leaf_sign(int l, int k)
-{
-    return l == 0 ? (k < 2 ? 1 : -1) : l == 1 ? (k == 0 || k == 3 ? -1 : 1) : l == 2 ? (k == 0 || k == 3 ? 1 : -1)
-                                                                                    : (k < 2 ? -1 : 1);
-}
+__host__ __device__ constexpr bool plane_first(int d, int v) { return clover_plane_a(plane_of(d, v)) == d; }
 
-// For one leaf (an E x E loop from x) with adjoint Gbar: every link P_i of the ordered product
-// L = P_0 ... P_{M-1} gets  (P_0..P_{i-1})^dag Gbar (P_{i+1}..P_{M-1})^dag, daggered when P_i = U^dag.
-template <typename R, int A, int B, int E, int LEAF>
-__device__ __forceinline__ void leaf_adjoint(const Field<R>& U, const Field<R>& G, const Geom& g, const Site& s,
-                                             int par, const Q<R>& Gbar)
+// Gradient of Q with respect to the e-link line L = L^e_D(x), all lines independent.  L is an edge of
+// the e x e loop above it in each plane (D, v) and of the one below, and each loop enters F at its four
+// corners.  With F-bar = dQ/dF (pure) and the path x -> x+v -> x+v+D -> x+D of lines B, A, B' (each e
+// links) around the loop above, those four terms are the path with F-bar inserted at each corner:
+//   F(x) M + M F(x+D) + B [F(x+v) A + A F(x+v+D)] B'^dag,  M = B A B'^dag;
+// the loop below runs the other way round and enters with the opposite sign, as does every loop of a
+// plane whose first direction is v.
+template <typename R, int D>
+__device__ __forceinline__ Q<R> line_gradient(const Field<R>& L, const R* __restrict__ fbar, const Geom& g,
+                                              const Site& s, int par, int h, int e)
 {
-    constexpr int M = 4 * E;
-    Q<R> pre[M];
-    int pos[M];
-    int n = s.n, ca = s.c[A], cb = s.c[B], p = par;
-    Q<R> acc = q_one<R>();
+    const int q1 = par ^ (e & 1);   // parity one segment away
+    const int upD = shift_by(g, D, s.c[D], e);
+    const auto F = [&](int p, int pr, int n) {
+        return ldq(fbar, (size_t)p * g.V + (unsigned)(pr * g.Vh + (int)((unsigned)n >> 1)));
+    };
+    Q<R> acc = q_zero<R>();
 #pragma unroll
-    for (int i = 0; i < M; ++i) {
-        const int k = i / E;
-        const bool on_a = leaf_on_a(LEAF, k);
-        const int D = on_a ? A : B;
-        int& c = on_a ? ca : cb;
-        if (leaf_sign(LEAF, k) > 0) {
-            pos[i] = n;
-            acc = q_mul(acc, U.ld(D, p, n));
-            if (c == g.L[D] - 1) { n -= (g.L[D] - 1) * g.S[D]; c = 0; }
-            else { n += g.S[D]; ++c; }
-        } else {
-            if (c == 0) { n += (g.L[D] - 1) * g.S[D]; c = g.L[D] - 1; }
-            else { n -= g.S[D]; --c; }
-            pos[i] = n;
-            acc = q_mul_nd(acc, U.ld(D, p ^ 1, n));
-        }
-        p ^= 1;
-        pre[i] = acc;
+    for (int v = 0; v < 4; ++v) {
+        if (v == D) continue;
+        const int p = plane_of(D, v);
+        const int up = s.n + shift_by(g, v, s.c[v], e), dn = s.n + shift_by(g, v, s.c[v], -e);
+        const Q<R> A = L.ld(D, q1, up), B = L.ldh(v, par, h), B2 = L.ld(v, q1, s.n + upD);
+        Q<R> m = q_pure_mul_add(q_zero<R>(), F(p, q1, up), A);
+        m = q_mul_pure_add(m, A, F(p, par, up + upD));
+        Q<R> M = q_mul_nd(q_mul(B, A), B2), N = q_mul_nd(q_mul(B, m), B2);
+        const Q<R> a = L.ld(D, q1, dn), b = L.ld(v, q1, dn), b2 = L.ld(v, par, dn + upD);
+        m = q_pure_mul_add(q_zero<R>(), F(p, q1, dn), a);
+        m = q_mul_pure_add(m, a, F(p, par, dn + upD));
+        M = q_sub(M, q_mul(q_mul_dn(b, a), b2));
+        N = q_sub(N, q_mul(q_mul_dn(b, m), b2));
+        N = q_pure_mul_add(N, F(p, par, s.n), M);
+        N = q_mul_pure_add(N, M, F(p, q1, s.n + upD));
+        acc = plane_first(D, v) ? q_add(acc, N) : q_sub(acc, N);
     }
-    Q<R> S = q_one<R>();
+    return acc;
+}
+
+// Line gradients T_e of all sites, directions D and sizes e, one per thread: CTA b takes (D, e) number
+// b mod 12 of site block b / 12 (parities paired per warp), so that the twelve share their loads in L2.
+// A gather: every result is written once, no atomics, and the sums run in a fixed order.  It replaced a
+// walk over every leaf that added each link's term with an atomic (1728 products and 576 atomics a site;
+// here 36 line gradients of about 15 products and 36 loads each): a whole VJP of five steps without the
+// gradient's copy at 24^4 on B200 1580 -> 825 us (FP32) and 5290 -> 1510 us (FP64), at 8^4 605 -> 200 us
+// (FP64).  Two to five CTAs per SM asked for in FP64 and four to eight in FP32 measured the same within
+// 3 %, so the compiler's own register count stands.
+constexpr int kLineBlock = 128;
+
+template <typename R>
+__global__ void __launch_bounds__(kLineBlock) k_line_gradient(Field<R> U, Field<R> L2, Field<R> L3, Field<R> T1, Field<R> T2,
+                                                              Field<R> T3, Geom g, const R* __restrict__ fbar)
+{
+    const int job = blockIdx.x % 12, D = job & 3, e = 1 + (job >> 2);
+    Site s;
+    int par, h;
+    if (!site_warp_pair(g, blockIdx.x / 12, threadIdx.x, blockDim.x, s, par, h)) return;
+    Field<R> L, T;
+    L.Vh = T.Vh = g.Vh;
 #pragma unroll
-    for (int i = M - 1; i >= 0; --i) {
-        const int k = i / E;
-        const int D = leaf_on_a(LEAF, k) ? A : B;
-        const bool fwd = leaf_sign(LEAF, k) > 0;
-        // parity of the link's site: the walk's parity before a forward step, after a backward one
-        const int lp = par ^ ((fwd ? i : i + 1) & 1);
-        const Q<R> link = U.ld(D, lp, pos[i]);
-        const Q<R> left = i > 0 ? pre[i > 0 ? i - 1 : 0] : q_one<R>();
-        const Q<R> gi = q_mul_nd(q_mul_dn(left, Gbar), S);
-        if (fwd) {
-            atomic_add_link(G, D, lp, pos[i], gi);
-            S = q_mul(link, S);
-        } else {
-            atomic_add_link(G, D, lp, pos[i], q_dag(gi));
-            S = q_mul_dn(link, S);
-        }
+    for (int d = 0; d < 4; ++d) {
+        L.p[d] = e == 1 ? U.p[d] : (e == 2 ? L2.p[d] : L3.p[d]);
+        T.p[d] = e == 1 ? T1.p[d] : (e == 2 ? T2.p[d] : T3.p[d]);
+    }
+    const R k4 = e == 1 ? R(1.5 * 0.25) : (e == 2 ? R(-0.15 * 0.25) : R(0.25 / 90.0));
+    switch (D) {
+        case 0: T.sth(0, par, h, q_scale(line_gradient<R, 0>(L, fbar, g, s, par, h, e), k4)); break;
+        case 1: T.sth(1, par, h, q_scale(line_gradient<R, 1>(L, fbar, g, s, par, h, e), k4)); break;
+        case 2: T.sth(2, par, h, q_scale(line_gradient<R, 2>(L, fbar, g, s, par, h, e), k4)); break;
+        default: T.sth(3, par, h, q_scale(line_gradient<R, 3>(L, fbar, g, s, par, h, e), k4)); break;
     }
 }
 
-template <typename R, int A, int B, int E>
-__device__ __forceinline__ void clover_adjoint_e(const Field<R>& U, const Field<R>& G, const Geom& g, const Site& s,
-                                                 int par, const Q<R>& Fbar)
+// dQ/dU_D(x) from the line gradients: U = U_D(x) is the first link of its lines at x, the second of
+// those at x - D and the third of L^3 at x - 2D,
+//   T1(x) + [T2(x) + U(x-D)^dag T3(x-D)] U(x+D)^dag + U(x-D)^dag T2(x-D)
+//   + T3(x) L2(x+D)^dag + L2(x-2D)^dag T3(x-2D).
+template <typename R>
+__global__ void __launch_bounds__(kBlock) k_line_chain(Field<R> U, Field<R> L2, Field<R> T1, Field<R> T2, Field<R> T3,
+                                                       Field<R> G, Geom g)
 {
-    const R kcoef = E == 1 ? R(1.5) : E == 2 ? R(-0.15) : R(1.0 / 90.0);
-    const Q<R> Gbar = q_scale(Fbar, kcoef * R(0.25));
-    leaf_adjoint<R, A, B, E, 0>(U, G, g, s, par, Gbar);
-    leaf_adjoint<R, A, B, E, 1>(U, G, g, s, par, Gbar);
-    leaf_adjoint<R, A, B, E, 2>(U, G, g, s, par, Gbar);
-    leaf_adjoint<R, A, B, E, 3>(U, G, g, s, par, Gbar);
-}
-
-template <typename R, int PLANE>
-__global__ void __launch_bounds__(kBlock) k_qgrad_scatter(Field<R> U, Field<R> G, Geom g, const R* __restrict__ fbar)
-{
-    constexpr int A = plane_a(PLANE), B = plane_b(PLANE);
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= g.V) return;
-    int par;
-    const Site s = site_lex(g, i, par);
-    const Q<R> Fbar = ldq(fbar, (size_t)PLANE * g.V + (size_t)s.n);
-    clover_adjoint_e<R, A, B, 1>(U, G, g, s, par, Fbar);
-    clover_adjoint_e<R, A, B, 2>(U, G, g, s, par, Fbar);
-    clover_adjoint_e<R, A, B, 3>(U, G, g, s, par, Fbar);
+    Site s;
+    int par, h;
+    if (!site_warp_pair(g, blockIdx.x, threadIdx.x, blockDim.x, s, par, h)) return;
+    const int q = par ^ 1;
+#pragma unroll
+    for (int D = 0; D < 4; ++D) {
+        const int up = s.n + up_off_rt(g, s.c, D), dn = s.n + dn_off_rt(g, s.c, D), dn2 = s.n + shift_by(g, D, s.c[D], -2);
+        const Q<R> um = U.ld(D, q, dn);
+        Q<R> a = T1.ldh(D, par, h);
+        a = q_mul_nd_add(a, q_mul_dn_add(T2.ldh(D, par, h), um, T3.ld(D, q, dn)), U.ld(D, q, up));
+        a = q_mul_dn_add(a, um, T2.ld(D, q, dn));
+        a = q_mul_nd_add(a, T3.ldh(D, par, h), L2.ld(D, q, up));
+        a = q_mul_dn_add(a, L2.ld(D, par, dn2), T3.ld(D, par, dn2));
+        G.sth(D, par, h, a);
+    }
 }
 
 // ------------------------------------------------------ one APE step back ---
@@ -372,21 +339,19 @@ int vjp_t(su2g_lattice* h, int n_ape, double alpha, int c, double* q_out, double
         if ((rc = ape_step(h, cur, dst, SU2G_APE_ALL, alpha))) return rc;
         cur = dst;
     }
-    if ((rc = ensure_lines(h)) || (rc = qtop_enqueue(h, cur, 0))) return rc;
-    // G_N = dQ/dU_N
-    const R scale = R(16.0 / (32.0 * kPi * kPi));
-    Field<R> UN = make_field<R>(cur, g.Vh);
-    Field<R> Gc = make_field<R>(G[0].dirs, g.Vh);
-    if ((rc = check_cuda(h, cudaMemsetAsync(G[0].base, 0, 4 * dir_bytes, h->stream), "clearing the gradient")))
-        return rc;
+    // Q, and F-bar = dQ/dF as it goes
+    if ((rc = ensure_lines(h)) || (rc = qtop_enqueue(h, cur, 0, fbar))) return rc;
+    // G_N = dQ/dU_N; the line gradients go into fields that are free until the smearing is reversed:
+    // v-bar's, the other gradient's and the forward scratch that does not hold U_N
+    void *l2[4], *l3[4];
+    line_dirs(h, l2, l3);
+    const Field<R> UN = make_field<R>(cur, g.Vh), L2 = make_field<R>(l2, g.Vh), L3 = make_field<R>(l3, g.Vh);
+    const Field<R> T1 = make_field<R>(Vb.dirs, g.Vh), T2 = make_field<R>(G[1].dirs, g.Vh),
+                   T3 = make_field<R>(tmp[n_ape & 1].dirs, g.Vh);
+    const int lblocks = (int)((g.V + kLineBlock - 1) / kLineBlock);
     launch_begin(h, SU2G_K_OTHER);
-    k_qgrad_fbar<R><<<grid, kBlock, 0, h->stream>>>(UN, g, fbar, scale);
-    k_qgrad_scatter<R, 0><<<grid, kBlock, 0, h->stream>>>(UN, Gc, g, fbar);
-    k_qgrad_scatter<R, 1><<<grid, kBlock, 0, h->stream>>>(UN, Gc, g, fbar);
-    k_qgrad_scatter<R, 2><<<grid, kBlock, 0, h->stream>>>(UN, Gc, g, fbar);
-    k_qgrad_scatter<R, 3><<<grid, kBlock, 0, h->stream>>>(UN, Gc, g, fbar);
-    k_qgrad_scatter<R, 4><<<grid, kBlock, 0, h->stream>>>(UN, Gc, g, fbar);
-    k_qgrad_scatter<R, 5><<<grid, kBlock, 0, h->stream>>>(UN, Gc, g, fbar);
+    k_line_gradient<R><<<12 * lblocks, kLineBlock, 0, h->stream>>>(UN, L2, L3, T1, T2, T3, g, fbar);
+    k_line_chain<R><<<grid, kBlock, 0, h->stream>>>(UN, L2, T1, T2, T3, make_field<R>(G[0].dirs, g.Vh), g);
     if ((rc = launch_end(h, SU2G_K_OTHER, "charge adjoint kernels"))) return rc;
     // backwards through the smearing, one checkpoint segment at a time
     int gi = 0;

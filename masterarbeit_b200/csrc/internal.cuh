@@ -204,8 +204,14 @@ int ape_tma_rows(const Geom& g, int max_smem);
 int ape_tma_launch(su2g_lattice* h, void* const in_dirs[4], void* const out_dirs[4], double alpha, int yb);
 // Scratch of the charge kernel (two fields of line products); allocate before any capture.
 int ensure_lines(su2g_lattice* h);
+// The directions' bases of the 2- and 3-link lines in it.
+void line_dirs(const su2g_lattice* h, void* l2[4], void* l3[4]);
 // Enqueue Q of the field at dirs (ensure_lines first); Q and sum|q| land in d_out[out_off], d_out[out_off + 1].
-int qtop_enqueue(su2g_lattice* h, void* const dirs[4], int out_off);
+// With fbar (6V quaternions) the kernel also leaves dQ/dF there, element plane V + parity Vh + h; the
+// lines of dirs stay in the scratch either way.
+int qtop_enqueue(su2g_lattice* h, void* const dirs[4], int out_off, void* fbar = nullptr);
+// Entries of the partial-sum scratch it uses (ensure_partial_entries before any capture).
+size_t qtop_partial_entries(const su2g_lattice* h);
 // FP64 AoS staging (the reference's pu layout) and the conversions of sites [n0, n0 + count)
 // between a device AoS buffer and the handle's field.
 int ensure_aos(su2g_lattice* h);

@@ -177,7 +177,7 @@ extern "C" int su2g_measure(su2g_lattice* h, const su2g_meas_spec* sp, double* q
         // everything the graph uses is allocated before the capture starts
         if ((rc = ensure_work(h))) return rc;
         if ((rc = ensure_partials(h, 8 * 32))) return rc;
-        if ((rc = ensure_partial_entries(h, 2 * (size_t)((h->g.V + kBlock - 1) / kBlock)))) return rc;
+        if (sp->n_q > 0 && (rc = ensure_partial_entries(h, qtop_partial_entries(h)))) return rc;
         if (sp->n_q > 0 && (rc = ensure_lines(h))) return rc;
         if ((rc = capture(h, sp))) return rc;
     }

@@ -12,7 +12,6 @@
 #include <cmath>
 
 #include "internal.cuh"
-#include "clover.cuh"
 #include "ape.cuh"
 
 using namespace su2g;
@@ -395,87 +394,99 @@ __global__ void __launch_bounds__(kBlock) k_lines(Field<R> U, Field<R> L2, Field
     }
 }
 
-// Offset of the lexicographic index for k steps (|k| <= 3) along direction d from coordinate c.
-__device__ __forceinline__ int shift_by(const Geom& g, int d, int c, int k)
-{
-    const int L = g.L[d];
-    int cc = c + k;
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {   // |k| <= 3 <= 2 L - 1 for L >= 2: two wraps at most
-        cc += cc < 0 ? L : 0;
-        cc -= cc >= L ? L : 0;
-    }
-    return (cc - c) * g.S[d];
-}
-
-// Improved clover field strength in plane (A, B) at site s from line products (the same
+// Improved clover field strengths of the planes P0 and P0 + 1 at site s, from line products:
 // F = [(k1 C1 + k2 C2 + k3 C3) - h.c.]/2, C_e = (1/4) sum of the four e x e leaves, (k1, k2, k3) =
-// (1.5, -0.15, 1/90), as clover_F in clover.cuh; topologicalcharge.c:46-162).  With a = eA, b = eB
-// and L the e-link lines of the two directions, the leaves starting and ending at x are
-//   +A +B -A -B:  LA(x) LB(x+a) LA(x+b)^dag LB(x)^dag
-//   -B +A +B -A:  LB(x-b)^dag LA(x-b) LB(x+a-b) LA(x)^dag
-//   +B -A -B +A:  LB(x) LA(x-a+b)^dag LB(x-a)^dag LA(x-a)
-//   -A -B +A +B:  LA(x-a)^dag LB(x-a-b)^dag LA(x-a-b) LB(x-b)
-// : twelve loads and twelve products per size.
-template <typename R, int A, int B>
-__device__ __forceinline__ Q<R> clover_F_lines(const Field<R>& U, const Field<R>& L2, const Field<R>& L3,
-                                               const Geom& g, const Site& s, int par)
+// (1.5, -0.15, 1/90)  (topologicalcharge.c:46-162).  With a = eA, b = eB and L the e-link lines of
+// the two directions, the leaves starting and ending at x are
+//   l0 = +A +B -A -B:  LA(x) LB(x+a) LA(x+b)^dag LB(x)^dag
+//   l1 = -B +A +B -A:  LB(x-b)^dag LA(x-b) LB(x+a-b) LA(x)^dag
+//   l2 = +B -A -B +A:  LB(x) LA(x-a+b)^dag LB(x-a)^dag LA(x-a)
+//   l3 = -A -B +A +B:  LA(x-a)^dag LB(x-a-b)^dag LA(x-a-b) LB(x-b).
+// Only the su(2) part of their sum enters, and a loop run backwards has the opposite one, so l2 and
+// l3 are taken backwards and share their last factor with l0 and l1:
+//   l0 + l2 -> [LA(x) LB(x+a) LA(x+b)^dag - LA(x-a)^dag LB(x-a) LA(x-a+b)] LB(x)^dag
+//   l1 + l3 -> LB(x-b)^dag [LA(x-b) LB(x+a-b) LA(x)^dag - LA(x-a-b)^dag LB(x-a-b) LA(x-a)]
+// : ten products per plane and size, two of them without their scalar component, instead of twelve.
+// The two planes share the sizes' loop and its periodic offsets (24 a call instead of 12 a plane).
+template <typename R, int P0>
+__device__ __forceinline__ void clover_F_lines(const Field<R>& U, const Field<R>& L2, const Field<R>& L3, const Geom& g,
+                                               const Site& s, int par, int h, Q<R> (&F)[2])
 {
-    Q<R> F = q_zero<R>();
+#pragma unroll
+    for (int p = 0; p < 2; ++p) F[p] = q_zero<R>();
 #pragma unroll 1
     for (int e = 1; e <= 3; ++e) {
-        // the two directions' e-link lines (pointers selected in registers, not a field by reference)
+        // the directions' e-link lines (pointers selected in registers, not a field by reference)
         Field<R> L;
         L.Vh = U.Vh;
-        L.p[A] = e == 1 ? U.p[A] : (e == 2 ? L2.p[A] : L3.p[A]);
-        L.p[B] = e == 1 ? U.p[B] : (e == 2 ? L2.p[B] : L3.p[B]);
-        const R kcoef = e == 1 ? R(1.5) : (e == 2 ? R(-0.15) : R(1.0 / 90.0));
-        const int pa = A, pb = B;
-        const int oa = shift_by(g, pa, s.c[pa], e), ma = shift_by(g, pa, s.c[pa], -e);
-        const int ob = shift_by(g, pb, s.c[pb], e), mb = shift_by(g, pb, s.c[pb], -e);
+        int up[4], dn[4];
+#pragma unroll
+        for (int d = 0; d < 4; ++d) {
+            L.p[d] = e == 1 ? U.p[d] : (e == 2 ? L2.p[d] : L3.p[d]);
+            up[d] = shift_by(g, d, s.c[d], e);
+            dn[d] = shift_by(g, d, s.c[d], -e);
+        }
+        const R k4 = e == 1 ? R(1.5 * 0.25) : (e == 2 ? R(-0.15 * 0.25) : R(0.25 / 90.0));
         const int q1 = par ^ (e & 1);   // parity one segment away
         const int n = s.n;
-        const Q<R> LAx = L.ld(A, par, n), LBx = L.ld(B, par, n);
-        const Q<R> LBxa = L.ld(B, q1, n + oa), LAxb = L.ld(A, q1, n + ob);
-        const Q<R> LBxmb = L.ld(B, q1, n + mb), LAxmb = L.ld(A, q1, n + mb);
-        const Q<R> LBxamb = L.ld(B, par, n + oa + mb), LAxmab = L.ld(A, par, n + ma + ob);
-        const Q<R> LBxma = L.ld(B, q1, n + ma), LAxma = L.ld(A, q1, n + ma);
-        const Q<R> LBxmamb = L.ld(B, par, n + ma + mb), LAxmamb = L.ld(A, par, n + ma + mb);
-        const Q<R> l0 = q_mul_nd(q_mul_nd(q_mul(LAx, LBxa), LAxb), LBx);
-        const Q<R> l1 = q_mul_nd(q_mul(q_mul_dn(LBxmb, LAxmb), LBxamb), LAx);
-        const Q<R> l2 = q_mul(q_mul_nd(q_mul_nd(LBx, LAxmab), LBxma), LAxma);
-        const Q<R> l3 = q_mul(q_mul(q_dag(q_mul(LBxmamb, LAxma)), LAxmamb), LBxmb);
-        F = q_axpy(kcoef * R(0.25), q_add(q_add(l0, l1), q_add(l2, l3)), F);
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+            const int A = clover_plane_a(P0 + p), B = clover_plane_b(P0 + p);
+            const Q<R> LAx = L.ldh(A, par, h), LBxmb = L.ld(B, q1, n + dn[B]), LAxma = L.ld(A, q1, n + dn[A]);
+            const Q<R> k0 = q_mul_nd(q_mul(LAx, L.ld(B, q1, n + up[A])), L.ld(A, q1, n + up[B]));
+            const Q<R> k2 = q_mul(q_mul_dn(LAxma, L.ld(B, q1, n + dn[A])), L.ld(A, par, n + dn[A] + up[B]));
+            const Q<R> k1 = q_mul_nd(q_mul(L.ld(A, q1, n + dn[B]), L.ld(B, par, n + up[A] + dn[B])), LAx);
+            const Q<R> k3 = q_mul(q_mul_dn(L.ld(A, par, n + dn[A] + dn[B]), L.ld(B, par, n + dn[A] + dn[B])), LAxma);
+            const Q<R> t = q_mul_dn_add(q_mul_nd(q_sub(k0, k2), L.ldh(B, par, h)), LBxmb, q_sub(k1, k3));
+            F[p] = q_axpy(k4, t, F[p]);
+        }
     }
-    F.c0 = R(0);   // (F - F^dag)/2 keeps the su(2) part
-    return F;
+#pragma unroll
+    for (int p = 0; p < 2; ++p) F[p].c0 = R(0);   // (F - F^dag)/2 keeps the su(2) part
 }
 
-// q(x) = 8 [tr F01 F23 + tr F02 F31 + tr F03 F12], tr = 2 c0 (topologicalcharge.c:175-178)
-template <typename R>
-__device__ __forceinline__ double qtop_density(const Field<R>& U, const Field<R>& L2, const Field<R>& L3,
-                                               const Geom& g, const Site& s, int par)
+// q(x) = 8 [tr F01 F23 + tr F02 F31 + tr F03 F12], tr = 2 c0 (topologicalcharge.c:175-178): the
+// product of the planes P0 and P0 + 1.  With FBAR the site's dQ/dF = -(16 / 32 pi^2) x (the other plane's F)
+// of both planes go to fbar, element
+// plane V + parity Vh + h (c0(F_a F_b) = -<F_a, F_b> for pure F).
+template <typename R, int P0, bool FBAR>
+__device__ __forceinline__ double qtop_product(const Field<R>& U, const Field<R>& L2, const Field<R>& L3, const Geom& g,
+                                               const Site& s, int par, int h, R* __restrict__ fbar)
 {
-    double d = 0.0;
-    d += 16.0 * (double)q_mul(clover_F_lines<R, 0, 1>(U, L2, L3, g, s, par), clover_F_lines<R, 2, 3>(U, L2, L3, g, s, par)).c0;
-    d += 16.0 * (double)q_mul(clover_F_lines<R, 0, 2>(U, L2, L3, g, s, par), clover_F_lines<R, 3, 1>(U, L2, L3, g, s, par)).c0;
-    d += 16.0 * (double)q_mul(clover_F_lines<R, 0, 3>(U, L2, L3, g, s, par), clover_F_lines<R, 1, 2>(U, L2, L3, g, s, par)).c0;
-    return d;
+    Q<R> F[2];
+    clover_F_lines<R, P0>(U, L2, L3, g, s, par, h, F);
+    if (FBAR) {
+        constexpr R scale = R(-16.0 / (32.0 * kPi * kPi));
+        const size_t i = (size_t)P0 * g.V + (unsigned)(par * g.Vh + h);
+        stq(fbar, i, q_scale(F[1], scale));
+        stq(fbar, i + g.V, q_scale(F[0], scale));
+    }
+    return 16.0 * (double)q_mul(F[0], F[1]).c0;
 }
 
-// One site per thread; CTA partials of q and |q| at partials[b] and partials[gridDim.x + b].
-// Resident CTAs per SM: three in FP32 and two in FP64.
-template <typename R>
-__global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 3 : 2) k_qtop(Field<R> U, Field<R> L2, Field<R> L3, Geom g,
-                                                                        DD* __restrict__ partials)
+// One site per thread, parities paired per warp (site_warp_pair); CTA partials of q and |q| at
+// partials[b] and partials[gridDim.x + b].  FMA-bound: 2736 multiply-adds a site, 0.39 ms (FP32) and
+// 1.53 ms (FP64) at 48^4 on B200.  128-thread CTAs, five per SM in FP32 (96 registers) and three in FP64
+// (168).  Measured, a whole Q at 24^4 / 48^4 with k_lines: FP32 104 us / 1.19 ms (six CTAs 105 / 1.24,
+// seven 114 / 1.26, three of 256 threads 109 / 1.26; the twelve-product form with offsets per plane
+// 118 / 1.40), FP64 167 us / 2.2-2.4 ms (four CTAs 169 / 2.4, five 183 / 2.7).  Slower: all six planes in one
+// pass over the sizes (179 us, 2.7 ms FP64: spills), three warps a site, one per product (190 us FP64).
+constexpr int kQtopBlock = 128;
+
+template <typename R, bool FBAR>
+__global__ void __launch_bounds__(kQtopBlock, sizeof(R) == 4 ? 5 : 3) k_qtop(Field<R> U, Field<R> L2, Field<R> L3, Geom g,
+                                                                            DD* __restrict__ partials, R* __restrict__ fbar)
 {
-    // parities paired per warp (site_warp_pair); grid ceil(V / kBlock)
     Site s;
     int par, h;
     double d = 0.0;
-    if (site_warp_pair(g, blockIdx.x, threadIdx.x, blockDim.x, s, par, h)) d = qtop_density<R>(U, L2, L3, g, s, par);
-    DD acc = dd_block_sum_d<kBlock>(d);
-    DD aabs = dd_block_sum_d<kBlock>(fabs(d));
+    if (site_warp_pair(g, blockIdx.x, threadIdx.x, kQtopBlock, s, par, h)) {
+        d += qtop_product<R, 0, FBAR>(U, L2, L3, g, s, par, h, fbar);
+        d += qtop_product<R, 2, FBAR>(U, L2, L3, g, s, par, h, fbar);
+        d += qtop_product<R, 4, FBAR>(U, L2, L3, g, s, par, h, fbar);
+    }
+    DD acc = dd_block_sum_d<kQtopBlock>(d);
+    DD aabs = dd_block_sum_d<kQtopBlock>(fabs(d));
     if (threadIdx.x == 0) {
         partials[blockIdx.x] = acc;
         partials[gridDim.x + blockIdx.x] = aabs;
@@ -627,31 +638,38 @@ int su2g::ensure_lines(su2g_lattice* h)
     return SU2G_OK;
 }
 
-int su2g::qtop_enqueue(su2g_lattice* h, void* const dirs[4], int out_off)
+static int qtop_grid(const su2g_lattice* h) { return (int)((h->g.V + kQtopBlock - 1) / kQtopBlock); }
+
+size_t su2g::qtop_partial_entries(const su2g_lattice* h) { return 2 * (size_t)qtop_grid(h); }
+
+void su2g::line_dirs(const su2g_lattice* h, void* l2[4], void* l3[4])
 {
-    if (!h->lines) return set_error(h, SU2G_EINVAL, "topological charge: line scratch not allocated");
-    const int grid = (int)((h->g.V + kBlock - 1) / kBlock);
-    int rc0 = ensure_partial_entries(h, 2ull * grid);
-    if (rc0) return rc0;
-    void* l2[4];
-    void* l3[4];
     for (int mu = 0; mu < 4; ++mu) {
         l2[mu] = (char*)h->lines + (size_t)mu * h->g.V * h->link_bytes;
         l3[mu] = (char*)h->lines + (size_t)(4 + mu) * h->g.V * h->link_bytes;
     }
-    const int lgrid = 2 * (int)((h->g.Vh + kBlock - 1) / kBlock);
+}
+
+template <typename R>
+static void launch_qtop(su2g_lattice* h, void* const dirs[4], int grid, void* fbar)
+{
+    void *l2[4], *l3[4];
+    line_dirs(h, l2, l3);
+    const Field<R> U = make_field<R>(dirs, h->g.Vh), L2 = make_field<R>(l2, h->g.Vh), L3 = make_field<R>(l3, h->g.Vh);
+    k_lines<R><<<2 * (int)((h->g.Vh + kBlock - 1) / kBlock), kBlock, 0, h->stream>>>(U, L2, L3, h->g);
+    if (fbar) k_qtop<R, true><<<grid, kQtopBlock, 0, h->stream>>>(U, L2, L3, h->g, h->partials, (R*)fbar);
+    else k_qtop<R, false><<<grid, kQtopBlock, 0, h->stream>>>(U, L2, L3, h->g, h->partials, nullptr);
+}
+
+int su2g::qtop_enqueue(su2g_lattice* h, void* const dirs[4], int out_off, void* fbar)
+{
+    if (!h->lines) return set_error(h, SU2G_EINVAL, "topological charge: line scratch not allocated");
+    const int grid = qtop_grid(h);
+    int rc0 = ensure_partial_entries(h, qtop_partial_entries(h));
+    if (rc0) return rc0;
     launch_begin(h, SU2G_K_QTOP);
-    if (h->prec == SU2G_FP32) {
-        const Field<float> U = make_field<float>(dirs, h->g.Vh), L2 = make_field<float>(l2, h->g.Vh),
-                           L3 = make_field<float>(l3, h->g.Vh);
-        k_lines<float><<<lgrid, kBlock, 0, h->stream>>>(U, L2, L3, h->g);
-        k_qtop<float><<<grid, kBlock, 0, h->stream>>>(U, L2, L3, h->g, h->partials);
-    } else {
-        const Field<double> U = make_field<double>(dirs, h->g.Vh), L2 = make_field<double>(l2, h->g.Vh),
-                            L3 = make_field<double>(l3, h->g.Vh);
-        k_lines<double><<<lgrid, kBlock, 0, h->stream>>>(U, L2, L3, h->g);
-        k_qtop<double><<<grid, kBlock, 0, h->stream>>>(U, L2, L3, h->g, h->partials);
-    }
+    if (h->prec == SU2G_FP32) launch_qtop<float>(h, dirs, grid, fbar);
+    else launch_qtop<double>(h, dirs, grid, fbar);
     int rc = launch_end(h, SU2G_K_QTOP, "topological charge kernel");
     // Q = sum_x q(x) / (32 pi^2)  (topologicalcharge.c:194)
     if (!rc) rc = finalize(h, grid, 2, 1.0 / (32.0 * kPi * kPi), out_off, grid);

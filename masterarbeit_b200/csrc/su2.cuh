@@ -299,6 +299,24 @@ __device__ __forceinline__ int dn_off_rt(const Geom& g, const int c[4], int mu)
     return c[mu] == 0 ? (g.L[mu] - 1) * g.S[mu] : -g.S[mu];
 }
 
+// Offset of the lexicographic index for k steps (|k| <= 3) along direction d from coordinate c.
+__device__ __forceinline__ int shift_by(const Geom& g, int d, int c, int k)
+{
+    const int L = g.L[d];
+    int cc = c + k;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {   // |k| <= 3 <= 2 L - 1 for L >= 2: two wraps at most
+        cc += cc < 0 ? L : 0;
+        cc -= cc >= L ? L : 0;
+    }
+    return (cc - c) * g.S[d];
+}
+
+// Planes of the clover field strength in the order of the charge's three products: (01)(23), (02)(31),
+// (03)(12).
+__host__ __device__ constexpr int clover_plane_a(int p) { return p == 0 ? 0 : p == 1 ? 2 : p == 2 ? 0 : p == 3 ? 3 : p == 4 ? 0 : 1; }
+__host__ __device__ constexpr int clover_plane_b(int p) { return p == 0 ? 1 : p == 1 ? 3 : p == 2 ? 2 : p == 3 ? 1 : p == 4 ? 3 : 2; }
+
 // ------------------------------------------------------------------ fields ---
 
 // View of one link field on the device: one base pointer per direction, so that a smearing
@@ -395,6 +413,25 @@ struct FieldCG<double> : Field<double> {
         return ldcg_256(p[mu] + (unsigned)(par * Vh + h));
     }
 };
+
+// Plain quaternion arrays (32-byte aligned in FP64).
+__device__ __forceinline__ Q<float> ldq(const float* p, size_t i)
+{
+    float4 v = reinterpret_cast<const float4*>(p)[i];
+    return q_make<float>(v.x, v.y, v.z, v.w);
+}
+__device__ __forceinline__ Q<double> ldq(const double* p, size_t i)
+{
+    return ldnc_256(reinterpret_cast<const Vec4d*>(p) + i);
+}
+__device__ __forceinline__ void stq(float* p, size_t i, const Q<float>& q)
+{
+    reinterpret_cast<float4*>(p)[i] = make_float4(q.c0, q.c1, q.c2, q.c3);
+}
+__device__ __forceinline__ void stq(double* p, size_t i, const Q<double>& q)
+{
+    st_256(reinterpret_cast<Vec4d*>(p) + i, q);
+}
 
 // Field view over four direction base pointers (each 2*Vh links long).
 template <typename R>
