@@ -24,9 +24,8 @@ __host__ __device__ constexpr bool ape_staple(int mode, int mu, int nu)
 // also the dagger of the middle product of the forward staple of nu in plane mu, so each plane's
 // P is formed once.  emit(mu, u_mu, S_mu) is called for each updated link as soon as its sum is
 // complete (the caller stores or differentiates it; one link's state at a time stays live).
-template <typename R, int MODE, typename Emit>
-__device__ __forceinline__ void ape_staples(const Field<R>& in, const Geom& g, const Site& s, int par, int h,
-                                            Emit&& emit)
+template <typename R, int MODE, typename F, typename Emit>
+__device__ __forceinline__ void ape_staples(const F& in, const Geom& g, const Site& s, int par, int h, Emit&& emit)
 {
     const int q = par ^ 1;
     int xp[4], xm[4];

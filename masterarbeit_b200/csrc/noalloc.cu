@@ -15,6 +15,7 @@
 // different host threads without ordering) race on it and must not be issued.
 #include <mutex>
 
+#include "ape.cuh"
 #include "internal.cuh"
 
 using namespace su2g;
@@ -53,59 +54,82 @@ int scratch_address(int dev, void** out)
     return SU2G_OK;
 }
 
-// A link of the reference's host layout double[V][4][4] (site, direction, c0..c3) on the device.
-__device__ __forceinline__ Q<double> aos_ld(const double2* f, int n, int mu)
-{
-    const double2* a = f + 2 * ((size_t)n * 4 + mu);
-    double2 x = a[0], y = a[1];
-    return q_make<double>(x.x, x.y, y.x, y.y);
-}
-
-__device__ __forceinline__ void aos_st(double2* f, int n, int mu, const Q<double>& q)
-{
-    double2* a = f + 2 * ((size_t)n * 4 + mu);
-    a[0] = make_double2(q.c0, q.c1);
-    a[1] = make_double2(q.c2, q.c3);
-}
-
-__device__ __forceinline__ bool updates(int mode, int mu)
-{
-    return mode == SU2G_APE_ALL ? true : (mode == SU2G_APE_SPATIAL ? mu != 0 : mu == 0);
-}
-
-// One Jacobi step from `src` into `dst` (both AoS FP64): the links of the smeared directions
-// become Proj(U + alpha S) with the staples of smearing.c:42-71; the other directions are copied,
-// so that `dst` is complete whatever the scratch held before.
-__global__ void __launch_bounds__(kBlock) k_ape_aos(const double2* __restrict__ src, double2* __restrict__ dst,
-                                                    Geom g, int mode, double alpha)
-{
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= g.V) return;
-    uint32_t t = fdiv((uint32_t)n, g.dS0);
-    uint32_t r = (uint32_t)n - t * (uint32_t)g.S[0];
-    uint32_t x = fdiv(r, g.dS1);
-    r -= x * (uint32_t)g.S[1];
-    uint32_t y = fdiv(r, g.dS2);
-    uint32_t z = r - y * (uint32_t)g.S[2];
-    const int c[4] = {(int)t, (int)x, (int)y, (int)z};
-    for (int mu = 0; mu < 4; ++mu) {
-        const Q<double> u = aos_ld(src, n, mu);
-        if (!updates(mode, mu)) {
-            aos_st(dst, n, mu, u);
-            continue;
+// A field in the reference's host layout double[V][4][4] (site, direction, c0..c3) on the device, seen
+// like a Field<double>.  A link is 32 bytes: one 256-bit access where the field starts at a 32-byte
+// boundary, two 128-bit ones where the caller's pointer is only 16-byte aligned.
+template <bool A32>
+struct AosField {
+    double2* p;
+    int Vh;
+    __device__ __forceinline__ Q<double> ld(int mu, int, int n) const
+    {
+        const double2* a = p + 2 * ((size_t)n * 4 + mu);
+        if (A32) return ldnc_256(reinterpret_cast<const Vec4d*>(a));
+        const double2 x = __ldg(a), y = __ldg(a + 1);
+        return q_make<double>(x.x, x.y, y.x, y.y);
+    }
+    __device__ __forceinline__ void st(int mu, int n, const Q<double>& q) const
+    {
+        double2* a = p + 2 * ((size_t)n * 4 + mu);
+        if (A32) {
+            st_256(reinterpret_cast<Vec4d*>(a), q);
+        } else {
+            a[0] = make_double2(q.c0, q.c1);
+            a[1] = make_double2(q.c2, q.c3);
         }
-        const int np = n + up_off_rt(g, c, mu);
-        Q<double> S = q_zero<double>();
-        for (int nu = 0; nu < 4; ++nu) {
-            if (nu == mu || (mode != SU2G_APE_ALL && nu == 0)) continue;
-            const int nn = n + up_off_rt(g, c, nu);
-            const int nm = n + dn_off_rt(g, c, nu);
-            // U_nu(x) U_mu(x+nu) U_nu(x+mu)^dag
-            S = q_add(S, q_mul_nd(q_mul(aos_ld(src, n, nu), aos_ld(src, nn, mu)), aos_ld(src, np, nu)));
-            // U_nu(x-nu)^dag U_mu(x-nu) U_nu(x-nu+mu)
-            S = q_add(S, q_mul(q_mul_dn(aos_ld(src, nm, nu), aos_ld(src, nm, mu)), aos_ld(src, nm + (np - n), nu)));
-        }
-        aos_st(dst, n, mu, q_project(q_axpy(alpha, S, u)));
+    }
+};
+
+template <bool A32>
+__device__ __forceinline__ void put(const AosField<A32>& f, int mu, int, int, int n, const Q<double>& q) { f.st(mu, n, q); }
+__device__ __forceinline__ void put(const Field<double>& f, int mu, int par, int h, int, const Q<double>& q)
+{
+    f.sth(mu, par, h, q);
+}
+
+// Own link of a site (ape_staples asks for it by half-volume index, which an AosField does not use).
+template <typename F>
+struct AtSite {
+    F f;
+    int n;
+    __device__ __forceinline__ Q<double> ld(int mu, int par, int m) const { return f.ld(mu, par, m); }
+    __device__ __forceinline__ Q<double> ldh(int mu, int par, int) const { return f.ld(mu, par, n); }
+};
+
+// One Jacobi step from `in` into `out`: the links of the smeared directions become Proj(U + alpha S)
+// with the staples of smearing.c:42-71; with COPY the other directions are copied.  One site per thread, parities paired per warp as in the handle's kernel,
+// whose staple sums these are.
+template <int MODE, bool COPY, typename In, typename Out>
+__global__ void __launch_bounds__(128) k_ape_any(In in, Out out, Geom g, double alpha)
+{
+    Site s;
+    int par, h;
+    if (!site_warp_pair(g, blockIdx.x, threadIdx.x, blockDim.x, s, par, h)) return;
+    const AtSite<In> at{in, s.n};
+#pragma unroll
+    for (int mu = 0; mu < 4; ++mu)
+        if (COPY && !ape_updates(MODE, mu)) put(out, mu, par, h, s.n, in.ld(mu, par, s.n));
+    ape_staples<double, MODE>(at, g, s, par, h, [&](int mu, const Q<double>& u, const Q<double>& S) {
+        put(out, mu, par, h, s.n, q_project(q_axpy(alpha, S, u)));
+    });
+}
+
+// Checkerboarded field with its smeared directions in one buffer and the others in another.
+Field<double> checkerboard(void* base, void* fixed, const Geom& g, int mode)
+{
+    void* dirs[4];
+    for (int mu = 0; mu < 4; ++mu) dirs[mu] = (char*)(ape_updates(mode, mu) ? base : fixed) + (size_t)mu * g.V * 32;
+    return make_field<double>(dirs, g.Vh);
+}
+
+template <bool COPY, typename In, typename Out>
+void step(const In& in, const Out& out, const Geom& g, int mode, double alpha, cudaStream_t st)
+{
+    const int grid = (g.V + 127) / 128;
+    switch (mode) {
+        case SU2G_APE_ALL: k_ape_any<SU2G_APE_ALL, COPY><<<grid, 128, 0, st>>>(in, out, g, alpha); break;
+        case SU2G_APE_SPATIAL: k_ape_any<SU2G_APE_SPATIAL, COPY><<<grid, 128, 0, st>>>(in, out, g, alpha); break;
+        default: k_ape_any<SU2G_APE_TEMPORAL, COPY><<<grid, 128, 0, st>>>(in, out, g, alpha); break;
     }
 }
 
@@ -166,17 +190,32 @@ extern "C" int su2g_ape_inplace_noalloc(double* links, const int32_t dims[4], in
 
     const Geom g = make_geom(dims);
     cudaStream_t st = (cudaStream_t)cuda_stream;
-    const int grid = (int)((V + kBlock - 1) / kBlock);
-    double2* field = reinterpret_cast<double2*>(links);
-    double2* tmp = reinterpret_cast<double2*>(scratch);
-    for (int step = 0; step < ns; ++step) {
-        const double2* src = (step & 1) ? tmp : field;
-        double2* dst = (step & 1) ? field : tmp;
-        k_ape_aos<<<grid, kBlock, 0, st>>>(src, dst, g, mode, alpha);
+    // Levels alternate between the caller's field and the scratch.  The first is read, and the last
+    // written, in the caller's layout; those between are kept in the handle's checkerboarded layout,
+    // whose loads are contiguous over a warp (the site-major one touches a line per lane), and only in
+    // the directions the mode changes: the others stay where the first step copied them, in the
+    // scratch -- or, for a last step that reads the field and writes over the scratch, where the second
+    // step copied them again.  Twenty spatial steps at 20x16x18x14 on B200: 173 us, against 819 us
+    // with every level site-major, one direction after another and no shared products.  A field that is
+    // not 32-byte aligned keeps its own layout throughout.
+    const bool a32 = ((uintptr_t)links & 31u) == 0;
+    void* const base[2] = {links, scratch};
+    for (int i = 0; i < ns; ++i) {
+        void *src = base[i & 1], *dst = base[(i & 1) ^ 1];
+        const bool first = i == 0, last = i + 1 == ns, again = i == 1 && (ns & 1);
+        const AosField<true> asrc{(double2*)src, g.Vh}, adst{(double2*)dst, g.Vh};
+        const Field<double> csrc = checkerboard(src, last && (ns & 1) ? src : scratch, g, mode),
+                            cdst = checkerboard(dst, dst, g, mode);
+        if (!a32) step<true>(AosField<false>{(double2*)src, g.Vh}, AosField<false>{(double2*)dst, g.Vh}, g, mode, alpha, st);
+        else if (first && last) step<true>(asrc, adst, g, mode, alpha, st);
+        else if (first) step<true>(asrc, cdst, g, mode, alpha, st);
+        else if (last) step<true>(csrc, adst, g, mode, alpha, st);
+        else if (again) step<true>(csrc, cdst, g, mode, alpha, st);
+        else step<false>(csrc, cdst, g, mode, alpha, st);
     }
     if (ns & 1) {   // the last level is in the scratch: copy it back into the caller's field
         const long long n2 = V * 8;
-        k_copy_aos<<<(int)((n2 + kBlock - 1) / kBlock), kBlock, 0, st>>>(tmp, field, n2);
+        k_copy_aos<<<(int)((n2 + kBlock - 1) / kBlock), kBlock, 0, st>>>((const double2*)scratch, (double2*)links, n2);
     }
     e = cudaGetLastError();
     if (e != cudaSuccess)
