@@ -31,7 +31,7 @@ namespace {
 
 struct Replica {
     Geom g;
-    double beta;
+    double beta, kb;   // kb: kp_beta of the batch's precision
     uint64_t seed;
     uint32_t id;
     int start;
@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(256, 4) k_batch_update(const Replica* __restri
     if (KIND == SU2G_HEATBATH) {
         Q<R> out;
         uint32_t trials = 0;
-        if (heatbath_link<R>(A, (R)rp.beta, rp.seed, (uint32_t)s.n, ctr[kCtrSweep] + sub, (uint32_t)MU, rp.id, trials,
+        if (heatbath_link<R>(A, (R)rp.kb, rp.seed, (uint32_t)s.n, ctr[kCtrSweep] + sub, (uint32_t)MU, rp.id, trials,
                              out, status))
             U.sth(MU, par, h, hb_store(out));
     } else {
@@ -329,7 +329,7 @@ __device__ __forceinline__ void persist_pass(const PersistArgs& a, const int* __
         if (KIND == SU2G_HEATBATH) {
             Q<R> out;
             uint32_t trials = 0;
-            if (heatbath_link<R>(A, (R)rp.beta, rp.seed, (uint32_t)s.n, sweep, (uint32_t)MU, rp.id, trials, out,
+            if (heatbath_link<R>(A, (R)rp.kb, rp.seed, (uint32_t)s.n, sweep, (uint32_t)MU, rp.id, trials, out,
                                  a.status))
                 U.sth(MU, par, h, hb_store(out));
         } else {
@@ -651,6 +651,7 @@ extern "C" int su2g_batch_create(const su2g_replica* reps, int32_t n, int32_t pr
         Replica rp;
         rp.g = make_geom(reps[r].dims);
         rp.beta = reps[r].beta;
+        rp.kb = precision == SU2G_FP32 ? rp.beta : kp_beta<double>(rp.beta);
         rp.seed = reps[r].seed;
         rp.id = reps[r].replica;
         rp.start = reps[r].start;

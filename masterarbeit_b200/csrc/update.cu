@@ -40,7 +40,7 @@ constexpr int update_block() { return 128; }
 // staple_update (U A = the sum of the plaquettes through U); the separate plaquette kernel
 // (plaquette.c:67-100) then need not run.
 template <typename R, int MU, int KIND, bool PLQ = false>
-__global__ void __launch_bounds__(update_block<KIND>(), 1024 / update_block<KIND>()) k_update(Field<R> U, Geom g, int par, R beta, PhiloxKeys seed, uint32_t sweep,
+__global__ void __launch_bounds__(update_block<KIND>(), 1024 / update_block<KIND>()) k_update(Field<R> U, Geom g, int par, R kb, PhiloxKeys seed, uint32_t sweep,
                                                    const uint32_t* __restrict__ sweep_base, uint32_t replica,
                                                    double* __restrict__ acc_sum, unsigned* __restrict__ status,
                                                    DD* __restrict__ plaq_part = nullptr)
@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(update_block<KIND>(), 1024 / update_block<KIND
             if (sweep_base) sweep += *sweep_base;
             Q<R> out;
             uint32_t trials = 0;
-            if (heatbath_link<R>(A, beta, seed, (uint32_t)s.n, sweep, (uint32_t)MU, replica, trials, out, status))
+            if (heatbath_link<R>(A, kb, seed, (uint32_t)s.n, sweep, (uint32_t)MU, replica, trials, out, status))
                 U.sth(MU, par, h, hb_store(out));
             if (acc_sum && trials) acc_thread = 1.0 / (double)trials;
         } else {
@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(update_block<KIND>(), 1024 / update_block<KIND
 //    count for the site's four links), heatbath or Metropolis once per visit.
 // The acceptance sum counts 1/trials per heatbath visit and accepted/hits per Metropolis visit.
 struct VisitArgs {
-    double beta, eps;
+    double beta, kb, eps;   // kb: kp_beta of the handle's precision
     int hits;
     double p0;   // (1 - 1/V)^V
     uint64_t seed;
@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_visit(Field<R> U, Geom g, int par
                 bool changed = false;
                 for (int v = 0; v < visits; ++v) {
                     uint32_t trials = 0;
-                    if (heatbath_link<R>(A, (R)a.beta, a.seed, (uint32_t)s.n, a.sweep, (uint32_t)MU, a.replica, trials,
+                    if (heatbath_link<R>(A, (R)a.kb, a.seed, (uint32_t)s.n, a.sweep, (uint32_t)MU, a.replica, trials,
                                          out, status, (uint32_t)v << kVisitShift)) {
                         cur = out;
                         changed = true;
@@ -171,23 +171,23 @@ void launch_update_t(su2g_lattice* h, int mu, int par, uint32_t sweep, const uin
                      DD* plaq_part)
 {
     Field<R> U = make_field<R>(h->dirp, h->g.Vh);
-    const R beta = (R)h->beta;
+    const R kb = kp_beta<R>(h->beta);
     const int nt = update_block<KIND>();
     cudaStream_t st = h->stream;
     const PhiloxKeys keys = philox_keys(h->seed);
     if (plaq_part) {   // parity-1 passes of MU >= 1 only
         switch (mu) {
-            case 1: k_update<R, 1, KIND, true><<<grid, nt, 0, st>>>(U, h->g, par, beta, keys, sweep, base, h->replica, acc_sum, h->d_status, plaq_part); break;
-            case 2: k_update<R, 2, KIND, true><<<grid, nt, 0, st>>>(U, h->g, par, beta, keys, sweep, base, h->replica, acc_sum, h->d_status, plaq_part); break;
-            default: k_update<R, 3, KIND, true><<<grid, nt, 0, st>>>(U, h->g, par, beta, keys, sweep, base, h->replica, acc_sum, h->d_status, plaq_part); break;
+            case 1: k_update<R, 1, KIND, true><<<grid, nt, 0, st>>>(U, h->g, par, kb, keys, sweep, base, h->replica, acc_sum, h->d_status, plaq_part); break;
+            case 2: k_update<R, 2, KIND, true><<<grid, nt, 0, st>>>(U, h->g, par, kb, keys, sweep, base, h->replica, acc_sum, h->d_status, plaq_part); break;
+            default: k_update<R, 3, KIND, true><<<grid, nt, 0, st>>>(U, h->g, par, kb, keys, sweep, base, h->replica, acc_sum, h->d_status, plaq_part); break;
         }
         return;
     }
     switch (mu) {
-        case 0: k_update<R, 0, KIND><<<grid, nt, 0, st>>>(U, h->g, par, beta, keys, sweep, base, h->replica, acc_sum, h->d_status); break;
-        case 1: k_update<R, 1, KIND><<<grid, nt, 0, st>>>(U, h->g, par, beta, keys, sweep, base, h->replica, acc_sum, h->d_status); break;
-        case 2: k_update<R, 2, KIND><<<grid, nt, 0, st>>>(U, h->g, par, beta, keys, sweep, base, h->replica, acc_sum, h->d_status); break;
-        default: k_update<R, 3, KIND><<<grid, nt, 0, st>>>(U, h->g, par, beta, keys, sweep, base, h->replica, acc_sum, h->d_status); break;
+        case 0: k_update<R, 0, KIND><<<grid, nt, 0, st>>>(U, h->g, par, kb, keys, sweep, base, h->replica, acc_sum, h->d_status); break;
+        case 1: k_update<R, 1, KIND><<<grid, nt, 0, st>>>(U, h->g, par, kb, keys, sweep, base, h->replica, acc_sum, h->d_status); break;
+        case 2: k_update<R, 2, KIND><<<grid, nt, 0, st>>>(U, h->g, par, kb, keys, sweep, base, h->replica, acc_sum, h->d_status); break;
+        default: k_update<R, 3, KIND><<<grid, nt, 0, st>>>(U, h->g, par, kb, keys, sweep, base, h->replica, acc_sum, h->d_status); break;
     }
 }
 
@@ -232,7 +232,7 @@ namespace {
 // the FP32 histogram exercises the FP32 sampler's fast logarithm, sine/cosine, approximate square
 // roots and delta clamp.  Draw i uses the Philox stream of site i (sweep i >> 32, direction 0).
 template <typename R>
-__global__ void __launch_bounds__(kBlock) k_kp_histogram(double alpha, uint64_t seed, long long n, int nbins,
+__global__ void __launch_bounds__(kBlock) k_kp_histogram(double kb, uint64_t seed, long long n, int nbins,
                                                          unsigned long long* __restrict__ counts,
                                                          unsigned* __restrict__ status)
 {
@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(kBlock) k_kp_histogram(double alpha, uint64_t 
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         Q<R> X;
         uint32_t trials = 0;
-        if (!heatbath_link<R>(A, (R)alpha, seed, (uint32_t)i, (uint32_t)(i >> 32), 0u, 0u, trials, X, status))
+        if (!heatbath_link<R>(A, (R)kb, seed, (uint32_t)i, (uint32_t)(i >> 32), 0u, 0u, trials, X, status))
             continue;   // trial bound hit: the status word tells the host
         int b = (int)(((double)X.c0 + 1.0) * 0.5 * nbins);   // bin of x0 on [-1, 1]
         b = b < 0 ? 0 : (b >= nbins ? nbins - 1 : b);
@@ -356,6 +356,7 @@ extern "C" int su2g_gauge_update(su2g_lattice* h, int32_t nup, int32_t utype, in
     }
     VisitArgs a;
     a.beta = h->beta;
+    a.kb = h->prec == SU2G_FP32 ? h->beta : kp_beta<double>(h->beta);
     a.eps = eps;
     a.hits = utype == 0 ? hits : 1;
     a.p0 = std::exp((double)h->g.V * std::log1p(-1.0 / (double)h->g.V));
@@ -399,10 +400,10 @@ extern "C" int su2g_kp_histogram(su2g_lattice* h, double alpha, uint64_t seed, i
         const int grid = grid_for(h, n, 8);
         launch_begin(h, SU2G_K_OTHER);
         if (h->prec == SU2G_FP32)
-            k_kp_histogram<float><<<grid, kBlock, nbins * sizeof(unsigned int), h->stream>>>(alpha, seed, n, nbins,
+            k_kp_histogram<float><<<grid, kBlock, nbins * sizeof(unsigned int), h->stream>>>(kp_beta<float>(alpha), seed, n, nbins,
                                                                                             d_counts, h->d_status);
         else
-            k_kp_histogram<double><<<grid, kBlock, nbins * sizeof(unsigned int), h->stream>>>(alpha, seed, n, nbins,
+            k_kp_histogram<double><<<grid, kBlock, nbins * sizeof(unsigned int), h->stream>>>(kp_beta<double>(alpha), seed, n, nbins,
                                                                                              d_counts, h->d_status);
         rc = launch_end(h, SU2G_K_OTHER, "sampler histogram");
     }

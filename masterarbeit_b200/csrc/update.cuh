@@ -5,6 +5,7 @@
 #include <cfloat>
 
 #include "internal.cuh"
+#include "kpmath.cuh"
 #include "philox.cuh"
 
 namespace su2g {
@@ -16,31 +17,42 @@ __device__ __forceinline__ float eps_r<float>() { return FLT_EPSILON; }
 template <>
 __device__ __forceinline__ double eps_r<double>() { return DBL_EPSILON; }
 
-// Sampler math.  FP64 uses the accurate library functions.  FP32 uses the hardware approximations
+// Sampler math on the 32-bit words themselves.  FP64: kpmath.cuh.  FP32 uses the hardware approximations
 // (__logf: absolute error ~2^-21 on (0,1]; __sincosf on [-pi, pi]: ~2^-21), which are below the
 // 2^-23 resolution of the FP32 uniforms' effect on delta and the angles.
-__device__ __forceinline__ float kp_log(float x) { return __logf(x); }
-__device__ __forceinline__ double kp_log(double x) { return log(x); }
+__device__ __forceinline__ float kp_log(uint32_t w, float) { return __logf(u01(w, 0.0f)); }
+__device__ __forceinline__ double kp_log(uint32_t w, double) { return kp_log_word(w); }
 // cos and sin of 2 pi u for u in (0,1)
-__device__ __forceinline__ void kp_sincos2pi(float u, float* s, float* c)
+__device__ __forceinline__ void kp_sincos2pi(uint32_t w, float* s, float* c)
 {
+    const float u = u01(w, 0.0f);
     float ss, cc;
     __sincosf(6.28318530717958647692f * (u - 0.5f), &ss, &cc);   // 2 pi (u - 1/2) in [-pi, pi]
     *s = -ss;
     *c = -cc;
 }
-__device__ __forceinline__ void kp_sincos2pi(double u, double* s, double* c) { sincospi(2.0 * u, s, c); }
-__device__ __forceinline__ float kp_cos2pi(float u) { return -__cosf(6.28318530717958647692f * (u - 0.5f)); }
-__device__ __forceinline__ double kp_cos2pi(double u) { return cospi(2.0 * u); }
-// Square root of x >= 0: FP32 uses the hardware approximation (sqrt.approx.f32, relative error
-// ~2^-23), FP64 the correctly rounded one.
+__device__ __forceinline__ void kp_sincos2pi(uint32_t w, double* s, double* c) { kp_sincos2pi_word(w, s, c); }
+__device__ __forceinline__ float kp_cos2pi_sq(uint32_t w, float)
+{
+    const float c = -__cosf(6.28318530717958647692f * (u01(w, 0.0f) - 0.5f));
+    return c * c;
+}
+__device__ __forceinline__ double kp_cos2pi_sq(uint32_t w, double) { return kp_cos2pi_sq_word(w); }
+// Square root of x > 0: FP32 uses the hardware approximation (sqrt.approx.f32, relative error
+// ~2^-23), FP64 the reciprocal square root.
 __device__ __forceinline__ float kp_sqrt(float x)
 {
     float r;
     asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
-__device__ __forceinline__ double kp_sqrt(double x) { return sqrt(x); }
+__device__ __forceinline__ double kp_sqrt(double x) { return x * rsqrt(x); }
+// What the sampler takes for beta: FP32 beta itself, FP64 its reciprocal (a division a link less).
+template <typename R>
+__host__ __device__ __forceinline__ R kp_beta(double beta)
+{
+    return sizeof(R) == 8 ? R(1.0 / beta) : R(beta);
+}
 // 1/|A| and 1/(beta |A|) from |A|^2, from one reciprocal square root (FP32: the hardware
 // approximation; FP64: rsqrt, within an ulp, in place of a square root and two divisions: the FP64
 // heatbath pass 152.9 -> 152.1 us at 48^4).  |A| = 0 gives k = NaN (0 * inf), which fails the
@@ -51,11 +63,11 @@ __device__ __forceinline__ void kp_norms(float n2, float beta, float& k, float& 
     k = n2 * ik;
     ia = __fdividef(ik, beta);
 }
-__device__ __forceinline__ void kp_norms(double n2, double beta, double& k, double& ik, double& ia)
+__device__ __forceinline__ void kp_norms(double n2, double ibeta, double& k, double& ik, double& ia)
 {
     ik = rsqrt(n2);
     k = n2 * ik;
-    ia = ik / beta;
+    ia = ik * ibeta;
 }
 // The FP32 logs of uniforms just below 1 may come out positive by their absolute error (~2^-21);
 // delta is clamped at 0 so that sqrt(delta (2 - delta)) stays real.  FP64 logs are exact in sign.
@@ -125,14 +137,15 @@ __device__ __forceinline__ Q<R> fallback_link(R r0, R r1, R r2)
 // `draw_base` (visit << kVisitShift) separates the draws of repeated visits in a random-order sweep.
 constexpr int kVisitShift = 21;   // above every trial index (kMaxTrials = 2^20)
 
-// `seed` is the 64-bit seed or its precomputed round keys (PhiloxKeys): the same draws either way.
+// `seed` is the 64-bit seed or its precomputed round keys (PhiloxKeys): the same draws either way; kb is
+// kp_beta<R>(beta).
 template <typename R, typename Seed>
-__device__ __forceinline__ bool heatbath_link(const Q<R>& A, R beta, const Seed& seed, uint32_t site, uint32_t sweep,
+__device__ __forceinline__ bool heatbath_link(const Q<R>& A, R kb, const Seed& seed, uint32_t site, uint32_t sweep,
                                               uint32_t mu, uint32_t replica, uint32_t& trials, Q<R>& out,
                                               unsigned* status, uint32_t draw_base = 0u)
 {
     R k, ik, ia;   // |A|, 1/|A|, 1/alpha with alpha = |A| beta (heatbath.c:142)
-    kp_norms(q_norm2(A), beta, k, ik, ia);
+    kp_norms(q_norm2(A), kb, k, ik, ia);
     if (!(k > eps_r<R>())) {
         U4 w = link_random(seed, site, sweep, mu, draw_base | 1u, 1u, kStreamUpdate, replica);
         trials = 0;
@@ -144,10 +157,9 @@ __device__ __forceinline__ bool heatbath_link(const Q<R>& A, R beta, const Seed&
     for (;;) {
         U4 w = link_random(seed, site, sweep, mu, draw_base | trial, 0u, kStreamUpdate, replica);
         ++trial;
-        const R u0 = u01(w.x, R(0)), u1 = u01(w.y, R(0)), u2 = u01(w.z, R(0)), u3 = u01(w.w, R(0));
-        const R c = kp_cos2pi(u2);
+        const R u3 = u01(w.w, R(0));
         // X1 = -ln(u0)/alpha, X2 = -ln(u1)/alpha, delta = X2 + X1 cos^2(2 pi u2)  (heatbath.c:86-90)
-        delta = kp_clamp(-(kp_log(u1) + kp_log(u0) * (c * c)) * ia);
+        delta = kp_clamp(-(kp_log(w.y, R(0)) + kp_log(w.x, R(0)) * kp_cos2pi_sq(w.z, R(0))) * ia);
         if (u3 * u3 <= R(1) - R(0.5) * delta) break;   // heatbath.c:94
         if (trial >= kMaxTrials) {   // the link keeps its value and the host sees the status bit
             atomicOr(status, kStatusKpTrials);
@@ -158,11 +170,11 @@ __device__ __forceinline__ bool heatbath_link(const Q<R>& A, R beta, const Seed&
     trials = trial;
     // x0 = 1 - delta; (x1,x2,x3) = sqrt(1-x0^2) (sin th cos ph, sin th sin ph, cos th)  (heatbath.c:96-107)
     U4 w = link_random(seed, site, sweep, mu, draw_base, 1u, kStreamUpdate, replica);
-    const R a0 = u01(w.x, R(0)), a1 = u01(w.y, R(0));
+    const R a1 = u01(w.y, R(0));
     const R cth = R(1) - R(2) * a1;
     const R sth = R(2) * kp_sqrt(a1 * (R(1) - a1));       // sin(acos(1 - 2 a1))
     R sph, cph;
-    kp_sincos2pi(a0, &sph, &cph);
+    kp_sincos2pi(w.x, &sph, &cph);
     const R len = kp_sqrt(delta * (R(2) - delta));          // sqrt(1 - (1-delta)^2)
     Q<R> X = q_make<R>(R(1) - delta, len * sth * cph, len * sth * sph, len * cth);
     // U = X V^dag, V = A/k  (heatbath.c:140-146)
