@@ -123,12 +123,15 @@ int ensure_partial_entries(su2g_lattice* h, size_t n)
 // (The plaquette's 20736 partials at 48^4 took 42 us with one chain per thread of 256.)
 constexpr int kFinalizeBlock = 1024;
 
-__global__ void __launch_bounds__(kFinalizeBlock) k_finalize(const DD* __restrict__ partials, int nparts, int stride,
-                                                             double scale, double* __restrict__ out)
+__global__ void __launch_bounds__(kFinalizeBlock) k_finalize(const DD* partials, int nparts, size_t stride, double scale,
+                                                             double* out, int out_stride)
 {
-    const DD* p = partials + (size_t)blockIdx.x * stride;
+    pdl_trigger();
+    int t0 = threadIdx.x, dummy = 0;
+    pdl_wait(t0, dummy);
+    const DD* p = partials + blockIdx.x * stride;
     DD acc[4] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
-    int i = threadIdx.x;
+    int i = t0;
     for (; i + 3 * kFinalizeBlock < nparts; i += 4 * kFinalizeBlock) {
         const DD a = p[i], b = p[i + kFinalizeBlock], c = p[i + 2 * kFinalizeBlock], d = p[i + 3 * kFinalizeBlock];
         acc[0] = dd_add(acc[0], a);
@@ -141,23 +144,28 @@ __global__ void __launch_bounds__(kFinalizeBlock) k_finalize(const DD* __restric
     if (i + 2 * kFinalizeBlock < nparts) acc[2] = dd_add(acc[2], p[i + 2 * kFinalizeBlock]);
     DD v = dd_add(dd_add(acc[0], acc[1]), dd_add(acc[2], acc[3]));
     v = dd_block_sum<kFinalizeBlock>(v);
-    if (threadIdx.x == 0) out[blockIdx.x] = (v.s + v.e) * scale;
+    if (threadIdx.x == 0) out[(size_t)blockIdx.x * out_stride] = (v.s + v.e) * scale;
 }
 
-// One slot of many partials: CTA b sums the contiguous chunk b (fixed assignment), and the CTA
-// that arrives last on the counter sums the CTA results in index order and clears the counter, so
-// the result does not depend on which CTA finished when.  (The fused plaquette's 249k partials
-// at 48^4 took 17 us in one CTA of k_finalize.)
+// Few slots of many partials: CTA (b, k) sums the contiguous chunk b of slot k (fixed assignment), and
+// the CTA of a slot that arrives last on its counter sums the slot's CTA results in index order and
+// clears the counter, so the result does not depend on which CTA finished when.  (The fused plaquette's
+// 249k partials at 48^4 took 17 us in one CTA of k_finalize.)
 constexpr int kFinWideThreads = 256;
 static_assert(kFinBlocks <= kFinWideThreads, "the last CTA sums one CTA result per thread");
 
-__global__ void __launch_bounds__(kFinWideThreads) k_finalize_wide(const DD* __restrict__ partials, int nparts,
-                                                                   double scale, double* __restrict__ out,
-                                                                   DD* __restrict__ blocks, unsigned* ticket)
+__global__ void __launch_bounds__(kFinWideThreads) k_finalize_wide(const DD* partials, int nparts, size_t stride,
+                                                                   double scale, double* out, int out_stride, DD* blocks,
+                                                                   unsigned* tickets)
 {
-    const int nb = gridDim.x;
+    pdl_trigger();
+    const int nb = gridDim.x, slot = blockIdx.y;
     const int chunk = (nparts + nb - 1) / nb;
-    const int lo = blockIdx.x * chunk, hi = min(nparts, lo + chunk);
+    int lo = blockIdx.x * chunk, dummy = 0;
+    pdl_wait(lo, dummy);
+    const int hi = min(nparts, lo + chunk);
+    partials += slot * stride;
+    blocks += slot * kFinBlocks;
     DD acc[2] = {{0.0, 0.0}, {0.0, 0.0}};
     int i = lo + threadIdx.x;
     for (; i + kFinWideThreads < hi; i += 2 * kFinWideThreads) {
@@ -170,7 +178,7 @@ __global__ void __launch_bounds__(kFinWideThreads) k_finalize_wide(const DD* __r
     if (threadIdx.x == 0) {
         blocks[blockIdx.x] = v;
         __threadfence();
-        last = atomicAdd(ticket, 1u) == (unsigned)nb - 1u;
+        last = atomicAdd(&tickets[slot], 1u) == (unsigned)nb - 1u;
     }
     __syncthreads();
     if (!last) return;
@@ -183,38 +191,39 @@ __global__ void __launch_bounds__(kFinWideThreads) k_finalize_wide(const DD* __r
     }
     w = dd_block_sum<kFinWideThreads>(w);
     if (threadIdx.x == 0) {
-        *out = (w.s + w.e) * scale;
-        *ticket = 0u;
+        out[(size_t)slot * out_stride] = (w.s + w.e) * scale;
+        tickets[slot] = 0u;
     }
 }
 
-int finalize(su2g_lattice* h, int nparts, int nslots, double scale, int out_off, int stride)
+int finalize(su2g_lattice* h, const DD* parts, int nparts, int nslots, size_t stride, double scale, double* out,
+             int out_stride)
 {
-    if (out_off + nslots > kOutSlots) return set_error(h, SU2G_EINVAL, "too many result slots");
     launch_begin(h, SU2G_K_REDUCE);
-    if (nslots == 1 && nparts > 4 * kFinalizeBlock) {
+    if (nslots <= kFinSlots && nparts > 4 * kFinalizeBlock) {
         const int nb = std::min(kFinBlocks, (nparts + 2 * kFinWideThreads - 1) / (2 * kFinWideThreads));
-        k_finalize_wide<<<nb, kFinWideThreads, 0, h->stream>>>(h->partials, nparts, scale, h->d_out + out_off,
-                                                              h->fin_blocks, h->fin_ticket);
+        launch_pdl(k_finalize_wide, dim3(nb, nslots), kFinWideThreads, h->stream, parts, nparts, stride, scale, out,
+                   out_stride, h->fin_blocks, h->fin_ticket);
     } else {
-        k_finalize<<<nslots, kFinalizeBlock, 0, h->stream>>>(h->partials, nparts, stride > 0 ? stride : kMaxPartials,
-                                                              scale, h->d_out + out_off);
+        launch_pdl(k_finalize, dim3(nslots), kFinalizeBlock, h->stream, parts, nparts, stride, scale, out, out_stride);
     }
     return launch_end(h, SU2G_K_REDUCE, "finalize reduction");
 }
 
 int fetch_results(su2g_lattice* h, int off, int n)
 {
-    int rc = check_cuda(h, cudaMemcpyAsync(h->h_out + off, h->d_out + off, n * sizeof(double),
-                                           cudaMemcpyDeviceToHost, h->stream),
+    // the status word and the slots up to off + n in one copy, or in two where the slots before off are many
+    const int head = off <= 64 ? 1 + off + n : 1;
+    int rc = check_cuda(h, cudaMemcpyAsync(h->h_base, h->d_base, head * sizeof(double), cudaMemcpyDeviceToHost, h->stream),
                         "copying results");
+    if (!rc && off > 64)
+        rc = check_cuda(h, cudaMemcpyAsync(h->h_out + off, h->d_out + off, n * sizeof(double), cudaMemcpyDeviceToHost,
+                                           h->stream),
+                        "copying results");
+    if (!rc) rc = check_cuda(h, cudaStreamSynchronize(h->stream), "synchronising");
     if (rc) return rc;
-    unsigned status = 0;
-    rc = check_cuda(h, cudaMemcpyAsync(&status, h->d_status, sizeof(unsigned), cudaMemcpyDeviceToHost, h->stream),
-                    "reading status word");
-    if (rc) return rc;
-    rc = check_cuda(h, cudaStreamSynchronize(h->stream), "synchronising");
-    if (rc) return rc;
+    unsigned status;
+    std::memcpy(&status, h->h_base, sizeof(status));
     // a reported failure is reported once: the word is cleared and the handle stays usable
     if (status && (rc = check_cuda(h, cudaMemsetAsync(h->d_status, 0, sizeof(unsigned), h->stream), "clearing status")))
         return rc;
@@ -412,6 +421,7 @@ extern "C" int su2g_create(const su2g_params* p, su2g_lattice** out)
     h->device = p->device;
     h->num_sms = prop.multiProcessorCount;
     h->max_smem = (int)prop.sharedMemPerBlockOptin;
+    h->l2_bytes = (size_t)prop.l2CacheSize;
     h->link_bytes = p->precision == SU2G_FP32 ? 16 : 32;
 
     int rc = SU2G_OK;
@@ -422,18 +432,21 @@ extern "C" int su2g_create(const su2g_params* p, su2g_lattice** out)
         rc = check_cuda(h, e, "allocating the gauge field");
     if (!rc)
         for (int mu = 0; mu < 4; ++mu) h->dirp[mu] = (char*)h->field + (size_t)mu * 2 * h->g.Vh * h->link_bytes;
-    if (!rc && (e = cudaMalloc(&h->d_out, kOutSlots * sizeof(double))) != cudaSuccess)
+    if (!rc && (e = cudaMalloc(&h->d_base, (1 + kOutSlots) * sizeof(double))) != cudaSuccess)
         rc = check_cuda(h, e, "allocating result slots");
-    if (!rc && (e = cudaMallocHost(&h->h_out, kOutSlots * sizeof(double))) != cudaSuccess)
+    if (!rc && (e = cudaMallocHost(&h->h_base, (1 + kOutSlots) * sizeof(double))) != cudaSuccess)
         rc = check_cuda(h, e, "allocating pinned result slots");
-    if (!rc && (e = cudaMalloc(&h->d_status, sizeof(unsigned))) != cudaSuccess)
-        rc = check_cuda(h, e, "allocating status word");
-    if (!rc) rc = check_cuda(h, cudaMemsetAsync(h->d_status, 0, sizeof(unsigned), h->stream), "clearing status");
-    if (!rc && (e = cudaMalloc(&h->fin_blocks, kFinBlocks * sizeof(DD))) != cudaSuccess)
+    if (!rc) {
+        h->d_out = h->d_base + 1;
+        h->h_out = h->h_base + 1;
+        h->d_status = reinterpret_cast<unsigned*>(h->d_base);
+        rc = check_cuda(h, cudaMemsetAsync(h->d_base, 0, sizeof(double), h->stream), "clearing status");
+    }
+    if (!rc && (e = cudaMalloc(&h->fin_blocks, kFinSlots * kFinBlocks * sizeof(DD))) != cudaSuccess)
         rc = check_cuda(h, e, "allocating reduction scratch");
-    if (!rc && (e = cudaMalloc(&h->fin_ticket, sizeof(unsigned))) != cudaSuccess)
+    if (!rc && (e = cudaMalloc(&h->fin_ticket, kFinSlots * sizeof(unsigned))) != cudaSuccess)
         rc = check_cuda(h, e, "allocating reduction scratch");
-    if (!rc) rc = check_cuda(h, cudaMemsetAsync(h->fin_ticket, 0, sizeof(unsigned), h->stream), "clearing reduction counter");
+    if (!rc) rc = check_cuda(h, cudaMemsetAsync(h->fin_ticket, 0, kFinSlots * sizeof(unsigned), h->stream), "clearing reduction counter");
     if (!rc) rc = ensure_partials(h, 2);
     if (!rc) wilson_prepare(h);
     if (!rc) rc = check_cuda(h, cudaEventCreate(&h->ev_begin), "creating events");
@@ -461,23 +474,19 @@ extern "C" int su2g_destroy(su2g_lattice* h)
     for (auto e : h->event_pool) cudaEventDestroy(e);
     if (h->ev_begin) cudaEventDestroy(h->ev_begin);
     if (h->ev_end) cudaEventDestroy(h->ev_end);
-    release_run_graph(h);
     release_meas_graph(h);
     if (h->pool) cudaMemPoolDestroy(h->pool);
     cudaFree(h->lines);
     cudaFree(h->meas_work);
     cudaFree(h->meas_alt);
-    cudaFree(h->d_run_ctr);
-    cudaFree(h->d_trace);
     cudaFree(h->field);
     cudaFree(h->field_alt);
     cudaFree(h->partials);
-    cudaFree(h->d_out);
-    cudaFree(h->d_status);
+    cudaFree(h->d_base);
     cudaFree(h->fin_blocks);
     cudaFree(h->fin_ticket);
     cudaFree(h->d_aos);
-    if (h->h_out) cudaFreeHost(h->h_out);
+    if (h->h_base) cudaFreeHost(h->h_base);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
     return SU2G_OK;

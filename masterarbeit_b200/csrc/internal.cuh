@@ -3,6 +3,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <utility>
 #include <vector>
 #include <cuda_runtime.h>
 
@@ -13,7 +14,8 @@ namespace su2g {
 
 constexpr int kBlock = 256;            // threads per CTA for the stencil kernels
 constexpr int kMaxPartials = 8192;     // per-CTA partial sums a reduction may write
-constexpr int kFinBlocks = 128;        // CTAs of the wide final reduction (one slot, many partials)
+constexpr int kFinBlocks = 128;        // CTAs per slot of the wide final reduction (many partials)
+constexpr int kFinSlots = 16;          // slots one wide final reduction may sum
 constexpr int kOutSlots = 16384;       // device result doubles per handle
 constexpr uint32_t kMaxTrials = 1u << 20;   // Kennedy-Pendleton trials before a link gives up
 
@@ -97,11 +99,6 @@ __device__ __forceinline__ DD dd_block_sum(DD v)
     return v;
 }
 
-// Sums `nparts` per-CTA partials for `nslots` independent slots (partials[slot*stride + part])
-// into out[slot] = scale * sum.  One CTA per slot, fixed order.
-__global__ void k_finalize(const DD* __restrict__ partials, int nparts, int stride, double scale,
-                           double* __restrict__ out);
-
 }  // namespace su2g
 
 struct su2g_meas_graph;   // measure.cu
@@ -122,35 +119,27 @@ struct su2g_lattice {
     void* altp[4] = {nullptr, nullptr, nullptr, nullptr};   // ping-pong partner of each direction
     su2g::DD* partials = nullptr;   // kMaxPartials x kPartialSlots compensated partial sums
     size_t partial_slots = 0;
-    double* d_out = nullptr;     // device result slots
+    // Results: one 8-byte head whose first word is the status word, then the result slots, so that one
+    // copy brings a call's results and the status back.
+    double* d_base = nullptr;
+    double* h_base = nullptr;    // pinned host mirror
+    double* d_out = nullptr;     // device result slots (d_base + 1)
     double* h_out = nullptr;     // pinned host mirror of d_out
     unsigned* d_status = nullptr;
-    su2g::DD* fin_blocks = nullptr;   // per-CTA sums of the wide final reduction (kFinBlocks)
-    unsigned* fin_ticket = nullptr;   // its arrival counter (zero between launches)
+    su2g::DD* fin_blocks = nullptr;   // per-CTA sums of the wide final reduction (kFinSlots x kFinBlocks)
+    unsigned* fin_ticket = nullptr;   // its arrival counters, one per slot (zero between launches)
     double* d_aos = nullptr;     // device staging for AoS FP64 transfers
     size_t aos_sites = 0;        // sites the staging buffer holds
     cudaStream_t stream = nullptr;
     cudaEvent_t ev_begin = nullptr, ev_end = nullptr;
     int max_smem = 0;            // opt-in shared memory per CTA
+    size_t l2_bytes = 0;
     int ape_variant = 0;         // 0: per-site APE kernel, 1: TMA-tiled FP32 APE_all where it applies
-    // Graph of one measurement block of su2g_run (recaptured when its key changes).
-    struct RunGraph {
-        cudaGraphExec_t exec = nullptr;
-        int meas_every = 0, n_hb = 0, n_or = 0;
-        double beta = 0.0;
-        uint64_t seed = 0;
-        const void* partials = nullptr;
-        const double* trace = nullptr;
-        void* dirp[4] = {nullptr, nullptr, nullptr, nullptr};
-    } run;
     cudaMemPool_t pool = nullptr;      // scratch of the adjoint; keeps its memory until destroy
     su2g_meas_graph* meas = nullptr;   // graph of one su2g_measure spec
     void* lines = nullptr;             // 2- and 3-link line products of the field Q is measured on
     void* meas_work = nullptr;         // measurement copy of the field and its ping-pong partner
     void* meas_alt = nullptr;
-    uint32_t* d_run_ctr = nullptr;   // [0] heatbath sweep index, [1] trace row (advanced by the graph)
-    double* d_trace = nullptr;       // per block: plaquette, acceptance
-    size_t trace_rows = 0;
     bool profiling = false;
     struct Prof {
         cudaEvent_t a, b;
@@ -180,12 +169,29 @@ int resident_grid(const su2g_lattice* h, const void* kernel, long long work, siz
 int launch_begin(su2g_lattice* h, int cls);
 int launch_end(su2g_lattice* h, int cls, const char* what);
 
+// Launch a kernel that calls pdl_wait: it may start before the launch ahead of it in the stream has ended.
+template <typename... Params, typename... Args>
+inline void launch_pdl(void (*kernel)(Params...), dim3 grid, int block, cudaStream_t stream, Args&&... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);   // the caller checks cudaGetLastError
+}
+
 // Make sure the partial-sum scratch holds `slots` x kMaxPartials entries (or at least n entries).
 int ensure_partials(su2g_lattice* h, size_t slots);
 int ensure_partial_entries(su2g_lattice* h, size_t n);
-// Launch k_finalize over `nslots` slots of `nparts` partials (slot k at partials[k * stride],
-// stride 0 = kMaxPartials) into d_out[out_off ...].
-int finalize(su2g_lattice* h, int nparts, int nslots, double scale, int out_off, int stride = 0);
+// Sum `nparts` partials for each of `nslots` independent slots (slot k at parts[k * stride]) into
+// out[k * out_stride] = scale * sum, in a fixed order.
+int finalize(su2g_lattice* h, const DD* parts, int nparts, int nslots, size_t stride, double scale, double* out,
+             int out_stride = 1);
 // Copy n result doubles from d_out[off] to h_out and synchronise; then check the status word.
 int fetch_results(su2g_lattice* h, int off, int n);
 
@@ -223,8 +229,6 @@ int tau_int_enqueue(const double* d_x, long long n, long long si, long long ss, 
                     double* d_out, int* d_resolved);
 // Destroy the captured su2g_measure graph, if any.
 void release_meas_graph(su2g_lattice* h);
-// Destroy the captured su2g_graph_run block, if any.
-void release_run_graph(su2g_lattice* h);
 // Enqueue W(R[i], T[i]) of the field at dirs.  Loops are measured in chunks of R and T; each
 // chunk's results land in consecutive d_out slots from out_off on, and slot[i] receives the d_out
 // index of pair i.  Fails (nothing enqueued) if the pairs need more than `max_slots` slots.
@@ -234,20 +238,17 @@ int wilson_enqueue(su2g_lattice* h, void* const dirs[4], const int32_t* R, const
 void wilson_prepare(su2g_lattice* h);
 // Check R, T >= 1 and T <= L_t - 1 (measureWilsonLoop, wilson.c:290-291).
 int wilson_check(su2g_lattice* h, const int32_t* R, const int32_t* T, int n, const char* who);
-// Enqueue the plaquette of the current field into d_out[out_off].
-int plaquette_enqueue(su2g_lattice* h, int out_off);
-// One (mu, parity) update pass.  The heatbath sweep index is `sweep`, plus *sweep_base when
-// sweep_base is given (a device counter, so that a captured graph advances it by itself).  With
-// plaq_part (parity-1 passes of mu >= 1 only) the pass also writes one plaquette partial per CTA.
-int launch_update(su2g_lattice* h, int kind, int mu, int par, uint32_t sweep, double* acc_sum,
-                  const uint32_t* sweep_base = nullptr, DD* plaq_part = nullptr);
-// CTAs of an update pass (one link per thread), and the plaquette partials of a fused pass.
-int update_grid(const su2g_lattice* h);
-int update_plaq_parts(const su2g_lattice* h);
+// Enqueue the plaquette of the current field into *out (device).
+int plaquette_enqueue(su2g_lattice* h, double* out);
+// One (mu, parity) update pass with heatbath sweep index `sweep`.  With plaq_part (parity-1 passes of
+// mu >= 1 only) the pass also writes one plaquette partial per warp.
+int launch_update(su2g_lattice* h, int kind, int mu, int par, uint32_t sweep, double* acc_sum, DD* plaq_part = nullptr);
+// Partials of the plaquette fused into a sub-sweep (its three passes together), and the reduction
+// that turns nslots sets of them, one after another from `parts`, into out[k * out_stride].
+int sweep_plaq_parts(const su2g_lattice* h);
+int sweep_plaq_finalize(su2g_lattice* h, const DD* parts, int nslots, double* out, int out_stride = 1);
 // Enqueue n_sweeps x (n_hb heatbath + n_or overrelaxation sweeps); heatbath sub-sweep j (counted
-// from 0 within the call) has index sweep0 + j (+ *base).  With plaq_off >= 0 the last sub-sweep
-// also sums the plaquette of the final field into d_out[plaq_off] (the plaquette kernel runs
-// instead when there is no sub-sweep); partials[0 .. 3 * update_plaq_parts) are used.
-int sweep_enqueue(su2g_lattice* h, int n_sweeps, int n_hb, int n_or, uint32_t sweep0, const uint32_t* base,
-                  double* acc_dev, int plaq_off);
+// from 0 within the call) has index sweep0 + j.  With plaq_part the last sub-sweep (there must be one)
+// also leaves the partials of the final field's plaquette there.
+int sweep_enqueue(su2g_lattice* h, int n_sweeps, int n_hb, int n_or, uint32_t sweep0, double* acc_dev, DD* plaq_part);
 }  // namespace su2g

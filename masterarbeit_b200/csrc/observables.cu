@@ -578,13 +578,13 @@ extern "C" int su2g_plaquette(su2g_lattice* h, double* p)
     if (!h) return set_error(nullptr, SU2G_EINVAL, "su2g_plaquette: null handle");
     if (!p) return set_error(h, SU2G_EINVAL, "su2g_plaquette: null output");
     cudaSetDevice(h->device);
-    int rc = plaquette_enqueue(h, 0);
+    int rc = plaquette_enqueue(h, h->d_out);
     if (!rc) rc = fetch_results(h, 0, 1);
     if (!rc) *p = h->h_out[0];
     return rc;
 }
 
-int su2g::plaquette_enqueue(su2g_lattice* h, int out_off)
+int su2g::plaquette_enqueue(su2g_lattice* h, double* out)
 {
     const int grid = 2 * (int)((h->g.Vh + 127) / 128);
     int rc = ensure_partial_entries(h, grid);
@@ -596,7 +596,7 @@ int su2g::plaquette_enqueue(su2g_lattice* h, int out_off)
         k_plaquette<double><<<grid, 128, 0, h->stream>>>(make_field<double>(h->dirp, h->g.Vh), h->g, h->partials);
     rc = launch_end(h, SU2G_K_PLAQUETTE, "plaquette kernel");
     // plaq = sum 2 c0 / (2 * 6 * V)  (plaquette.c:97); the kernel sums c0 = (1/2) Re tr
-    if (!rc) rc = finalize(h, grid, 1, 1.0 / (6.0 * (double)h->g.V), out_off, grid);
+    if (!rc) rc = finalize(h, h->partials, grid, 1, grid, 1.0 / (6.0 * (double)h->g.V), out);
     return rc;
 }
 
@@ -672,7 +672,7 @@ int su2g::qtop_enqueue(su2g_lattice* h, void* const dirs[4], int out_off, void* 
     else launch_qtop<double>(h, dirs, grid, fbar);
     int rc = launch_end(h, SU2G_K_QTOP, "topological charge kernel");
     // Q = sum_x q(x) / (32 pi^2)  (topologicalcharge.c:194)
-    if (!rc) rc = finalize(h, grid, 2, 1.0 / (32.0 * kPi * kPi), out_off, grid);
+    if (!rc) rc = finalize(h, h->partials, grid, 2, grid, 1.0 / (32.0 * kPi * kPi), h->d_out + out_off);
     return rc;
 }
 
@@ -762,7 +762,8 @@ int su2g::wilson_enqueue(su2g_lattice* h, void* const dirs[4], const int32_t* R,
                                               : launch_wilson<double>(h, dirs, c.rc_n, c.r0, c.tlo, c.thi);
         if ((rc = launch_end(h, SU2G_K_WILSON, "Wilson loop kernel"))) return rc;
         // W = sum_x,k c0 / (3 V)  (wilson.c:322: sum of Re tr / (3 V 2))
-        if ((rc = finalize(h, grid, c.rc_n * kWilsonTChunk, 1.0 / (3.0 * (double)h->g.V), c.base))) return rc;
+        if ((rc = finalize(h, h->partials, grid, c.rc_n * kWilsonTChunk, kMaxPartials, 1.0 / (3.0 * (double)h->g.V),
+                           h->d_out + c.base))) return rc;
     }
     for (int i = 0; i < n; ++i) slot[i] = slot_rt[(size_t)(R[i] - 1) * tmax + (T[i] - 1)];
     return SU2G_OK;

@@ -358,6 +358,12 @@ __device__ __forceinline__ Q<double> ldnc_256(const Vec4d* a)
     asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(q.c0), "=d"(q.c1), "=d"(q.c2), "=d"(q.c3) : "l"(a));
     return q;
 }
+__device__ __forceinline__ Q<double> ld_256(const Vec4d* a)
+{
+    Q<double> q;
+    asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(q.c0), "=d"(q.c1), "=d"(q.c2), "=d"(q.c3) : "l"(a));
+    return q;
+}
 __device__ __forceinline__ Q<double> ldcg_256(const Vec4d* a)
 {
     Q<double> q;
@@ -432,6 +438,50 @@ __device__ __forceinline__ void stq(double* p, size_t i, const Q<double>& q)
 {
     st_256(reinterpret_cast<Vec4d*>(p) + i, q);
 }
+
+// The same views with plain loads, for a kernel that may start while the launch before it is still
+// writing (programmatic dependent launch): such a kernel's links are not read-only for its lifetime,
+// which the read-only path of __ldg requires.  The loads are pure functions of their addresses to the
+// compiler; pdl_wait below keeps them behind the wait.
+template <typename R>
+struct FieldCA;
+
+template <>
+struct FieldCA<float> : Field<float> {
+    __device__ __forceinline__ Q<float> ld(int mu, int par, int n) const { return ldh(mu, par, (int)((unsigned)n >> 1)); }
+    __device__ __forceinline__ Q<float> ldh(int mu, int par, int h) const
+    {
+        Q<float> q;
+        asm("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
+            : "=f"(q.c0), "=f"(q.c1), "=f"(q.c2), "=f"(q.c3)
+            : "l"(p[mu] + (unsigned)(par * Vh + h)));
+        return q;
+    }
+};
+
+template <>
+struct FieldCA<double> : Field<double> {
+    __device__ __forceinline__ Q<double> ld(int mu, int par, int n) const { return ldh(mu, par, (int)((unsigned)n >> 1)); }
+    __device__ __forceinline__ Q<double> ldh(int mu, int par, int h) const { return ld_256(p[mu] + (unsigned)(par * Vh + h)); }
+};
+
+template <typename R>
+__device__ __forceinline__ FieldCA<R> field_ca(const Field<R>& f)
+{
+    FieldCA<R> c;
+    for (int mu = 0; mu < 4; ++mu) c.p[mu] = f.p[mu];
+    c.Vh = f.Vh;
+    return c;
+}
+
+// Programmatic dependent launch.  pdl_trigger: the next launch of the stream may start once every CTA
+// of this one has got here.  pdl_wait: every launch before this one has completed and its writes are
+// visible; h and n, the indices all later accesses are formed from, pass through it, so that none of
+// them can be moved ahead of it.  Every thread calls pdl_wait, so that a launch never completes
+// before the one it waited for.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void pdl_wait(int& h, int& n) { asm volatile("griddepcontrol.wait;" : "+r"(h), "+r"(n)::"memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Field view over four direction base pointers (each 2*Vh links long).
 template <typename R>

@@ -23,12 +23,47 @@ using namespace su2g;
 
 namespace {
 
-// 32 resident warps per SM (at most 64 registers a thread): measured at 48^4 on B200 against 8, 16,
-// 24 and 48, it is the fastest for both kinds and precisions (OR FP32 64 us against 79 us unbounded).
-// Both kinds run them as eight 128-thread CTAs: finer CTAs shorten the pass's tail (OR 65.8 against
-// 66.7 us, HB 86.7 against 88.1 us with four CTAs of 256).
-template <int KIND>
-constexpr int update_block() { return 128; }
+// 128-thread CTAs (finer CTAs shorten the tail: at 48^4 on B200 OR 65.8 against 66.7 us, HB 86.7 against
+// 88.1 us with four CTAs of 256).
+constexpr int kUpdateBlock = 128;
+
+// How many CTAs per SM a pass's kernel is compiled for, which fixes its registers, and how many
+// Kennedy-Pendleton trials a heatbath draws before its pass may read links (EARLY, below).
+//  - A grid that fits one wave of n CTAs per SM takes the kernel for n: nothing is gained by leaving
+//    room for more, and the registers keep more of the 18 staple links in flight.
+//  - Larger grids: six CTAs per SM while the FP64 field stays in L2, or while a FP32 grid is at most
+//    one wave of eight; else eight (32 warps per SM; against 8, 16, 24 and 48 the fastest at 48^4), where
+//    FP64 draws nothing early (no registers left).
+// Twenty FP64 / FP32 heatbath sweeps on B200, ms, with the kernel for 2, 3, 4, 6, 8 CTAs (FP64: eight without
+// early draws):
+//    16^4           0.69 0.81 0.85 1.01 0.95      0.57 0.63 0.63 0.72 0.85
+//    24x14x18x22    1.11 1.05 0.92 1.21 1.04      0.59 0.60 0.60 0.77 0.82
+//    24^4           2.10 1.72 1.67 1.64 1.90      1.10 1.10 1.10 0.94 0.97
+//    28^4           3.80 3.08 2.88 2.65 2.82      1.74 1.74 1.74 1.48 1.47
+//    48^4                          24.6 23.5                     12.8 12.7
+struct UpdateShape {
+    int ctas, early;
+};
+constexpr UpdateShape kShapes[] = {{2, 3}, {3, 3}, {4, 3}, {6, 2}, {8, 2}, {8, 0}};
+constexpr int kShape8Early = 4, kShape8 = 5;
+
+// The shapes compiled: FP32 gains little from two or three CTAs; overrelaxation draws nothing.
+template <typename R, int KIND>
+constexpr bool shape_used(int i)
+{
+    return KIND == SU2G_OVERRELAX ? (sizeof(R) == 8 ? i == 0 || i == 2 || i == kShape8 : i == 2 || i == kShape8)
+                                  : (sizeof(R) == 8 ? i != kShape8Early : i >= 2 && i != kShape8);
+}
+
+template <typename R, int KIND>
+int update_shape(const su2g_lattice* h, int grid)
+{
+    for (int i = 0; i < 3; ++i)
+        if (shape_used<R, KIND>(i) && grid <= kShapes[i].ctas * h->num_sms) return i;
+    if (KIND == SU2G_OVERRELAX) return kShape8;
+    if (sizeof(R) == 8) return 4ull * h->g.V * h->link_bytes <= h->l2_bytes ? 3 : kShape8;
+    return grid <= 8 * h->num_sms ? 3 : kShape8Early;
+}
 
 // PLQ: the pass also sums the plaquettes of the planes (MU, nu < MU) of the configuration it leaves
 // (one partial per warp into plaq_part).  Run in the parity-1 passes of MU = 1, 2, 3 of a
@@ -39,25 +74,40 @@ constexpr int update_block() { return 128; }
 // (1/2) Re tr of those plaquettes summed is (U'_MU(x) A_low(x)).c0, for the staple convention of
 // staple_update (U A = the sum of the plaquettes through U); the separate plaquette kernel
 // (plaquette.c:67-100) then need not run.
-template <typename R, int MU, int KIND, bool PLQ = false>
-__global__ void __launch_bounds__(update_block<KIND>(), 1024 / update_block<KIND>()) k_update(Field<R> U, Geom g, int par, R kb, PhiloxKeys seed, uint32_t sweep,
-                                                   const uint32_t* __restrict__ sweep_base, uint32_t replica,
-                                                   double* __restrict__ acc_sum, unsigned* __restrict__ status,
-                                                   DD* __restrict__ plaq_part = nullptr)
+//
+// A pass is a programmatic dependent launch: its CTAs take the slots that the tail of the pass before
+// frees, find their sites, and wait there.  EARLY > 0: they also draw that many trials and the angles
+// before the wait (they need no links), which leaves loads, staple and the end of the draw behind it.
+// One trial is refused in 30, so with one drawn early most passes still end with a warp that draws
+// again (20 FP64 sweeps at 10x12x14x12: 0.81, 0.72, 0.59 ms with one, two, three; 0.82 with none).
+template <typename R, int MU, int KIND, bool PLQ, int CTAS, int EARLY>
+__global__ void __launch_bounds__(kUpdateBlock, CTAS)
+    k_update(Field<R> Unc, Geom g, int par, R kb, PhiloxKeys seed, uint32_t sweep, uint32_t replica, double* __restrict__ acc_sum, unsigned* __restrict__ status, DD* __restrict__ plaq_part)
 {
     // one link per thread; CTAs are dispatched in index order, so the CTAs in flight cover a
     // contiguous window of the lattice and neighbours one t-slice away are still in L2
+    pdl_trigger();
     double acc_thread = 0.0, plaq_thread = 0.0;
-    const int h = blockIdx.x * blockDim.x + threadIdx.x;
+    int h = blockIdx.x * blockDim.x + threadIdx.x;
+    Site s = site_of(g, par, h);
+    const FieldCA<R> U = field_ca(Unc);
+    KpTrial<R> early[EARLY > 0 ? EARLY : 1];
+    KpAngles<R> angles;
+    if (EARLY > 0) {
+#pragma unroll
+        for (int i = 0; i < EARLY; ++i)
+            early[i] = kp_trial<R>(seed, (uint32_t)s.n, sweep, (uint32_t)MU, replica, (uint32_t)i);
+        angles = kp_angles<R>(seed, (uint32_t)s.n, sweep, (uint32_t)MU, replica, 0u);
+    }
+    pdl_wait(h, s.n);
     if (h < g.Vh) {
-        const Site s = site_of(g, par, h);
         Q<R> low;
         const Q<R> A = staple_update<R, MU, PLQ ? MU : 0>(U, g, s, par, PLQ ? &low : nullptr);
         if (KIND == SU2G_HEATBATH) {
-            if (sweep_base) sweep += *sweep_base;
             Q<R> out;
             uint32_t trials = 0;
-            if (heatbath_link<R>(A, kb, seed, (uint32_t)s.n, sweep, (uint32_t)MU, replica, trials, out, status))
+            if (heatbath_link<R, EARLY>(A, kb, seed, (uint32_t)s.n, sweep, (uint32_t)MU, replica, trials, out, status,
+                                        0u, early, angles))
                 U.sth(MU, par, h, hb_store(out));
             if (acc_sum && trials) acc_thread = 1.0 / (double)trials;
         } else {
@@ -75,7 +125,7 @@ __global__ void __launch_bounds__(update_block<KIND>(), 1024 / update_block<KIND
     }
     if (KIND == SU2G_HEATBATH && acc_sum) {
         DD v = {acc_thread, 0.0};
-        v = dd_block_sum<update_block<KIND>()>(v);
+        v = dd_block_sum<kUpdateBlock>(v);
         if (threadIdx.x == 0) atomicAdd(acc_sum, v.s + v.e);
     }
     if (PLQ) {
@@ -84,7 +134,7 @@ __global__ void __launch_bounds__(update_block<KIND>(), 1024 / update_block<KIND
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) plaq_thread += __shfl_xor_sync(0xffffffffu, plaq_thread, o);
         if ((threadIdx.x & 31) == 0)
-            plaq_part[blockIdx.x * (update_block<KIND>() / 32) + (threadIdx.x >> 5)] = DD{plaq_thread, 0.0};
+            plaq_part[blockIdx.x * (kUpdateBlock / 32) + (threadIdx.x >> 5)] = DD{plaq_thread, 0.0};
     }
 }
 
@@ -166,58 +216,74 @@ void launch_visit_r(su2g_lattice* h, int kind, int order, int mu, int par, const
     else launch_visit_t<R, SU2G_METROPOLIS, 0>(h, mu, par, a, acc_sum, grid);
 }
 
+template <typename R, int MU, int KIND, int I>
+void launch_update_i(su2g_lattice* h, int par, uint32_t sweep, double* acc_sum, int grid, DD* plaq_part)
+{
+    if constexpr (shape_used<R, KIND>(I)) {
+        constexpr int ctas = kShapes[I].ctas, early = KIND == SU2G_HEATBATH ? kShapes[I].early : 0;
+        auto* kernel = MU > 0 && plaq_part ? k_update<R, MU, KIND, MU != 0, ctas, early>   // parity-1 passes of MU >= 1 only
+                                           : k_update<R, MU, KIND, false, ctas, early>;
+        launch_pdl(kernel, grid, kUpdateBlock, h->stream, make_field<R>(h->dirp, h->g.Vh), h->g, par, kp_beta<R>(h->beta),
+                   philox_keys(h->seed), sweep, h->replica, acc_sum, h->d_status, plaq_part);
+    }
+}
+
+template <typename R, int MU, int KIND>
+void launch_update_mu(su2g_lattice* h, int par, uint32_t sweep, double* acc_sum, int grid, DD* plaq_part)
+{
+    switch (update_shape<R, KIND>(h, grid)) {
+        case 0: launch_update_i<R, MU, KIND, 0>(h, par, sweep, acc_sum, grid, plaq_part); break;
+        case 1: launch_update_i<R, MU, KIND, 1>(h, par, sweep, acc_sum, grid, plaq_part); break;
+        case 2: launch_update_i<R, MU, KIND, 2>(h, par, sweep, acc_sum, grid, plaq_part); break;
+        case 3: launch_update_i<R, MU, KIND, 3>(h, par, sweep, acc_sum, grid, plaq_part); break;
+        case kShape8Early: launch_update_i<R, MU, KIND, kShape8Early>(h, par, sweep, acc_sum, grid, plaq_part); break;
+        default: launch_update_i<R, MU, KIND, kShape8>(h, par, sweep, acc_sum, grid, plaq_part); break;
+    }
+}
+
 template <typename R, int KIND>
-void launch_update_t(su2g_lattice* h, int mu, int par, uint32_t sweep, const uint32_t* base, double* acc_sum, int grid,
+void launch_update_t(su2g_lattice* h, int mu, int par, uint32_t sweep, double* acc_sum, int grid,
                      DD* plaq_part)
 {
-    Field<R> U = make_field<R>(h->dirp, h->g.Vh);
-    const R kb = kp_beta<R>(h->beta);
-    const int nt = update_block<KIND>();
-    cudaStream_t st = h->stream;
-    const PhiloxKeys keys = philox_keys(h->seed);
-    if (plaq_part) {   // parity-1 passes of MU >= 1 only
-        switch (mu) {
-            case 1: k_update<R, 1, KIND, true><<<grid, nt, 0, st>>>(U, h->g, par, kb, keys, sweep, base, h->replica, acc_sum, h->d_status, plaq_part); break;
-            case 2: k_update<R, 2, KIND, true><<<grid, nt, 0, st>>>(U, h->g, par, kb, keys, sweep, base, h->replica, acc_sum, h->d_status, plaq_part); break;
-            default: k_update<R, 3, KIND, true><<<grid, nt, 0, st>>>(U, h->g, par, kb, keys, sweep, base, h->replica, acc_sum, h->d_status, plaq_part); break;
-        }
-        return;
-    }
     switch (mu) {
-        case 0: k_update<R, 0, KIND><<<grid, nt, 0, st>>>(U, h->g, par, kb, keys, sweep, base, h->replica, acc_sum, h->d_status); break;
-        case 1: k_update<R, 1, KIND><<<grid, nt, 0, st>>>(U, h->g, par, kb, keys, sweep, base, h->replica, acc_sum, h->d_status); break;
-        case 2: k_update<R, 2, KIND><<<grid, nt, 0, st>>>(U, h->g, par, kb, keys, sweep, base, h->replica, acc_sum, h->d_status); break;
-        default: k_update<R, 3, KIND><<<grid, nt, 0, st>>>(U, h->g, par, kb, keys, sweep, base, h->replica, acc_sum, h->d_status); break;
+        case 0: launch_update_mu<R, 0, KIND>(h, par, sweep, acc_sum, grid, plaq_part); break;
+        case 1: launch_update_mu<R, 1, KIND>(h, par, sweep, acc_sum, grid, plaq_part); break;
+        case 2: launch_update_mu<R, 2, KIND>(h, par, sweep, acc_sum, grid, plaq_part); break;
+        default: launch_update_mu<R, 3, KIND>(h, par, sweep, acc_sum, grid, plaq_part); break;
     }
 }
 
 }  // namespace
 
-int su2g::update_grid(const su2g_lattice* h)
+static int update_grid(const su2g_lattice* h)
 {
-    return (int)((h->g.Vh + update_block<SU2G_HEATBATH>() - 1) / update_block<SU2G_HEATBATH>());
+    return (int)((h->g.Vh + kUpdateBlock - 1) / kUpdateBlock);
 }
 
-int su2g::update_plaq_parts(const su2g_lattice* h)
+static int update_plaq_parts(const su2g_lattice* h) { return update_grid(h) * (kUpdateBlock / 32); }
+
+int su2g::sweep_plaq_parts(const su2g_lattice* h) { return 3 * update_plaq_parts(h); }
+
+int su2g::sweep_plaq_finalize(su2g_lattice* h, const DD* parts, int nslots, double* out, int out_stride)
 {
-    return update_grid(h) * (update_block<SU2G_HEATBATH>() / 32);
+    // the partials of the passes (1, 1), (2, 1), (3, 1): 6V plaquettes, (1/2) Re tr each
+    const int n = sweep_plaq_parts(h);
+    return finalize(h, parts, n, nslots, n, 1.0 / (6.0 * (double)h->g.V), out, out_stride);
 }
 
-int su2g::launch_update(su2g_lattice* h, int kind, int mu, int par, uint32_t sweep, double* acc_sum,
-                        const uint32_t* base, DD* plaq_part)
+int su2g::launch_update(su2g_lattice* h, int kind, int mu, int par, uint32_t sweep, double* acc_sum, DD* plaq_part)
 {
-    static_assert(update_block<SU2G_HEATBATH>() == update_block<SU2G_OVERRELAX>(), "one grid for both kinds");
     const int cls = kind == SU2G_HEATBATH ? SU2G_K_HEATBATH : SU2G_K_OVERRELAX;
     const int grid = update_grid(h);
     if (plaq_part && (mu < 1 || par != 1))
         return set_error(h, SU2G_EINVAL, "fused plaquette: only the parity-1 passes of mu >= 1 sum plaquettes");
     launch_begin(h, cls);
     if (h->prec == SU2G_FP32) {
-        if (kind == SU2G_HEATBATH) launch_update_t<float, SU2G_HEATBATH>(h, mu, par, sweep, base, acc_sum, grid, plaq_part);
-        else launch_update_t<float, SU2G_OVERRELAX>(h, mu, par, sweep, base, acc_sum, grid, plaq_part);
+        if (kind == SU2G_HEATBATH) launch_update_t<float, SU2G_HEATBATH>(h, mu, par, sweep, acc_sum, grid, plaq_part);
+        else launch_update_t<float, SU2G_OVERRELAX>(h, mu, par, sweep, acc_sum, grid, plaq_part);
     } else {
-        if (kind == SU2G_HEATBATH) launch_update_t<double, SU2G_HEATBATH>(h, mu, par, sweep, base, acc_sum, grid, plaq_part);
-        else launch_update_t<double, SU2G_OVERRELAX>(h, mu, par, sweep, base, acc_sum, grid, plaq_part);
+        if (kind == SU2G_HEATBATH) launch_update_t<double, SU2G_HEATBATH>(h, mu, par, sweep, acc_sum, grid, plaq_part);
+        else launch_update_t<double, SU2G_OVERRELAX>(h, mu, par, sweep, acc_sum, grid, plaq_part);
     }
     return launch_end(h, cls, kind == SU2G_HEATBATH ? "heatbath pass" : "overrelaxation pass");
 }
@@ -265,30 +331,24 @@ extern "C" int su2g_update_pass(su2g_lattice* h, int32_t kind, int32_t mu, int32
     return launch_update(h, kind, mu, parity, sweep, nullptr);
 }
 
-int su2g::sweep_enqueue(su2g_lattice* h, int n_sweeps, int n_hb, int n_or, uint32_t sweep0, const uint32_t* base,
-                        double* acc_dev, int plaq_off)
+int su2g::sweep_enqueue(su2g_lattice* h, int n_sweeps, int n_hb, int n_or, uint32_t sweep0, double* acc_dev, DD* plaq_part)
 {
     const int parts = update_plaq_parts(h);   // per fused pass
     const int subs = n_sweeps * (n_hb + n_or);
-    int rc = SU2G_OK;
-    if (plaq_off >= 0 && subs > 0 && (rc = ensure_partial_entries(h, 3 * (size_t)parts))) return rc;
     int sub = 0;
     for (int s = 0; s < n_sweeps; ++s)
         for (int i = 0; i < n_hb + n_or; ++i) {
             const bool hb = i < n_hb;
-            const bool last = ++sub == subs && plaq_off >= 0;
+            const bool last = ++sub == subs && plaq_part;
             for (int mu = 0; mu < 4; ++mu)
                 for (int par = 0; par < 2; ++par) {
-                    DD* part = last && mu >= 1 && par == 1 ? h->partials + (size_t)(mu - 1) * parts : nullptr;
-                    rc = hb ? launch_update(h, SU2G_HEATBATH, mu, par, sweep0 + (uint32_t)(s * n_hb + i), acc_dev, base, part)
-                            : launch_update(h, SU2G_OVERRELAX, mu, par, 0u, nullptr, nullptr, part);
+                    DD* part = last && mu >= 1 && par == 1 ? plaq_part + (size_t)(mu - 1) * parts : nullptr;
+                    const int rc = hb ? launch_update(h, SU2G_HEATBATH, mu, par, sweep0 + (uint32_t)(s * n_hb + i), acc_dev, part)
+                                      : launch_update(h, SU2G_OVERRELAX, mu, par, 0u, nullptr, part);
                     if (rc) return rc;
                 }
         }
-    if (plaq_off < 0) return SU2G_OK;
-    if (subs == 0) return plaquette_enqueue(h, plaq_off);
-    // the partials of the passes (1, 1), (2, 1), (3, 1): 6V plaquettes, (1/2) Re tr each
-    return finalize(h, 3 * parts, 1, 1.0 / (6.0 * (double)h->g.V), plaq_off);
+    return SU2G_OK;
 }
 
 namespace {
@@ -307,7 +367,11 @@ int sweep_call(su2g_lattice* h, int32_t n_sweeps, int32_t n_hb, int32_t n_or, do
         if ((rc = check_cuda(h, cudaMemsetAsync(acc_dev, 0, sizeof(double), h->stream), "clearing acceptance")))
             return rc;
     }
-    rc = sweep_enqueue(h, n_sweeps, n_hb, n_or, h->hb_sweeps, nullptr, acc_dev, plaq_out ? slot_plaq : -1);
+    const bool fused = plaq_out && n_sweeps * (n_hb + n_or) > 0;
+    if (fused && (rc = ensure_partial_entries(h, sweep_plaq_parts(h)))) return rc;
+    if ((rc = sweep_enqueue(h, n_sweeps, n_hb, n_or, h->hb_sweeps, acc_dev, fused ? h->partials : nullptr))) return rc;
+    if (fused) rc = sweep_plaq_finalize(h, h->partials, 1, h->d_out + slot_plaq);
+    else if (plaq_out) rc = plaquette_enqueue(h, h->d_out + slot_plaq);
     if (rc) return rc;
     h->hb_sweeps += (uint32_t)(n_sweeps * n_hb);
     if (acc_out || plaq_out) {

@@ -137,12 +137,49 @@ __device__ __forceinline__ Q<R> fallback_link(R r0, R r1, R r2)
 // `draw_base` (visit << kVisitShift) separates the draws of repeated visits in a random-order sweep.
 constexpr int kVisitShift = 21;   // above every trial index (kMaxTrials = 2^20)
 
-// `seed` is the 64-bit seed or its precomputed round keys (PhiloxKeys): the same draws either way; kb is
-// kp_beta<R>(beta).
+// One trial, up to the factor 1/alpha: X1 = -ln(u0)/alpha, X2 = -ln(u1)/alpha, delta = X2 + X1 cos^2(2 pi u2)
+// = -lc / alpha, accepted when u3^2 <= 1 - delta/2  (heatbath.c:86-94).
+template <typename R>
+struct KpTrial {
+    R lc, u3;
+};
+// The direction's angles, cos theta = 1 - 2 a1, phi = 2 pi a0  (heatbath.c:101-107).
+template <typename R>
+struct KpAngles {
+    R sth, cth, sph, cph;
+};
+
+// `seed` is the 64-bit seed or its precomputed round keys (PhiloxKeys): the same draws either way.
 template <typename R, typename Seed>
+__device__ __forceinline__ KpTrial<R> kp_trial(const Seed& seed, uint32_t site, uint32_t sweep, uint32_t mu,
+                                               uint32_t replica, uint32_t draw)
+{
+    const U4 w = link_random(seed, site, sweep, mu, draw, 0u, kStreamUpdate, replica);
+    KpTrial<R> t;
+    t.u3 = u01(w.w, R(0));
+    t.lc = kp_log(w.y, R(0)) + kp_log(w.x, R(0)) * kp_cos2pi_sq(w.z, R(0));
+    return t;
+}
+template <typename R, typename Seed>
+__device__ __forceinline__ KpAngles<R> kp_angles(const Seed& seed, uint32_t site, uint32_t sweep, uint32_t mu,
+                                                 uint32_t replica, uint32_t draw)
+{
+    const U4 w = link_random(seed, site, sweep, mu, draw, 1u, kStreamUpdate, replica);
+    KpAngles<R> a;
+    const R a1 = u01(w.y, R(0));
+    a.cth = R(1) - R(2) * a1;
+    a.sth = R(2) * kp_sqrt(a1 * (R(1) - a1));       // sin(acos(1 - 2 a1))
+    kp_sincos2pi(w.x, &a.sph, &a.cph);
+    return a;
+}
+
+// kb is kp_beta<R>(beta).  With EARLY > 0 that many first trials and the angles were drawn by the caller
+// (draw_base 0), which needs no staple for them.
+template <typename R, int EARLY = 0, typename Seed>
 __device__ __forceinline__ bool heatbath_link(const Q<R>& A, R kb, const Seed& seed, uint32_t site, uint32_t sweep,
                                               uint32_t mu, uint32_t replica, uint32_t& trials, Q<R>& out,
-                                              unsigned* status, uint32_t draw_base = 0u)
+                                              unsigned* status, uint32_t draw_base = 0u,
+                                              const KpTrial<R>* early = nullptr, const KpAngles<R>& angles = {})
 {
     R k, ik, ia;   // |A|, 1/|A|, 1/alpha with alpha = |A| beta (heatbath.c:142)
     kp_norms(q_norm2(A), kb, k, ik, ia);
@@ -154,29 +191,32 @@ __device__ __forceinline__ bool heatbath_link(const Q<R>& A, R kb, const Seed& s
     }
     R delta;
     uint32_t trial = 0;
-    for (;;) {
-        U4 w = link_random(seed, site, sweep, mu, draw_base | trial, 0u, kStreamUpdate, replica);
-        ++trial;
-        const R u3 = u01(w.w, R(0));
-        // X1 = -ln(u0)/alpha, X2 = -ln(u1)/alpha, delta = X2 + X1 cos^2(2 pi u2)  (heatbath.c:86-90)
-        delta = kp_clamp(-(kp_log(w.y, R(0)) + kp_log(w.x, R(0)) * kp_cos2pi_sq(w.z, R(0))) * ia);
-        if (u3 * u3 <= R(1) - R(0.5) * delta) break;   // heatbath.c:94
-        if (trial >= kMaxTrials) {   // the link keeps its value and the host sees the status bit
-            atomicOr(status, kStatusKpTrials);
-            trials = 0;
-            return false;
+    bool taken = false;
+#pragma unroll
+    for (int i = 0; i < EARLY; ++i)
+        if (!taken) {
+            ++trial;
+            delta = kp_clamp(-early[i].lc * ia);
+            taken = early[i].u3 * early[i].u3 <= R(1) - R(0.5) * delta;
+        }
+    if (EARLY == 0 || !taken) {
+        for (;;) {
+            const KpTrial<R> t = kp_trial<R>(seed, site, sweep, mu, replica, draw_base | trial);
+            ++trial;
+            delta = kp_clamp(-t.lc * ia);
+            if (t.u3 * t.u3 <= R(1) - R(0.5) * delta) break;   // heatbath.c:94
+            if (trial >= kMaxTrials) {   // the link keeps its value and the host sees the status bit
+                atomicOr(status, kStatusKpTrials);
+                trials = 0;
+                return false;
+            }
         }
     }
     trials = trial;
     // x0 = 1 - delta; (x1,x2,x3) = sqrt(1-x0^2) (sin th cos ph, sin th sin ph, cos th)  (heatbath.c:96-107)
-    U4 w = link_random(seed, site, sweep, mu, draw_base, 1u, kStreamUpdate, replica);
-    const R a1 = u01(w.y, R(0));
-    const R cth = R(1) - R(2) * a1;
-    const R sth = R(2) * kp_sqrt(a1 * (R(1) - a1));       // sin(acos(1 - 2 a1))
-    R sph, cph;
-    kp_sincos2pi(w.x, &sph, &cph);
+    const KpAngles<R> a = EARLY > 0 ? angles : kp_angles<R>(seed, site, sweep, mu, replica, draw_base);
     const R len = kp_sqrt(delta * (R(2) - delta));          // sqrt(1 - (1-delta)^2)
-    Q<R> X = q_make<R>(R(1) - delta, len * sth * cph, len * sth * sph, len * cth);
+    Q<R> X = q_make<R>(R(1) - delta, len * a.sth * a.cph, len * a.sth * a.sph, len * a.cth);
     // U = X V^dag, V = A/k  (heatbath.c:140-146)
     out = q_mul_nd(X, q_scale(A, ik));
     return true;
