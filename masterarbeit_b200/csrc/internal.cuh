@@ -240,15 +240,19 @@ void wilson_prepare(su2g_lattice* h);
 int wilson_check(su2g_lattice* h, const int32_t* R, const int32_t* T, int n, const char* who);
 // Enqueue the plaquette of the current field into *out (device).
 int plaquette_enqueue(su2g_lattice* h, double* out);
-// One (mu, parity) update pass with heatbath sweep index `sweep`.  With plaq_part (parity-1 passes of
-// mu >= 1 only) the pass also writes one plaquette partial per warp.
-int launch_update(su2g_lattice* h, int kind, int mu, int par, uint32_t sweep, double* acc_sum, DD* plaq_part = nullptr);
-// Partials of the plaquette fused into a sub-sweep (its three passes together), and the reduction
-// that turns nslots sets of them, one after another from `parts`, into out[k * out_stride].
-int sweep_plaq_parts(const su2g_lattice* h);
-int sweep_plaq_finalize(su2g_lattice* h, const DD* parts, int nslots, double* out, int out_stride = 1);
+// One (mu, parity) update pass with heatbath sweep index `sweep`.  With acc_part a heatbath pass adds each
+// warp's sum of 1 / trials to that warp's entry (acc_first: sets it); with plaq_part (parity-1 passes of
+// mu >= 1 only) it also writes one plaquette partial per warp.
+int launch_update(su2g_lattice* h, int kind, int mu, int par, uint32_t sweep, DD* acc_part, bool acc_first, DD* plaq_part);
+// Warps of a pass (entries of acc_part, partials per fused pass), and the reductions that turn nslots
+// sets of entries -- three passes' plaquette partials, or the acceptance's -- `stride` apart, into
+// out[k * out_stride].
+int sweep_warps(const su2g_lattice* h);
+int sweep_plaq_finalize(su2g_lattice* h, const DD* parts, int nslots, size_t stride, double* out, int out_stride = 1);
+int sweep_acc_finalize(su2g_lattice* h, const DD* parts, int nslots, size_t stride, double* out, int out_stride = 1);
 // Enqueue n_sweeps x (n_hb heatbath + n_or overrelaxation sweeps); heatbath sub-sweep j (counted
-// from 0 within the call) has index sweep0 + j.  With plaq_part the last sub-sweep (there must be one)
-// also leaves the partials of the final field's plaquette there.
-int sweep_enqueue(su2g_lattice* h, int n_sweeps, int n_hb, int n_or, uint32_t sweep0, double* acc_dev, DD* plaq_part);
+// from 0 within the call) has index sweep0 + j.  acc_part (there must be a heatbath sub-sweep) receives
+// the acceptance of them all; with plaq_part (there must be a sub-sweep) the last sub-sweep also leaves
+// the three fused passes' plaquette partials there.
+int sweep_enqueue(su2g_lattice* h, int n_sweeps, int n_hb, int n_or, uint32_t sweep0, DD* acc_part, DD* plaq_part);
 }  // namespace su2g

@@ -3,10 +3,10 @@
 // Reference: the driver loop of LGT_Code/main/qcd.c:55-60, gaugefieldUpdate (update.c:102-175)
 // followed by plaquette() (plaquette.c:67-100) after every sweep.  One block is `meas_every`
 // sweeps of (n_hb heatbath + n_or overrelaxation) and the plaquette, summed inside the last
-// sweep's update passes.  All blocks are enqueued without returning to the caller; each accumulates
-// its acceptance in a result slot of its own and leaves its plaquette partials in a region of its
-// own, and one reduction sums the plaquettes of several blocks, so that nothing but update passes runs
-// between one block's sweeps and the next's.
+// sweep's update passes.  All blocks are enqueued without returning to the caller; each
+// leaves the partial sums of its plaquette and acceptance in a region of its own, and one reduction sums
+// those of several blocks, so that nothing but update passes runs between one block's sweeps and
+// the next's.
 //
 // The launches are programmatic dependent ones (k_update), each starting in the tail of the one before.
 // A captured graph of a block, replayed, ran slower on B200: its nodes did not overlap in that way and
@@ -33,28 +33,33 @@ extern "C" int su2g_graph_run(su2g_lattice* h, int32_t n_blocks, int32_t meas_ev
                          meas_every, n_hb, n_or);
     if (n_blocks == 0) return SU2G_OK;
     cudaSetDevice(h->device);
-    const bool fused = n_hb + n_or > 0;
-    const size_t parts = sweep_plaq_parts(h);
+    const bool fused = n_hb + n_or > 0, with_acc = n_hb > 0;
+    const size_t warps = sweep_warps(h), parts = 4 * warps;   // a block's: the plaquette's three passes, the acceptance
     const int group = std::max<int>(1, std::min<size_t>(kFinSlots, kPlaqScratchBytes / (parts * sizeof(DD))));
     int rc = fused ? ensure_partial_entries(h, parts * std::min(group, (int)n_blocks)) : SU2G_OK;
     const double nupd = (double)meas_every * n_hb * 4.0 * (double)h->g.V;
     // as many blocks at a time as there are result slots: slot 2i takes block i's plaquette, 2i + 1 its acceptance
     for (int b0 = 0; b0 < n_blocks && !rc; b0 += kOutSlots / 2) {
         const int n = std::min(n_blocks - b0, kOutSlots / 2);
-        rc = check_cuda(h, cudaMemsetAsync(h->d_out, 0, 2 * sizeof(double) * (size_t)n, h->stream), "clearing acceptance");
         for (int i = 0; i < n && !rc; ++i) {
             const int j = i % group;
-            rc = sweep_enqueue(h, meas_every, n_hb, n_or, h->hb_sweeps, h->d_out + 2 * i + 1,
-                               fused ? h->partials + j * parts : nullptr);
+            DD* part = h->partials + j * parts;
+            rc = sweep_enqueue(h, meas_every, n_hb, n_or, h->hb_sweeps, with_acc ? part + 3 * warps : nullptr,
+                               fused ? part : nullptr);
             h->hb_sweeps += (uint32_t)(meas_every * n_hb);
             if (rc) break;
-            if (!fused) rc = plaquette_enqueue(h, h->d_out + 2 * i);
-            else if (j == group - 1 || i == n - 1) rc = sweep_plaq_finalize(h, h->partials, j + 1, h->d_out + 2 * (i - j), 2);
+            double* out = h->d_out + 2 * (i - j);
+            if (!fused) {
+                rc = plaquette_enqueue(h, h->d_out + 2 * i);
+            } else if (j == group - 1 || i == n - 1) {
+                rc = sweep_plaq_finalize(h, h->partials, j + 1, parts, out, 2);
+                if (!rc && with_acc) rc = sweep_acc_finalize(h, h->partials + 3 * warps, j + 1, parts, out + 1, 2);
+            }
         }
         if (!rc) rc = fetch_results(h, 0, 2 * n);
         for (int i = 0; i < n && !rc; ++i) {
             if (plaq) plaq[b0 + i] = h->h_out[2 * i];
-            if (acc) acc[b0 + i] = nupd > 0 ? h->h_out[2 * i + 1] / nupd : 0.0;
+            if (acc) acc[b0 + i] = with_acc ? h->h_out[2 * i + 1] / nupd : 0.0;
         }
     }
     return rc;

@@ -82,13 +82,16 @@ int update_shape(const su2g_lattice* h, int grid)
 // again (20 FP64 sweeps at 10x12x14x12: 0.81, 0.72, 0.59 ms with one, two, three; 0.82 with none).
 template <typename R, int MU, int KIND, bool PLQ, int CTAS, int EARLY>
 __global__ void __launch_bounds__(kUpdateBlock, CTAS)
-    k_update(Field<R> Unc, Geom g, int par, R kb, PhiloxKeys seed, uint32_t sweep, uint32_t replica, double* __restrict__ acc_sum, unsigned* __restrict__ status, DD* __restrict__ plaq_part)
+    k_update(Field<R> Unc, Geom g, int par, R kb, PhiloxKeys seed, uint32_t sweep, uint32_t replica,
+             DD* acc_part, int acc_first, unsigned* __restrict__ status, DD* __restrict__ plaq_part)
 {
     // one link per thread; CTAs are dispatched in index order, so the CTAs in flight cover a
     // contiguous window of the lattice and neighbours one t-slice away are still in L2
     pdl_trigger();
-    double acc_thread = 0.0, plaq_thread = 0.0;
+    double plaq_thread = 0.0, acc_warp = 0.0;
+    uint32_t trials = 0;
     int h = blockIdx.x * blockDim.x + threadIdx.x;
+    const int warp = blockIdx.x * (kUpdateBlock / 32) + (threadIdx.x >> 5);
     Site s = site_of(g, par, h);
     const FieldCA<R> U = field_ca(Unc);
     KpTrial<R> early[EARLY > 0 ? EARLY : 1];
@@ -100,16 +103,15 @@ __global__ void __launch_bounds__(kUpdateBlock, CTAS)
         angles = kp_angles<R>(seed, (uint32_t)s.n, sweep, (uint32_t)MU, replica, 0u);
     }
     pdl_wait(h, s.n);
+    if (KIND == SU2G_HEATBATH && acc_part && !acc_first) acc_warp = acc_part[warp].s;   // of the passes before
     if (h < g.Vh) {
         Q<R> low;
         const Q<R> A = staple_update<R, MU, PLQ ? MU : 0>(U, g, s, par, PLQ ? &low : nullptr);
         if (KIND == SU2G_HEATBATH) {
             Q<R> out;
-            uint32_t trials = 0;
             if (heatbath_link<R, EARLY>(A, kb, seed, (uint32_t)s.n, sweep, (uint32_t)MU, replica, trials, out, status,
                                         0u, early, angles))
                 U.sth(MU, par, h, hb_store(out));
-            if (acc_sum && trials) acc_thread = 1.0 / (double)trials;
         } else {
             U.sth(MU, par, h, q_project(overrelax_link<R>(A, U.ldh(MU, par, h))));
         }
@@ -123,18 +125,22 @@ __global__ void __launch_bounds__(kUpdateBlock, CTAS)
             plaq_thread = (double)q_mul(Uc.ldh(MU, par, h), low).c0;
         }
     }
-    if (KIND == SU2G_HEATBATH && acc_sum) {
-        DD v = {acc_thread, 0.0};
-        v = dd_block_sum<kUpdateBlock>(v);
-        if (threadIdx.x == 0) atomicAdd(acc_sum, v.s + v.e);
+    // Sums are kept per warp (plain FP64), without a CTA barrier, which would hold the CTA's warps until its
+    // slowest Kennedy-Pendleton lane is done.  (The acceptance summed per CTA and added to one address with
+    // an atomic: the loop of sweeps with plaquette and
+    // acceptance at 24^4 94.5 us a sweep, 91.3 us this way; FP32 61.2 and 58.1.)
+    if (KIND == SU2G_HEATBATH && acc_part) {
+        // the sum of 1 / trials: nearly every lane needed one
+        double a = (double)__popc(__ballot_sync(0xffffffffu, trials == 1u));
+        for (unsigned more = __ballot_sync(0xffffffffu, trials > 1u); more; more &= more - 1u)
+            a += 1.0 / (double)__shfl_sync(0xffffffffu, trials, __ffs(more) - 1);
+        if ((threadIdx.x & 31) == 0) acc_part[warp] = DD{acc_warp + a, 0.0};
     }
     if (PLQ) {
-        // one partial per warp (plain FP64 over its 32 terms), no CTA barrier: a barrier would
-        // hold the CTA's warps until its slowest Kennedy-Pendleton lane is done
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) plaq_thread += __shfl_xor_sync(0xffffffffu, plaq_thread, o);
         if ((threadIdx.x & 31) == 0)
-            plaq_part[blockIdx.x * (kUpdateBlock / 32) + (threadIdx.x >> 5)] = DD{plaq_thread, 0.0};
+            plaq_part[warp] = DD{plaq_thread, 0.0};
     }
 }
 
@@ -217,39 +223,39 @@ void launch_visit_r(su2g_lattice* h, int kind, int order, int mu, int par, const
 }
 
 template <typename R, int MU, int KIND, int I>
-void launch_update_i(su2g_lattice* h, int par, uint32_t sweep, double* acc_sum, int grid, DD* plaq_part)
+void launch_update_i(su2g_lattice* h, int par, uint32_t sweep, DD* acc_part, bool acc_first, int grid, DD* plaq_part)
 {
     if constexpr (shape_used<R, KIND>(I)) {
         constexpr int ctas = kShapes[I].ctas, early = KIND == SU2G_HEATBATH ? kShapes[I].early : 0;
         auto* kernel = MU > 0 && plaq_part ? k_update<R, MU, KIND, MU != 0, ctas, early>   // parity-1 passes of MU >= 1 only
                                            : k_update<R, MU, KIND, false, ctas, early>;
         launch_pdl(kernel, grid, kUpdateBlock, h->stream, make_field<R>(h->dirp, h->g.Vh), h->g, par, kp_beta<R>(h->beta),
-                   philox_keys(h->seed), sweep, h->replica, acc_sum, h->d_status, plaq_part);
+                   philox_keys(h->seed), sweep, h->replica, acc_part, (int)acc_first, h->d_status, plaq_part);
     }
 }
 
 template <typename R, int MU, int KIND>
-void launch_update_mu(su2g_lattice* h, int par, uint32_t sweep, double* acc_sum, int grid, DD* plaq_part)
+void launch_update_mu(su2g_lattice* h, int par, uint32_t sweep, DD* acc_part, bool acc_first, int grid, DD* plaq_part)
 {
     switch (update_shape<R, KIND>(h, grid)) {
-        case 0: launch_update_i<R, MU, KIND, 0>(h, par, sweep, acc_sum, grid, plaq_part); break;
-        case 1: launch_update_i<R, MU, KIND, 1>(h, par, sweep, acc_sum, grid, plaq_part); break;
-        case 2: launch_update_i<R, MU, KIND, 2>(h, par, sweep, acc_sum, grid, plaq_part); break;
-        case 3: launch_update_i<R, MU, KIND, 3>(h, par, sweep, acc_sum, grid, plaq_part); break;
-        case kShape8Early: launch_update_i<R, MU, KIND, kShape8Early>(h, par, sweep, acc_sum, grid, plaq_part); break;
-        default: launch_update_i<R, MU, KIND, kShape8>(h, par, sweep, acc_sum, grid, plaq_part); break;
+        case 0: launch_update_i<R, MU, KIND, 0>(h, par, sweep, acc_part, acc_first, grid, plaq_part); break;
+        case 1: launch_update_i<R, MU, KIND, 1>(h, par, sweep, acc_part, acc_first, grid, plaq_part); break;
+        case 2: launch_update_i<R, MU, KIND, 2>(h, par, sweep, acc_part, acc_first, grid, plaq_part); break;
+        case 3: launch_update_i<R, MU, KIND, 3>(h, par, sweep, acc_part, acc_first, grid, plaq_part); break;
+        case kShape8Early: launch_update_i<R, MU, KIND, kShape8Early>(h, par, sweep, acc_part, acc_first, grid, plaq_part); break;
+        default: launch_update_i<R, MU, KIND, kShape8>(h, par, sweep, acc_part, acc_first, grid, plaq_part); break;
     }
 }
 
 template <typename R, int KIND>
-void launch_update_t(su2g_lattice* h, int mu, int par, uint32_t sweep, double* acc_sum, int grid,
+void launch_update_t(su2g_lattice* h, int mu, int par, uint32_t sweep, DD* acc_part, bool acc_first, int grid,
                      DD* plaq_part)
 {
     switch (mu) {
-        case 0: launch_update_mu<R, 0, KIND>(h, par, sweep, acc_sum, grid, plaq_part); break;
-        case 1: launch_update_mu<R, 1, KIND>(h, par, sweep, acc_sum, grid, plaq_part); break;
-        case 2: launch_update_mu<R, 2, KIND>(h, par, sweep, acc_sum, grid, plaq_part); break;
-        default: launch_update_mu<R, 3, KIND>(h, par, sweep, acc_sum, grid, plaq_part); break;
+        case 0: launch_update_mu<R, 0, KIND>(h, par, sweep, acc_part, acc_first, grid, plaq_part); break;
+        case 1: launch_update_mu<R, 1, KIND>(h, par, sweep, acc_part, acc_first, grid, plaq_part); break;
+        case 2: launch_update_mu<R, 2, KIND>(h, par, sweep, acc_part, acc_first, grid, plaq_part); break;
+        default: launch_update_mu<R, 3, KIND>(h, par, sweep, acc_part, acc_first, grid, plaq_part); break;
     }
 }
 
@@ -260,18 +266,21 @@ static int update_grid(const su2g_lattice* h)
     return (int)((h->g.Vh + kUpdateBlock - 1) / kUpdateBlock);
 }
 
-static int update_plaq_parts(const su2g_lattice* h) { return update_grid(h) * (kUpdateBlock / 32); }
+int su2g::sweep_warps(const su2g_lattice* h) { return update_grid(h) * (kUpdateBlock / 32); }
 
-int su2g::sweep_plaq_parts(const su2g_lattice* h) { return 3 * update_plaq_parts(h); }
-
-int su2g::sweep_plaq_finalize(su2g_lattice* h, const DD* parts, int nslots, double* out, int out_stride)
+int su2g::sweep_plaq_finalize(su2g_lattice* h, const DD* parts, int nslots, size_t stride, double* out, int out_stride)
 {
     // the partials of the passes (1, 1), (2, 1), (3, 1): 6V plaquettes, (1/2) Re tr each
-    const int n = sweep_plaq_parts(h);
-    return finalize(h, parts, n, nslots, n, 1.0 / (6.0 * (double)h->g.V), out, out_stride);
+    return finalize(h, parts, 3 * sweep_warps(h), nslots, stride, 1.0 / (6.0 * (double)h->g.V), out, out_stride);
 }
 
-int su2g::launch_update(su2g_lattice* h, int kind, int mu, int par, uint32_t sweep, double* acc_sum, DD* plaq_part)
+int su2g::sweep_acc_finalize(su2g_lattice* h, const DD* parts, int nslots, size_t stride, double* out, int out_stride)
+{
+    return finalize(h, parts, sweep_warps(h), nslots, stride, 1.0, out, out_stride);
+}
+
+int su2g::launch_update(su2g_lattice* h, int kind, int mu, int par, uint32_t sweep, DD* acc_part, bool acc_first,
+                        DD* plaq_part)
 {
     const int cls = kind == SU2G_HEATBATH ? SU2G_K_HEATBATH : SU2G_K_OVERRELAX;
     const int grid = update_grid(h);
@@ -279,11 +288,11 @@ int su2g::launch_update(su2g_lattice* h, int kind, int mu, int par, uint32_t swe
         return set_error(h, SU2G_EINVAL, "fused plaquette: only the parity-1 passes of mu >= 1 sum plaquettes");
     launch_begin(h, cls);
     if (h->prec == SU2G_FP32) {
-        if (kind == SU2G_HEATBATH) launch_update_t<float, SU2G_HEATBATH>(h, mu, par, sweep, acc_sum, grid, plaq_part);
-        else launch_update_t<float, SU2G_OVERRELAX>(h, mu, par, sweep, acc_sum, grid, plaq_part);
+        if (kind == SU2G_HEATBATH) launch_update_t<float, SU2G_HEATBATH>(h, mu, par, sweep, acc_part, acc_first, grid, plaq_part);
+        else launch_update_t<float, SU2G_OVERRELAX>(h, mu, par, sweep, acc_part, acc_first, grid, plaq_part);
     } else {
-        if (kind == SU2G_HEATBATH) launch_update_t<double, SU2G_HEATBATH>(h, mu, par, sweep, acc_sum, grid, plaq_part);
-        else launch_update_t<double, SU2G_OVERRELAX>(h, mu, par, sweep, acc_sum, grid, plaq_part);
+        if (kind == SU2G_HEATBATH) launch_update_t<double, SU2G_HEATBATH>(h, mu, par, sweep, acc_part, acc_first, grid, plaq_part);
+        else launch_update_t<double, SU2G_OVERRELAX>(h, mu, par, sweep, acc_part, acc_first, grid, plaq_part);
     }
     return launch_end(h, cls, kind == SU2G_HEATBATH ? "heatbath pass" : "overrelaxation pass");
 }
@@ -328,12 +337,12 @@ extern "C" int su2g_update_pass(su2g_lattice* h, int32_t kind, int32_t mu, int32
     if ((kind != SU2G_HEATBATH && kind != SU2G_OVERRELAX) || mu < 0 || mu > 3 || (parity != 0 && parity != 1))
         return set_error(h, SU2G_EINVAL, "su2g_update_pass: bad kind/mu/parity (%d, %d, %d)", kind, mu, parity);
     cudaSetDevice(h->device);
-    return launch_update(h, kind, mu, parity, sweep, nullptr);
+    return launch_update(h, kind, mu, parity, sweep, nullptr, false, nullptr);
 }
 
-int su2g::sweep_enqueue(su2g_lattice* h, int n_sweeps, int n_hb, int n_or, uint32_t sweep0, double* acc_dev, DD* plaq_part)
+int su2g::sweep_enqueue(su2g_lattice* h, int n_sweeps, int n_hb, int n_or, uint32_t sweep0, DD* acc_part, DD* plaq_part)
 {
-    const int parts = update_plaq_parts(h);   // per fused pass
+    const int parts = sweep_warps(h);   // per fused pass
     const int subs = n_sweeps * (n_hb + n_or);
     int sub = 0;
     for (int s = 0; s < n_sweeps; ++s)
@@ -343,8 +352,10 @@ int su2g::sweep_enqueue(su2g_lattice* h, int n_sweeps, int n_hb, int n_or, uint3
             for (int mu = 0; mu < 4; ++mu)
                 for (int par = 0; par < 2; ++par) {
                     DD* part = last && mu >= 1 && par == 1 ? plaq_part + (size_t)(mu - 1) * parts : nullptr;
-                    const int rc = hb ? launch_update(h, SU2G_HEATBATH, mu, par, sweep0 + (uint32_t)(s * n_hb + i), acc_dev, part)
-                                      : launch_update(h, SU2G_OVERRELAX, mu, par, 0u, nullptr, part);
+                    const bool first = s == 0 && i == 0 && mu == 0 && par == 0;
+                    const int rc = hb ? launch_update(h, SU2G_HEATBATH, mu, par, sweep0 + (uint32_t)(s * n_hb + i), acc_part,
+                                                      first, part)
+                                      : launch_update(h, SU2G_OVERRELAX, mu, par, 0u, nullptr, false, part);
                     if (rc) return rc;
                 }
         }
@@ -359,25 +370,23 @@ int sweep_call(su2g_lattice* h, int32_t n_sweeps, int32_t n_hb, int32_t n_or, do
     if (!h) return set_error(nullptr, SU2G_EINVAL, "%s: null handle", who);
     if (n_sweeps < 0 || n_hb < 0 || n_or < 0) return set_error(h, SU2G_EINVAL, "%s: negative count", who);
     cudaSetDevice(h->device);
-    double* acc_dev = nullptr;
     const int slot_acc = 0, slot_plaq = 1;
-    int rc = SU2G_OK;
-    if (acc_out) {
-        acc_dev = h->d_out + slot_acc;
-        if ((rc = check_cuda(h, cudaMemsetAsync(acc_dev, 0, sizeof(double), h->stream), "clearing acceptance")))
-            return rc;
-    }
-    const bool fused = plaq_out && n_sweeps * (n_hb + n_or) > 0;
-    if (fused && (rc = ensure_partial_entries(h, sweep_plaq_parts(h)))) return rc;
-    if ((rc = sweep_enqueue(h, n_sweeps, n_hb, n_or, h->hb_sweeps, acc_dev, fused ? h->partials : nullptr))) return rc;
-    if (fused) rc = sweep_plaq_finalize(h, h->partials, 1, h->d_out + slot_plaq);
+    const size_t warps = sweep_warps(h);
+    const bool fused = plaq_out && n_sweeps * (n_hb + n_or) > 0, acc = acc_out && n_sweeps * n_hb > 0;
+    int rc = fused || acc ? ensure_partial_entries(h, 4 * warps) : SU2G_OK;
+    if (rc) return rc;
+    // partials: three passes of the plaquette, then the acceptance
+    DD *part = fused ? h->partials : nullptr, *acc_part = acc ? h->partials + 3 * warps : nullptr;
+    if ((rc = sweep_enqueue(h, n_sweeps, n_hb, n_or, h->hb_sweeps, acc_part, part))) return rc;
+    if (fused) rc = sweep_plaq_finalize(h, part, 1, 0, h->d_out + slot_plaq);
     else if (plaq_out) rc = plaquette_enqueue(h, h->d_out + slot_plaq);
+    if (!rc && acc) rc = sweep_acc_finalize(h, acc_part, 1, 0, h->d_out + slot_acc);
     if (rc) return rc;
     h->hb_sweeps += (uint32_t)(n_sweeps * n_hb);
     if (acc_out || plaq_out) {
         if ((rc = fetch_results(h, slot_acc, 2))) return rc;
         const double nupd = (double)n_sweeps * n_hb * 4.0 * (double)h->g.V;
-        if (acc_out) *acc_out = nupd > 0 ? h->h_out[slot_acc] / nupd : 0.0;
+        if (acc_out) *acc_out = acc ? h->h_out[slot_acc] / nupd : 0.0;
         if (plaq_out) *plaq_out = h->h_out[slot_plaq];
     }
     return SU2G_OK;
