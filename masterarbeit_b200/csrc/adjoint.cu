@@ -62,13 +62,13 @@ __host__ __device__ constexpr bool plane_first(int d, int v) { return clover_pla
 // the loop below runs the other way round and enters with the opposite sign, as does every loop of a
 // plane whose first direction is v.
 template <typename R, int D>
-__device__ __forceinline__ Q<R> line_gradient(const Field<R>& L, const R* __restrict__ fbar, const Geom& g,
+__device__ __forceinline__ Q<R> line_gradient(const FieldCA<R>& L, const R* fbar, const Geom& g,
                                               const Site& s, int par, int h, int e)
 {
     const int q1 = par ^ (e & 1);   // parity one segment away
     const int upD = shift_by(g, D, s.c[D], e);
     const auto F = [&](int p, int pr, int n) {
-        return ldq(fbar, (size_t)p * g.V + (unsigned)(pr * g.Vh + (int)((unsigned)n >> 1)));
+        return ldq_ca(fbar, (size_t)p * g.V + (unsigned)(pr * g.Vh + (int)((unsigned)n >> 1)));
     };
     Q<R> acc = q_zero<R>();
 #pragma unroll
@@ -104,13 +104,17 @@ constexpr int kLineBlock = 128;
 
 template <typename R>
 __global__ void __launch_bounds__(kLineBlock) k_line_gradient(Field<R> U, Field<R> L2, Field<R> L3, Field<R> T1, Field<R> T2,
-                                                              Field<R> T3, Geom g, const R* __restrict__ fbar)
+                                                              Field<R> T3, Geom g, const R* fbar)
 {
+    pdl_trigger();
     const int job = blockIdx.x % 12, D = job & 3, e = 1 + (job >> 2);
-    Site s;
+    Site s{};
     int par, h;
-    if (!site_warp_pair(g, blockIdx.x / 12, threadIdx.x, blockDim.x, s, par, h)) return;
-    Field<R> L, T;
+    const bool valid = site_warp_pair(g, blockIdx.x / 12, threadIdx.x, blockDim.x, s, par, h);
+    pdl_wait(h, s.n);
+    if (!valid) return;
+    FieldCA<R> L;
+    Field<R> T;
     L.Vh = T.Vh = g.Vh;
 #pragma unroll
     for (int d = 0; d < 4; ++d) {
@@ -131,12 +135,16 @@ __global__ void __launch_bounds__(kLineBlock) k_line_gradient(Field<R> U, Field<
 //   T1(x) + [T2(x) + U(x-D)^dag T3(x-D)] U(x+D)^dag + U(x-D)^dag T2(x-D)
 //   + T3(x) L2(x+D)^dag + L2(x-2D)^dag T3(x-2D).
 template <typename R>
-__global__ void __launch_bounds__(kBlock) k_line_chain(Field<R> U, Field<R> L2, Field<R> T1, Field<R> T2, Field<R> T3,
+__global__ void __launch_bounds__(kBlock) k_line_chain(Field<R> Unc, Field<R> L2nc, Field<R> T1nc, Field<R> T2nc, Field<R> T3nc,
                                                        Field<R> G, Geom g)
 {
-    Site s;
+    pdl_trigger();
+    Site s{};
     int par, h;
-    if (!site_warp_pair(g, blockIdx.x, threadIdx.x, blockDim.x, s, par, h)) return;
+    const bool valid = site_warp_pair(g, blockIdx.x, threadIdx.x, blockDim.x, s, par, h);
+    pdl_wait(h, s.n);
+    if (!valid) return;
+    const FieldCA<R> U = field_ca(Unc), L2 = field_ca(L2nc), T1 = field_ca(T1nc), T2 = field_ca(T2nc), T3 = field_ca(T3nc);
     const int q = par ^ 1;
 #pragma unroll
     for (int D = 0; D < 4; ++D) {
@@ -157,12 +165,16 @@ __global__ void __launch_bounds__(kBlock) k_line_chain(Field<R> U, Field<R> L2, 
 // The staple sums are the forward step's own (ape_staples), so v is exactly the forward's
 // pre-projection link; same site order and occupancy as the forward kernel.
 template <typename R>
-__global__ void __launch_bounds__(kBlock, 2) k_ape_vbar(Field<R> U, Field<R> Gn, Field<R> Vbar, Geom g, R alpha)
+__global__ void __launch_bounds__(kBlock, 2) k_ape_vbar(Field<R> U, Field<R> Gnc, Field<R> Vbar, Geom g, R alpha)
 {
-    Site s;
+    pdl_trigger();
+    Site s{};
     int par, h;
-    if (!site_warp_pair(g, blockIdx.x, threadIdx.x, blockDim.x, s, par, h)) return;
-    ape_staples<R, SU2G_APE_ALL>(U, g, s, par, h, [&](int mu, const Q<R>& u, const Q<R>& S) {
+    const bool valid = site_warp_pair(g, blockIdx.x, threadIdx.x, blockDim.x, s, par, h);
+    pdl_wait(h, s.n);
+    if (!valid) return;
+    const FieldCA<R> Gn = field_ca(Gnc);
+    ape_staples<R, SU2G_APE_ALL>(field_ca(U), g, s, par, h, [&](int mu, const Q<R>& u, const Q<R>& S) {
         const Q<R> v = q_axpy(alpha, S, u);
         const R inv = rsqrt_r(q_norm2(v));
         const Q<R> up = q_scale(v, inv);
@@ -180,7 +192,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_ape_vbar(Field<R> U, Field<R> Gn,
 //  for nu != l:  U_nu(y-nu)^dag vbar(y-nu,l) U_nu(y-nu+l)    (middle, upper staple of (y-nu, l))
 //                U_nu(y) vbar(y+nu,l) U_nu(y+l)^dag          (middle, lower staple of (y+nu, l))
 template <typename R, int L>
-__device__ __forceinline__ void gather_link(const Field<R>& U, const Field<R>& Vb, const Field<R>& G, const Geom& g,
+__device__ __forceinline__ void gather_link(const FieldCA<R>& U, const FieldCA<R>& Vb, const Field<R>& G, const Geom& g,
                                             const Site& s, int par, int h, R alpha)
 {
     const int q = par ^ 1;
@@ -221,11 +233,15 @@ __device__ __forceinline__ void gather_link(const Field<R>& U, const Field<R>& V
 // of the same 32 half-volume indices (site_warp_pair): every warp reads consecutive links of one
 // parity array, and both parities of a region are loaded by the same SM.
 template <typename R>
-__global__ void __launch_bounds__(kBlock) k_ape_gather(Field<R> U, Field<R> Vb, Field<R> G, Geom g, R alpha)
+__global__ void __launch_bounds__(kBlock) k_ape_gather(Field<R> Unc, Field<R> Vbnc, Field<R> G, Geom g, R alpha)
 {
-    Site s;
+    pdl_trigger();
+    Site s{};
     int par, h;
-    if (!site_warp_pair(g, blockIdx.x, threadIdx.x, blockDim.x, s, par, h)) return;
+    const bool valid = site_warp_pair(g, blockIdx.x, threadIdx.x, blockDim.x, s, par, h);
+    pdl_wait(h, s.n);
+    if (!valid) return;
+    const FieldCA<R> U = field_ca(Unc), Vb = field_ca(Vbnc);
     switch (blockIdx.y) {
         case 0: gather_link<R, 0>(U, Vb, G, g, s, par, h, alpha); break;
         case 1: gather_link<R, 1>(U, Vb, G, g, s, par, h, alpha); break;
@@ -236,13 +252,14 @@ __global__ void __launch_bounds__(kBlock) k_ape_gather(Field<R> U, Field<R> Vb, 
 
 // su(2) gradient g = vec(G U^dag) per link, written in the reference's site-major order [n][mu][3].
 template <typename R>
-__global__ void __launch_bounds__(kBlock) k_grad_out(Field<R> G, Field<R> U, Geom g, double* __restrict__ out)
+__global__ void __launch_bounds__(kBlock) k_grad_out(Field<R> Gnc, Field<R> Unc, Geom g, double* __restrict__ out)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    int par, h = i >> 1;
+    Site s = site_lex(g, i, par);
+    pdl_wait(h, s.n);
     if (i >= g.V) return;
-    int par;
-    const Site s = site_lex(g, i, par);
-    const int h = i >> 1;
+    const FieldCA<R> G = field_ca(Gnc), U = field_ca(Unc);
 #pragma unroll
     for (int mu = 0; mu < 4; ++mu) {
         const Q<R> v = q_mul_nd(G.ldh(mu, par, h), U.ldh(mu, par, h));
@@ -350,8 +367,8 @@ int vjp_t(su2g_lattice* h, int n_ape, double alpha, int c, double* q_out, double
                    T3 = make_field<R>(tmp[n_ape & 1].dirs, g.Vh);
     const int lblocks = (int)((g.V + kLineBlock - 1) / kLineBlock);
     launch_begin(h, SU2G_K_OTHER);
-    k_line_gradient<R><<<12 * lblocks, kLineBlock, 0, h->stream>>>(UN, L2, L3, T1, T2, T3, g, fbar);
-    k_line_chain<R><<<grid, kBlock, 0, h->stream>>>(UN, L2, T1, T2, T3, make_field<R>(G[0].dirs, g.Vh), g);
+    launch_pdl(k_line_gradient<R>, 12 * lblocks, kLineBlock, h->stream, UN, L2, L3, T1, T2, T3, g, fbar);
+    launch_pdl(k_line_chain<R>, grid, kBlock, h->stream, UN, L2, T1, T2, T3, make_field<R>(G[0].dirs, g.Vh), g);
     if ((rc = launch_end(h, SU2G_K_OTHER, "charge adjoint kernels"))) return rc;
     // backwards through the smearing, one checkpoint segment at a time
     int gi = 0;
@@ -368,17 +385,17 @@ int vjp_t(su2g_lattice* h, int n_ape, double alpha, int c, double* q_out, double
             Field<R> Gn = make_field<R>(G[gi].dirs, g.Vh), Gk = make_field<R>(G[gi ^ 1].dirs, g.Vh);
             Field<R> Vbf = make_field<R>(Vb.dirs, g.Vh);
             launch_begin(h, SU2G_K_OTHER);
-            k_ape_vbar<R><<<2 * (int)((g.Vh + kBlock - 1) / kBlock), kBlock, 0, h->stream>>>(Uk, Gn, Vbf, g, (R)alpha);
-            k_ape_gather<R><<<dim3(2 * (int)((g.Vh + kBlock - 1) / kBlock), 4), kBlock, 0, h->stream>>>(Uk, Vbf, Gk, g,
-                                                                                                      (R)alpha);
+            const int blocks = 2 * (int)((g.Vh + kBlock - 1) / kBlock);
+            launch_pdl(k_ape_vbar<R>, blocks, kBlock, h->stream, Uk, Gn, Vbf, g, (R)alpha);
+            launch_pdl(k_ape_gather<R>, dim3(blocks, 4), kBlock, h->stream, Uk, Vbf, Gk, g, (R)alpha);
             if ((rc = launch_end(h, SU2G_K_OTHER, "smearing adjoint kernels"))) return rc;
             gi ^= 1;
         }
     }
     if (grad_host) {
         launch_begin(h, SU2G_K_OTHER);
-        k_grad_out<R><<<grid, kBlock, 0, h->stream>>>(make_field<R>(G[gi].dirs, g.Vh), make_field<R>(ck[0].dirs, g.Vh),
-                                                      g, gout);
+        launch_pdl(k_grad_out<R>, grid, kBlock, h->stream, make_field<R>(G[gi].dirs, g.Vh), make_field<R>(ck[0].dirs, g.Vh), g,
+                   gout);
         if ((rc = launch_end(h, SU2G_K_OTHER, "gradient output"))) return rc;
         if ((rc = check_cuda(h, cudaMemcpyAsync(grad_host, gout, (size_t)g.V * 12 * sizeof(double),
                                                 cudaMemcpyDeviceToHost, h->stream), "copying the gradient")))

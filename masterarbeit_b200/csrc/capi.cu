@@ -474,7 +474,6 @@ extern "C" int su2g_destroy(su2g_lattice* h)
     for (auto e : h->event_pool) cudaEventDestroy(e);
     if (h->ev_begin) cudaEventDestroy(h->ev_begin);
     if (h->ev_end) cudaEventDestroy(h->ev_end);
-    release_meas_graph(h);
     if (h->pool) cudaMemPoolDestroy(h->pool);
     cudaFree(h->lines);
     cudaFree(h->meas_work);

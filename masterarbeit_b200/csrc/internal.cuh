@@ -101,8 +101,6 @@ __device__ __forceinline__ DD dd_block_sum(DD v)
 
 }  // namespace su2g
 
-struct su2g_meas_graph;   // measure.cu
-
 struct su2g_lattice {
     su2g::Geom g;
     int prec = SU2G_FP32;
@@ -136,9 +134,8 @@ struct su2g_lattice {
     size_t l2_bytes = 0;
     int ape_variant = 0;         // 0: per-site APE kernel, 1: TMA-tiled FP32 APE_all where it applies
     cudaMemPool_t pool = nullptr;      // scratch of the adjoint; keeps its memory until destroy
-    su2g_meas_graph* meas = nullptr;   // graph of one su2g_measure spec
     void* lines = nullptr;             // 2- and 3-link line products of the field Q is measured on
-    void* meas_work = nullptr;         // measurement copy of the field and its ping-pong partner
+    void* meas_work = nullptr;         // the measurement's smeared field and its ping-pong partner
     void* meas_alt = nullptr;
     bool profiling = false;
     struct Prof {
@@ -171,11 +168,12 @@ int launch_end(su2g_lattice* h, int cls, const char* what);
 
 // Launch a kernel that calls pdl_wait: it may start before the launch ahead of it in the stream has ended.
 template <typename... Params, typename... Args>
-inline void launch_pdl(void (*kernel)(Params...), dim3 grid, int block, cudaStream_t stream, Args&&... args)
+inline void launch_pdl_smem(void (*kernel)(Params...), dim3 grid, int block, size_t smem, cudaStream_t stream, Args&&... args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -183,6 +181,11 @@ inline void launch_pdl(void (*kernel)(Params...), dim3 grid, int block, cudaStre
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);   // the caller checks cudaGetLastError
+}
+template <typename... Params, typename... Args>
+inline void launch_pdl(void (*kernel)(Params...), dim3 grid, int block, cudaStream_t stream, Args&&... args)
+{
+    launch_pdl_smem(kernel, grid, block, 0, stream, std::forward<Args>(args)...);
 }
 
 // Make sure the partial-sum scratch holds `slots` x kMaxPartials entries (or at least n entries).
@@ -227,8 +230,6 @@ int field_to_aos(su2g_lattice* h, double* d_dst, size_t n0, int count);
 // {mean, tau_int, naive error, error} per series, d_resolved 100 tau <= n (stats.cu).
 int tau_int_enqueue(const double* d_x, long long n, long long si, long long ss, int n_series, cudaStream_t stream,
                     double* d_out, int* d_resolved);
-// Destroy the captured su2g_measure graph, if any.
-void release_meas_graph(su2g_lattice* h);
 // Enqueue W(R[i], T[i]) of the field at dirs.  Loops are measured in chunks of R and T; each
 // chunk's results land in consecutive d_out slots from out_off on, and slot[i] receives the d_out
 // index of pair i.  Fails (nothing enqueued) if the pairs need more than `max_slots` slots.

@@ -26,12 +26,16 @@ constexpr double kPi = 3.14159265358979323846;
 // Eight 128-thread CTAs per SM: at 48^4 on B200, 182 against 189 us (FP64) and 103 against 106.5 us
 // (FP32) with four CTAs of 256 threads.
 template <typename R>
-__global__ void __launch_bounds__(128, 8) k_plaquette(Field<R> U, Geom g, DD* __restrict__ partials)
+__global__ void __launch_bounds__(128, 8) k_plaquette(Field<R> Unc, Geom g, DD* __restrict__ partials)
 {
+    pdl_trigger();
     double site = 0.0;
-    Site s;
+    Site s{};
     int par, h;
-    if (site_cta_pair(g, blockIdx.x, threadIdx.x, blockDim.x, s, par, h)) {
+    const bool valid = site_cta_pair(g, blockIdx.x, threadIdx.x, blockDim.x, s, par, h);
+    pdl_wait(h, s.n);
+    if (valid) {
+        const FieldCA<R> U = field_ca(Unc);
         const int q = par ^ 1;
         Q<R> u[4];
         int xp[4];
@@ -76,16 +80,34 @@ constexpr int ape_block()
     return 128;
 }
 
-template <typename R, int MODE>
+// With PDL a step is a programmatic dependent launch (pdl_wait): the CTAs of the next step take the slots
+// that the tail of this one frees (ten steps, us, 24x14x18x22: FP64 all 166 -> 141, spatial 105 -> 84; FP32
+// 24^4 all 185 -> 162, spatial 116 -> 94; 48^4 within 2 %).  Its links are stored together at the end: with
+// plain loads, a store between them keeps the later ones behind it (FP32 all at 24^4 190 -> 169 us).  Only
+// FP32 APE_all at sizes whose two fields exceed L2 is faster without, its loads through the read-only
+// path (48^4 264 against 276 us a step; equal at 36^4).
+template <typename R, int MODE, bool PDL>
 __global__ void __launch_bounds__(ape_block<R, MODE>(), ape_min_blocks<R, MODE>()) k_ape(Field<R> in, Field<R> out,
                                                                                         Geom g, R alpha)
 {
     // one site per thread; CTAs dispatched in order, warps alternating parity over the same h run
     // (so that both parities of a region share an L1: FP32 APE_all 237.8 against 240.7 us, spatial
     // 129.1 against 131.6 us, FP64 spatial 355 against 367 us with parity-alternating CTAs)
-    Site s;
+    Site s{};
     int par, h;
-    if (site_warp_pair(g, blockIdx.x, threadIdx.x, blockDim.x, s, par, h)) {
+    if (PDL) pdl_trigger();
+    const bool valid = site_warp_pair(g, blockIdx.x, threadIdx.x, blockDim.x, s, par, h);
+    if (PDL) pdl_wait(h, s.n);
+    if (!valid) return;
+    if (PDL) {
+        Q<R> res[4];
+        ape_staples<R, MODE>(field_ca(in), g, s, par, h, [&](int mu, const Q<R>& u, const Q<R>& S) {
+            res[mu] = q_project(q_axpy(alpha, S, u));
+        });
+#pragma unroll
+        for (int mu = 0; mu < 4; ++mu)
+            if (ape_updates(MODE, mu)) out.sth(mu, par, h, res[mu]);
+    } else {
         ape_staples<R, MODE>(in, g, s, par, h, [&](int mu, const Q<R>& u, const Q<R>& S) {
             out.sth(mu, par, h, q_project(q_axpy(alpha, S, u)));
         });
@@ -375,11 +397,15 @@ size_t wilson_col_smem(int threads, int nT)
 // leaves of size e are then products of four e-link segments, each one line (computeLine,
 // topologicalcharge.c:18-44, evaluated once per segment and site instead of once per leaf).
 template <typename R>
-__global__ void __launch_bounds__(kBlock) k_lines(Field<R> U, Field<R> L2, Field<R> L3, Geom g)
+__global__ void __launch_bounds__(kBlock) k_lines(Field<R> Unc, Field<R> L2, Field<R> L3, Geom g)
 {
-    Site s;
+    pdl_trigger();
+    Site s{};
     int par, h;
-    if (!site_cta_pair(g, blockIdx.x, threadIdx.x, blockDim.x, s, par, h)) return;
+    const bool valid = site_cta_pair(g, blockIdx.x, threadIdx.x, blockDim.x, s, par, h);
+    pdl_wait(h, s.n);
+    if (!valid) return;
+    const FieldCA<R> U = field_ca(Unc);
 #pragma unroll
     for (int D = 0; D < 4; ++D) {
         int c = s.c[D] + 1;
@@ -409,7 +435,7 @@ __global__ void __launch_bounds__(kBlock) k_lines(Field<R> U, Field<R> L2, Field
 // : ten products per plane and size, two of them without their scalar component, instead of twelve.
 // The two planes share the sizes' loop and its periodic offsets (24 a call instead of 12 a plane).
 template <typename R, int P0>
-__device__ __forceinline__ void clover_F_lines(const Field<R>& U, const Field<R>& L2, const Field<R>& L3, const Geom& g,
+__device__ __forceinline__ void clover_F_lines(const FieldCA<R>& U, const FieldCA<R>& L2, const FieldCA<R>& L3, const Geom& g,
                                                const Site& s, int par, int h, Q<R> (&F)[2])
 {
 #pragma unroll
@@ -417,7 +443,7 @@ __device__ __forceinline__ void clover_F_lines(const Field<R>& U, const Field<R>
 #pragma unroll 1
     for (int e = 1; e <= 3; ++e) {
         // the directions' e-link lines (pointers selected in registers, not a field by reference)
-        Field<R> L;
+        FieldCA<R> L;
         L.Vh = U.Vh;
         int up[4], dn[4];
 #pragma unroll
@@ -450,7 +476,7 @@ __device__ __forceinline__ void clover_F_lines(const Field<R>& U, const Field<R>
 // of both planes go to fbar, element
 // plane V + parity Vh + h (c0(F_a F_b) = -<F_a, F_b> for pure F).
 template <typename R, int P0, bool FBAR>
-__device__ __forceinline__ double qtop_product(const Field<R>& U, const Field<R>& L2, const Field<R>& L3, const Geom& g,
+__device__ __forceinline__ double qtop_product(const FieldCA<R>& U, const FieldCA<R>& L2, const FieldCA<R>& L3, const Geom& g,
                                                const Site& s, int par, int h, R* __restrict__ fbar)
 {
     Q<R> F[2];
@@ -474,13 +500,17 @@ __device__ __forceinline__ double qtop_product(const Field<R>& U, const Field<R>
 constexpr int kQtopBlock = 128;
 
 template <typename R, bool FBAR>
-__global__ void __launch_bounds__(kQtopBlock, sizeof(R) == 4 ? 5 : 3) k_qtop(Field<R> U, Field<R> L2, Field<R> L3, Geom g,
+__global__ void __launch_bounds__(kQtopBlock, sizeof(R) == 4 ? 5 : 3) k_qtop(Field<R> Unc, Field<R> L2nc, Field<R> L3nc, Geom g,
                                                                             DD* __restrict__ partials, R* __restrict__ fbar)
 {
-    Site s;
+    pdl_trigger();
+    Site s{};
     int par, h;
     double d = 0.0;
-    if (site_warp_pair(g, blockIdx.x, threadIdx.x, kQtopBlock, s, par, h)) {
+    const bool valid = site_warp_pair(g, blockIdx.x, threadIdx.x, kQtopBlock, s, par, h);
+    pdl_wait(h, s.n);
+    if (valid) {
+        const FieldCA<R> U = field_ca(Unc), L2 = field_ca(L2nc), L3 = field_ca(L3nc);
         d += qtop_product<R, 0, FBAR>(U, L2, L3, g, s, par, h, fbar);
         d += qtop_product<R, 2, FBAR>(U, L2, L3, g, s, par, h, fbar);
         d += qtop_product<R, 4, FBAR>(U, L2, L3, g, s, par, h, fbar);
@@ -511,7 +541,14 @@ void launch_ape_t(su2g_lattice* h, const Field<R>& in, const Field<R>& out, R al
 {
     constexpr int block = ape_block<R, MODE>();
     const int grid = (int)((2 * (long long)h->g.Vh + block - 1) / block);   // warp pairs over the same h run
-    k_ape<R, MODE><<<grid, block, 0, h->stream>>>(in, out, h->g, alpha);
+    // FP32 APE_all on fields beyond L2: in order, through the read-only path (below)
+    if constexpr (MODE == SU2G_APE_ALL && sizeof(R) == 4) {
+        if (8ull * h->g.V * h->link_bytes > h->l2_bytes) {
+            k_ape<R, MODE, false><<<grid, block, 0, h->stream>>>(in, out, h->g, alpha);
+            return;
+        }
+    }
+    launch_pdl(k_ape<R, MODE, true>, grid, block, h->stream, in, out, h->g, alpha);
 }
 
 template <typename R>
@@ -591,9 +628,9 @@ int su2g::plaquette_enqueue(su2g_lattice* h, double* out)
     if (rc) return rc;
     launch_begin(h, SU2G_K_PLAQUETTE);
     if (h->prec == SU2G_FP32)
-        k_plaquette<float><<<grid, 128, 0, h->stream>>>(make_field<float>(h->dirp, h->g.Vh), h->g, h->partials);
+        launch_pdl(k_plaquette<float>, grid, 128, h->stream, make_field<float>(h->dirp, h->g.Vh), h->g, h->partials);
     else
-        k_plaquette<double><<<grid, 128, 0, h->stream>>>(make_field<double>(h->dirp, h->g.Vh), h->g, h->partials);
+        launch_pdl(k_plaquette<double>, grid, 128, h->stream, make_field<double>(h->dirp, h->g.Vh), h->g, h->partials);
     rc = launch_end(h, SU2G_K_PLAQUETTE, "plaquette kernel");
     // plaq = sum 2 c0 / (2 * 6 * V)  (plaquette.c:97); the kernel sums c0 = (1/2) Re tr
     if (!rc) rc = finalize(h, h->partials, grid, 1, grid, 1.0 / (6.0 * (double)h->g.V), out);
@@ -656,9 +693,9 @@ static void launch_qtop(su2g_lattice* h, void* const dirs[4], int grid, void* fb
     void *l2[4], *l3[4];
     line_dirs(h, l2, l3);
     const Field<R> U = make_field<R>(dirs, h->g.Vh), L2 = make_field<R>(l2, h->g.Vh), L3 = make_field<R>(l3, h->g.Vh);
-    k_lines<R><<<2 * (int)((h->g.Vh + kBlock - 1) / kBlock), kBlock, 0, h->stream>>>(U, L2, L3, h->g);
-    if (fbar) k_qtop<R, true><<<grid, kQtopBlock, 0, h->stream>>>(U, L2, L3, h->g, h->partials, (R*)fbar);
-    else k_qtop<R, false><<<grid, kQtopBlock, 0, h->stream>>>(U, L2, L3, h->g, h->partials, nullptr);
+    launch_pdl(k_lines<R>, 2 * (int)((h->g.Vh + kBlock - 1) / kBlock), kBlock, h->stream, U, L2, L3, h->g);
+    if (fbar) launch_pdl(k_qtop<R, true>, grid, kQtopBlock, h->stream, U, L2, L3, h->g, h->partials, (R*)fbar);
+    else launch_pdl(k_qtop<R, false>, grid, kQtopBlock, h->stream, U, L2, L3, h->g, h->partials, (R*)nullptr);
 }
 
 int su2g::qtop_enqueue(su2g_lattice* h, void* const dirs[4], int out_off, void* fbar)

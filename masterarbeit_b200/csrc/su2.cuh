@@ -421,15 +421,15 @@ struct FieldCG<double> : Field<double> {
 };
 
 // Plain quaternion arrays (32-byte aligned in FP64).
-__device__ __forceinline__ Q<float> ldq(const float* p, size_t i)
+__device__ __forceinline__ Q<float> ldq_ca(const float* p, size_t i)
 {
-    float4 v = reinterpret_cast<const float4*>(p)[i];
-    return q_make<float>(v.x, v.y, v.z, v.w);
+    Q<float> q;
+    asm("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
+        : "=f"(q.c0), "=f"(q.c1), "=f"(q.c2), "=f"(q.c3)
+        : "l"(reinterpret_cast<const float4*>(p) + i));
+    return q;
 }
-__device__ __forceinline__ Q<double> ldq(const double* p, size_t i)
-{
-    return ldnc_256(reinterpret_cast<const Vec4d*>(p) + i);
-}
+__device__ __forceinline__ Q<double> ldq_ca(const double* p, size_t i) { return ld_256(reinterpret_cast<const Vec4d*>(p) + i); }
 __device__ __forceinline__ void stq(float* p, size_t i, const Q<float>& q)
 {
     reinterpret_cast<float4*>(p)[i] = make_float4(q.c0, q.c1, q.c2, q.c3);
