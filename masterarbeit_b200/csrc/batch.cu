@@ -4,11 +4,10 @@
 // hot/cold start and id).  Here a batch holds R replicas of possibly different extents, beta,
 // seed and start in one device pool.  A replica-offset table maps every CTA of a launch to its
 // replica, so one launch per checkerboard pass (mu, parity) updates all replicas, and one launch
-// measures every replica's plaquette.  A whole measurement block (meas_every sweeps of n_hb
-// heatbath + n_or overrelaxation passes, then the plaquettes) is captured once in a CUDA graph and
-// replayed; the Philox sweep index and the measurement slot live in device counters that the graph
-// advances itself.  Each replica draws the same Philox streams as a single-lattice handle with the
-// same (seed, replica id), so a batch and a set of single handles give identical fields.
+// measures every replica's plaquette.  The launches of a run are enqueued at once, as programmatic
+// dependent ones (pdl_wait): each starts in the tail of the one before.  Each replica draws the same Philox
+// streams as a single-lattice handle with the same (seed, replica id), so a batch and a set of single
+// handles give identical fields.
 //
 // Persistent form.  Alternatively one cooperative launch runs every measurement block of a
 // su2g_batch_run: its CTAs (all resident) walk the links of each pass as one global index over all
@@ -19,6 +18,7 @@
 #include <algorithm>
 #include <cmath>
 #include <new>
+#include <type_traits>
 #include <vector>
 
 #include "internal.cuh"
@@ -38,8 +38,6 @@ struct Replica {
     void* dirs[4];
 };
 
-enum { kCtrSweep = 0, kCtrMeas = 1 };
-
 // Grid-wide barrier state of the persistent form (zeroed before every launch).
 struct GridBarrier {
     unsigned count, gen, abort, pad;
@@ -57,13 +55,17 @@ struct su2g_batch {
     void* pool = nullptr;
     size_t pool_bytes = 0;
     DD* partials = nullptr;
-    uint32_t* d_ctr = nullptr;                     // [sweep index, measurement slot]
+    uint32_t sweeps = 0;                           // heatbath sweeps done, the Philox sweep index
+    bool uniform = false;                          // all replicas have the same extents
+    long long links = 0;                           // links a pass updates
+    size_t stride = 0;                             // bytes from one replica's field to the next, if uniform
     unsigned* d_status = nullptr;
     double* d_trace = nullptr;
     size_t trace_cap = 0;
     int trace_rows = 0;                            // measurements in the trace of the last run
     cudaStream_t stream = nullptr;
-    cudaGraphExec_t graph = nullptr;
+    uint32_t* d_ctr = nullptr;                     // {sweep index, trace row} of a replayed block
+    cudaGraphExec_t graph = nullptr;               // one measurement block (small batches)
     int g_hb = -1, g_or = -1, g_meas = -1, g_every = -1, g_block = -1;
     int mode = SU2G_BATCH_GRAPH;                   // su2g_batch_mode
     int* d_upre = nullptr;                         // first global link index of each replica in a pass (n+1)
@@ -99,82 +101,160 @@ __device__ __forceinline__ Field<R> rep_field(const Replica& r)
     return f;
 }
 
-template <typename R, int MU, int KIND>
-__global__ void __launch_bounds__(256, 4) k_batch_update(const Replica* __restrict__ reps, const int* __restrict__ map,
-                                                      const int* __restrict__ blk0, int par, int sub,
-                                                      const uint32_t* __restrict__ ctr, unsigned* __restrict__ status)
+// One replica's field as one array of 4 x 2Vh links (the pool's layout), for a batch whose replicas share
+// their extents: one base pointer, the direction enters the 32-bit element index.  Plain loads, as FieldCA.
+template <typename R>
+struct PoolField {
+    char* base;
+    int Vh;
+    __device__ __forceinline__ unsigned at(int mu, int par, int h) const { return (unsigned)(2 * mu + par) * (unsigned)Vh + (unsigned)h; }
+    __device__ __forceinline__ Q<R> ldh(int mu, int par, int h) const
+    {
+        return ldq_ca(reinterpret_cast<const R*>(base), (size_t)at(mu, par, h));
+    }
+    __device__ __forceinline__ Q<R> ld(int mu, int par, int n) const { return ldh(mu, par, (int)((unsigned)n >> 1)); }
+    __device__ __forceinline__ void sth(int mu, int par, int h, const Q<R>& q) const
+    {
+        stq(reinterpret_cast<R*>(base), (size_t)at(mu, par, h), q);
+    }
+};
+
+// The links or sites of a launch.  UNI: CTA (b, r) is CTA b of replica r, whose geometry is a launch
+// parameter, in the constant bank, instead of read from the replica table into registers (64 x 12^4 with a
+// plaquette, us a sweep, with the overlapping launches below: FP32 heatbath 186 -> 161, overrelaxation 133 -> 115;
+// FP64 416 -> 345, 327 -> 272).  Otherwise a map gives each CTA's replica.
+struct BatchGrid {
+    const Replica* reps;
+    const int *map, *blk0;   // not UNI
+    Geom g;                  // UNI
+    char* pool;
+    size_t stride;
+};
+
+template <typename R, bool UNI>
+struct BatchCta {
+    const Replica& rp;
+    int cta;
+    __device__ __forceinline__ explicit BatchCta(const BatchGrid& a)
+        : BatchCta(a, UNI ? (int)blockIdx.y : a.map[blockIdx.x])
+    {
+    }
+    __device__ __forceinline__ BatchCta(const BatchGrid& a, int r)
+        : rp(a.reps[r]), cta(UNI ? (int)blockIdx.x : (int)blockIdx.x - a.blk0[r])
+    {
+    }
+};
+
+template <typename R>
+__device__ __forceinline__ PoolField<R> batch_field(const BatchGrid& a, const Replica&, PoolField<R>*)
 {
-    const int r = map[blockIdx.x];
-    const Replica& rp = reps[r];
-    const Geom g = rp.g;
-    const int h = (blockIdx.x - blk0[r]) * blockDim.x + threadIdx.x;
+    return PoolField<R>{a.pool + blockIdx.y * a.stride, a.g.Vh};
+}
+template <typename R>
+__device__ __forceinline__ FieldCA<R> batch_field(const BatchGrid&, const Replica& rp, FieldCA<R>*)
+{
+    return field_ca(rep_field<R>(rp));
+}
+template <typename R, bool UNI>
+using BatchField = std::conditional_t<UNI, PoolField<R>, FieldCA<R>>;
+
+// EARLY: that many trials and the angles are drawn before the wait, as in the handle's passes (k_update).
+template <typename R, int MU, int KIND, bool UNI, int EARLY>
+__global__ void __launch_bounds__(256, 4) k_batch_update(BatchGrid a, int par, uint32_t sweep, const uint32_t* ctr, unsigned* __restrict__ status)
+{
+    pdl_trigger();
+    if (KIND == SU2G_HEATBATH && ctr) sweep += ctr[0];   // written by no launch this one can overlap
+    const BatchCta<R, UNI> c(a);
+    const Replica& rp = c.rp;
+    const Geom g = UNI ? a.g : rp.g;
+    int h = c.cta * blockDim.x + threadIdx.x;
+    Site s = site_of(g, par, h);
+    KpTrial<R> early[EARLY > 0 ? EARLY : 1];
+    KpAngles<R> angles;
+    if (EARLY > 0) {
+#pragma unroll
+        for (int i = 0; i < EARLY; ++i)
+            early[i] = kp_trial<R>(rp.seed, (uint32_t)s.n, sweep, (uint32_t)MU, rp.id, (uint32_t)i);
+        angles = kp_angles<R>(rp.seed, (uint32_t)s.n, sweep, (uint32_t)MU, rp.id, 0u);
+    }
+    pdl_wait(h, s.n);
     if (h >= g.Vh) return;
-    const Field<R> U = rep_field<R>(rp);
-    const Site s = site_of(g, par, h);
-    const Q<R> A = staple_update<R, MU>(U, g, s, par);
+    const auto U = batch_field(a, rp, (BatchField<R, UNI>*)nullptr);
+    const Q<R> A = staple_update<R, MU, 0>(U, g, s, par);
     if (KIND == SU2G_HEATBATH) {
         Q<R> out;
         uint32_t trials = 0;
-        if (heatbath_link<R>(A, (R)rp.kb, rp.seed, (uint32_t)s.n, ctr[kCtrSweep] + sub, (uint32_t)MU, rp.id, trials,
-                             out, status))
+        if (heatbath_link<R, EARLY>(A, (R)rp.kb, rp.seed, (uint32_t)s.n, sweep, (uint32_t)MU, rp.id, trials, out, status, 0u,
+                                    early, angles))
             U.sth(MU, par, h, hb_store(out));
     } else {
         U.sth(MU, par, h, q_project(overrelax_link<R>(A, U.ldh(MU, par, h))));
     }
 }
 
-template <typename R>
-__global__ void __launch_bounds__(256) k_batch_plaquette(const Replica* __restrict__ reps, const int* __restrict__ map,
-                                                         const int* __restrict__ blk0, DD* __restrict__ partials)
+// One site per thread, parities paired per warp; one partial per CTA (plain FP64 within a warp,
+// compensated across its warps), 256 threads at most.
+template <typename R, bool UNI>
+__global__ void __launch_bounds__(256) k_batch_plaquette(BatchGrid a, DD* __restrict__ partials)
 {
-    const int r = map[blockIdx.x];
-    const Replica& rp = reps[r];
-    const Geom g = rp.g;
-    const int i = (blockIdx.x - blk0[r]) * blockDim.x + threadIdx.x;
+    pdl_trigger();
+    const BatchCta<R, UNI> c(a);
+    const Geom g = UNI ? a.g : c.rp.g;
+    Site s{};
+    int par, h;
+    const bool valid = site_warp_pair(g, c.cta, threadIdx.x, blockDim.x, s, par, h);
+    pdl_wait(h, s.n);
     double site = 0.0;
-    if (i < g.V) {
-        const Field<R> U = rep_field<R>(rp);
-        int par;
-        const Site s = site_lex(g, i, par);
-        const int h = i >> 1, q = par ^ 1;
+    if (valid) {
+        const auto U = batch_field(a, c.rp, (BatchField<R, UNI>*)nullptr);
+        const int q = par ^ 1;
+        Q<R> u[4];
+        int xp[4];
+#pragma unroll
+        for (int mu = 0; mu < 4; ++mu) {
+            u[mu] = U.ldh(mu, par, h);
+            xp[mu] = s.n + up_off_rt(g, s.c, mu);
+        }
 #pragma unroll
         for (int mu = 0; mu < 3; ++mu)
 #pragma unroll
             for (int nu = mu + 1; nu < 4; ++nu) {
-                const Q<R> a = q_mul(U.ldh(mu, par, h), U.ld(nu, q, s.n + up_off_rt(g, s.c, mu)));
-                const Q<R> b = q_mul(U.ldh(nu, par, h), U.ld(mu, q, s.n + up_off_rt(g, s.c, nu)));
-                site += (double)q_dot(a, b);
+                const Q<R> x = q_mul(u[mu], U.ld(nu, q, xp[mu]));
+                const Q<R> y = q_mul(u[nu], U.ld(mu, q, xp[nu]));
+                site += (double)q_dot(x, y);
             }
     }
-    // block sums with 256 threads at most; inactive threads contribute 0
-    __shared__ DD part[8];
-    DD v = dd_warp_sum(DD{site, 0.0});
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+    __shared__ double part[8];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) site += __shfl_xor_sync(0xffffffffu, site, o);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = site;
     __syncthreads();
-    if (threadIdx.x < 32) {
-        DD w = threadIdx.x < (blockDim.x >> 5) ? part[threadIdx.x] : DD{0.0, 0.0};
-        w = dd_warp_sum(w);
-        if (threadIdx.x == 0) partials[blockIdx.x] = w;
+    if (threadIdx.x == 0) {
+        DD v = {0.0, 0.0};
+        for (int w = 0; w < (int)blockDim.x >> 5; ++w) v = dd_add(v, part[w]);
+        partials[UNI ? blockIdx.y * gridDim.x + blockIdx.x : blockIdx.x] = v;
     }
 }
 
-// One CTA per replica: fixed-order sum of its CTAs' partials into trace[slot][r].
-__global__ void __launch_bounds__(kBlock) k_batch_plaq_final(const Replica* __restrict__ reps,
-                                                             const int* __restrict__ blk0, const DD* __restrict__ partials,
-                                                             int nrep, double* __restrict__ trace,
-                                                             const uint32_t* __restrict__ ctr)
+// One CTA per replica: fixed-order sum of its CTAs' partials into row[r].
+__global__ void __launch_bounds__(kBlock) k_batch_plaq_final(const Replica* __restrict__ reps, const int* __restrict__ blk0,
+                                                             const DD* partials, double* __restrict__ row,
+                                                             const uint32_t* ctr)
 {
+    pdl_trigger();
     const int r = blockIdx.x;
+    int first = blk0[r] + threadIdx.x, last = blk0[r + 1];
+    pdl_wait(first, last);
     DD acc = {0.0, 0.0};
-    for (int b = blk0[r] + threadIdx.x; b < blk0[r + 1]; b += blockDim.x) acc = dd_add(acc, partials[b]);
+    for (int b = first; b < last; b += blockDim.x) acc = dd_add(acc, partials[b]);
     acc = dd_block_sum<kBlock>(acc);
-    if (threadIdx.x == 0) trace[(size_t)ctr[kCtrMeas] * nrep + r] = (acc.s + acc.e) / (6.0 * (double)reps[r].g.V);
+    if (threadIdx.x == 0) row[(ctr ? (size_t)ctr[1] * gridDim.x : 0) + r] = (acc.s + acc.e) / (6.0 * (double)reps[r].g.V);
 }
 
-__global__ void k_batch_tick(uint32_t* ctr, int n_hb, int meas)
+__global__ void k_batch_tick(uint32_t* ctr, uint32_t n_hb)
 {
-    ctr[kCtrSweep] += (uint32_t)n_hb;
-    ctr[kCtrMeas] += (uint32_t)meas;
+    ctr[0] += n_hb;
+    ctr[1] += 1u;
 }
 
 template <typename R>
@@ -288,7 +368,7 @@ struct PersistArgs {
     const int* smap;     // site chunk -> replica, chunks of blockDim sites (the plaquette)
     const int* sblk;     // n+1 first site chunk of each replica
     int n, nblocks, every, n_hb, n_or, meas;
-    uint32_t* ctr;
+    uint32_t sweep0;
     double* trace;
     DD* partials;
     GridBarrier* gb;
@@ -351,15 +431,14 @@ __device__ __forceinline__ void persist_pass_mu(const PersistArgs& a, const int*
 
 // Every measurement block of a run in one launch: `every` sweeps of n_hb heatbath and n_or
 // overrelaxation passes, then (if meas) each replica's plaquette into its trace slot, exactly the
-// work and the Philox streams of the replayed graph of launches.
+// work and the Philox streams of the launches per pass.
 template <typename R, int NT>
 __global__ void __launch_bounds__(NT, (sizeof(R) == 8 ? 512 : 1024) / NT) k_batch_persist(PersistArgs a)
 {
     extern __shared__ int s_pre[];
     for (int i = threadIdx.x; i <= a.n; i += NT) s_pre[i] = a.upre[i];
     __syncthreads();
-    // every CTA reads the counters here; CTA 0 writes them back only after the last barrier
-    uint32_t sweep = a.ctr[kCtrSweep], slot = a.ctr[kCtrMeas];
+    uint32_t sweep = a.sweep0, slot = 0;
     const int nchunks = a.sblk[a.n];
     for (int blk = 0; blk < a.nblocks; ++blk) {
         for (int s = 0; s < a.every; ++s) {
@@ -413,10 +492,6 @@ __global__ void __launch_bounds__(NT, (sizeof(R) == 8 ? 512 : 1024) / NT) k_batc
         ++slot;
         if (!grid_sync(a.gb, a.status)) return;   // the partials are written again by the next block
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        a.ctr[kCtrSweep] = sweep;
-        a.ctr[kCtrMeas] = slot;
-    }
 }
 
 // CTA maps for a block size: CTAs of replica r are [blk[r], blk[r+1]).
@@ -458,50 +533,97 @@ int build_maps(su2g_batch* b, int block)
 const int* ublk0(const su2g_batch* b) { return b->d_umap + b->ublk[b->n]; }
 const int* sblk0(const su2g_batch* b) { return b->d_smap + b->sblk[b->n]; }
 
-template <typename R, int KIND>
-void launch_pass(su2g_batch* b, int mu, int par, int sub)
+BatchGrid batch_grid(const su2g_batch* b, bool sites)
 {
-    const int grid = b->ublk[b->n];
-    switch (mu) {
-        case 0: k_batch_update<R, 0, KIND><<<grid, b->block, 0, b->stream>>>(b->d_reps, b->d_umap, ublk0(b), par, sub, b->d_ctr, b->d_status); break;
-        case 1: k_batch_update<R, 1, KIND><<<grid, b->block, 0, b->stream>>>(b->d_reps, b->d_umap, ublk0(b), par, sub, b->d_ctr, b->d_status); break;
-        case 2: k_batch_update<R, 2, KIND><<<grid, b->block, 0, b->stream>>>(b->d_reps, b->d_umap, ublk0(b), par, sub, b->d_ctr, b->d_status); break;
-        default: k_batch_update<R, 3, KIND><<<grid, b->block, 0, b->stream>>>(b->d_reps, b->d_umap, ublk0(b), par, sub, b->d_ctr, b->d_status); break;
+    BatchGrid a;
+    a.reps = b->d_reps;
+    a.map = sites ? b->d_smap : b->d_umap;
+    a.blk0 = sites ? sblk0(b) : ublk0(b);
+    a.g = b->reps[0].g;
+    a.pool = (char*)b->pool;
+    a.stride = b->stride;
+    return a;
+}
+
+// A batch is small when a pass has fewer links than fill the SMs about twice over at 256 threads a CTA.
+// A pass of a small batch is as short as a launch takes the host, and the CTAs of an overlapping launch
+// crowd on the SMs the running one leaves idle (16 x 8^4, 1 HB + 4 OR, us a sweep: 115 FP32, 184 FP64
+// one after another; 143, 234 overlapping).  Small batches therefore replay a captured block of ordinary
+// launches; the others launch pass by pass, programmatically, FP32 with two trials drawn early (64 x 8^4:
+// 193 -> 172 FP32, 377 -> 282 FP64).
+bool small_batch(const su2g_batch* b) { return b->links <= 640ll * b->num_sms; }
+
+template <typename R, int MU, int KIND>
+void launch_pass_mu(su2g_batch* b, int par, uint32_t sweep, const uint32_t* ctr)
+{
+    constexpr int kEarly = KIND == SU2G_HEATBATH && sizeof(R) == 4 ? 2 : 0;   // FP64 has no registers left for it
+    const BatchGrid a = batch_grid(b, false);
+    const dim3 grid = b->uniform ? dim3(b->ublk[1], b->n) : dim3(b->ublk[b->n]);
+    if (small_batch(b)) {
+        auto* kernel = b->uniform ? k_batch_update<R, MU, KIND, true, 0> : k_batch_update<R, MU, KIND, false, 0>;
+        kernel<<<grid, b->block, 0, b->stream>>>(a, par, sweep, ctr, b->d_status);
+    } else {
+        auto* kernel = b->uniform ? k_batch_update<R, MU, KIND, true, kEarly> : k_batch_update<R, MU, KIND, false, kEarly>;
+        launch_pdl(kernel, grid, b->block, b->stream, a, par, sweep, ctr, b->d_status);
     }
 }
 
-// The launches of one measurement block: `every` sweeps, then (if meas) the plaquettes.
+template <typename R, int KIND>
+void launch_pass(su2g_batch* b, int mu, int par, uint32_t sweep, const uint32_t* ctr)
+{
+    switch (mu) {
+        case 0: launch_pass_mu<R, 0, KIND>(b, par, sweep, ctr); break;
+        case 1: launch_pass_mu<R, 1, KIND>(b, par, sweep, ctr); break;
+        case 2: launch_pass_mu<R, 2, KIND>(b, par, sweep, ctr); break;
+        default: launch_pass_mu<R, 3, KIND>(b, par, sweep, ctr); break;
+    }
+}
+
+// The launches of one measurement block: `every` sweeps, the first of index sweep0 (+ ctr[0]), then (if
+// row) the plaquettes into row[replica] (ctr[1] rows further on).
 template <typename R>
-void enqueue_block(su2g_batch* b, int n_hb, int n_or, int every, int meas)
+void enqueue_block(su2g_batch* b, int n_hb, int n_or, int every, uint32_t sweep0, double* row, const uint32_t* ctr)
 {
     for (int s = 0; s < every; ++s) {
         for (int i = 0; i < n_hb; ++i)
             for (int mu = 0; mu < 4; ++mu)
-                for (int par = 0; par < 2; ++par) launch_pass<R, SU2G_HEATBATH>(b, mu, par, s * n_hb + i);
+                for (int par = 0; par < 2; ++par) launch_pass<R, SU2G_HEATBATH>(b, mu, par, sweep0 + (uint32_t)(s * n_hb + i), ctr);
         for (int i = 0; i < n_or; ++i)
             for (int mu = 0; mu < 4; ++mu)
-                for (int par = 0; par < 2; ++par) launch_pass<R, SU2G_OVERRELAX>(b, mu, par, 0);
+                for (int par = 0; par < 2; ++par) launch_pass<R, SU2G_OVERRELAX>(b, mu, par, 0u, nullptr);
     }
-    if (meas) {
-        k_batch_plaquette<R><<<b->sblk[b->n], b->block, 0, b->stream>>>(b->d_reps, b->d_smap, sblk0(b), b->partials);
-        k_batch_plaq_final<<<b->n, kBlock, 0, b->stream>>>(b->d_reps, sblk0(b), b->partials, b->n, b->d_trace, b->d_ctr);
+    if (!row) return;
+    const BatchGrid a = batch_grid(b, true);
+    const dim3 grid = b->uniform ? dim3(b->sblk[1], b->n) : dim3(b->sblk[b->n]);
+    auto* kernel = b->uniform ? k_batch_plaquette<R, true> : k_batch_plaquette<R, false>;
+    if (small_batch(b)) {
+        kernel<<<grid, b->block, 0, b->stream>>>(a, b->partials);
+        k_batch_plaq_final<<<b->n, kBlock, 0, b->stream>>>(b->d_reps, sblk0(b), b->partials, row, ctr);
+    } else {
+        launch_pdl(kernel, grid, b->block, b->stream, a, b->partials);
+        launch_pdl(k_batch_plaq_final, b->n, kBlock, b->stream, b->d_reps, sblk0(b), b->partials, row, ctr);
     }
-    k_batch_tick<<<1, 1, 0, b->stream>>>(b->d_ctr, n_hb * every, meas);
 }
 
+void enqueue_block(su2g_batch* b, int n_hb, int n_or, int every, uint32_t sweep0, double* row, const uint32_t* ctr)
+{
+    if (b->prec == SU2G_FP32) enqueue_block<float>(b, n_hb, n_or, every, sweep0, row, ctr);
+    else enqueue_block<double>(b, n_hb, n_or, every, sweep0, row, ctr);
+}
+
+// A captured measurement block, which advances the sweep index and trace row it reads by itself.
 int ensure_graph(su2g_batch* b, int n_hb, int n_or, int every, int meas)
 {
-    if (b->graph && b->g_hb == n_hb && b->g_or == n_or && b->g_every == every && b->g_meas == meas &&
-        b->g_block == b->block)
+    if (b->graph && b->g_hb == n_hb && b->g_or == n_or && b->g_every == every && b->g_meas == meas && b->g_block == b->block)
         return SU2G_OK;
     if (b->graph) cudaGraphExecDestroy(b->graph);
     b->graph = nullptr;
     cudaGraph_t gr = nullptr;
     int rc = bcuda(b, cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal), "beginning graph capture");
     if (rc) return rc;
-    if (b->prec == SU2G_FP32) enqueue_block<float>(b, n_hb, n_or, every, meas);
-    else enqueue_block<double>(b, n_hb, n_or, every, meas);
-    cudaError_t launch_err = cudaGetLastError();
+    enqueue_block(b, n_hb, n_or, every, 0u, meas ? b->d_trace : nullptr, b->d_ctr);
+    k_batch_tick<<<1, 1, 0, b->stream>>>(b->d_ctr, (uint32_t)(n_hb * every));
+    const cudaError_t launch_err = cudaGetLastError();
     rc = bcuda(b, cudaStreamEndCapture(b->stream, &gr), "ending graph capture");
     if (!rc) rc = bcuda(b, launch_err, "capturing the sweep");
     if (!rc) rc = bcuda(b, cudaGraphInstantiate(&b->graph, gr, 0), "instantiating the sweep graph");
@@ -556,7 +678,7 @@ int launch_persist(su2g_batch* b, int nblocks, int n_hb, int n_or, int every, in
     a.n_hb = n_hb;
     a.n_or = n_or;
     a.meas = meas;
-    a.ctr = b->d_ctr;
+    a.sweep0 = b->sweeps;
     a.trace = b->d_trace;
     a.partials = b->partials;
     a.gb = b->d_gb;
@@ -591,12 +713,12 @@ extern "C" int su2g_batch_destroy(su2g_batch* b)
     cudaSetDevice(b->device);
     if (b->stream) cudaStreamSynchronize(b->stream);
     if (b->graph) cudaGraphExecDestroy(b->graph);
+    cudaFree(b->d_ctr);
     cudaFree(b->d_reps);
     cudaFree(b->d_umap);
     cudaFree(b->d_smap);
     cudaFree(b->pool);
     cudaFree(b->partials);
-    cudaFree(b->d_ctr);
     cudaFree(b->d_status);
     cudaFree(b->d_trace);
     cudaFree(b->d_upre);
@@ -660,6 +782,10 @@ extern "C" int su2g_batch_create(const su2g_replica* reps, int32_t n, int32_t pr
         b->reps.push_back(rp);
     }
     b->pool_bytes = total;
+    b->uniform = n <= 65535;   // replicas are the y extent of a uniform batch's grids
+    for (int r = 1; r < n; ++r)
+        for (int d = 0; d < 4; ++d) b->uniform = b->uniform && reps[r].dims[d] == reps[0].dims[d];
+    b->stride = n > 1 ? off[1] : total;
     int rc = bcuda(b, cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking), "creating stream");
     if (!rc) rc = bcuda(b, cudaMalloc(&b->pool, total), "allocating the replica pool");
     if (!rc)
@@ -677,12 +803,12 @@ extern "C" int su2g_batch_create(const su2g_replica* reps, int32_t n, int32_t pr
         }
         if (tot > (1ll << 30)) rc = berr(b, SU2G_EINVAL, "the replicas hold more than 2^31 links");
         upre[n] = (int)tot;
+        b->links = tot;
         if (!rc) rc = bcuda(b, cudaMalloc(&b->d_upre, (n + 1) * sizeof(int)), "allocating the link prefix table");
         if (!rc) rc = bcuda(b, cudaMemcpy(b->d_upre, upre.data(), (n + 1) * sizeof(int), cudaMemcpyHostToDevice), "table");
         if (!rc) rc = bcuda(b, cudaMalloc(&b->d_gb, sizeof(GridBarrier)), "allocating the grid barrier");
     }
     if (!rc) rc = bcuda(b, cudaMalloc(&b->d_ctr, 2 * sizeof(uint32_t)), "allocating counters");
-    if (!rc) rc = bcuda(b, cudaMemset(b->d_ctr, 0, 2 * sizeof(uint32_t)), "clearing counters");
     if (!rc) rc = bcuda(b, cudaMalloc(&b->d_status, sizeof(unsigned)), "allocating status");
     if (!rc) rc = bcuda(b, cudaMemset(b->d_status, 0, sizeof(unsigned)), "clearing status");
     if (!rc) rc = bcuda(b, cudaEventCreate(&b->ev0), "events");
@@ -729,19 +855,30 @@ extern "C" int su2g_batch_run(su2g_batch* b, int32_t n_sweeps, int32_t n_hb, int
         b->trace_cap = b->n;
     }
     const bool persist = b->mode == SU2G_BATCH_PERSISTENT;
-    if (!persist && (rc = ensure_graph(b, n_hb, n_or, every, meas))) return rc;
-    // measurement slots restart at 0 for every run
-    uint32_t zero = 0;
-    if ((rc = bcuda(b, cudaMemcpyAsync(b->d_ctr + kCtrMeas, &zero, sizeof(zero), cudaMemcpyHostToDevice, b->stream),
-                    "resetting the slot counter")))
-        return rc;
+    const bool replay = !persist && small_batch(b);
+    if (replay && nblocks > 0) {
+        if ((rc = ensure_graph(b, n_hb, n_or, every, meas))) return rc;
+        const uint32_t ctr[2] = {b->sweeps, 0u};
+        if ((rc = bcuda(b, cudaMemcpyAsync(b->d_ctr, ctr, sizeof(ctr), cudaMemcpyHostToDevice, b->stream), "setting counters")))
+            return rc;
+    }
     cudaEventRecord(b->ev0, b->stream);
     if (persist) {
         if (nblocks > 0 && (rc = launch_persist(b, nblocks, n_hb, n_or, every, meas))) return rc;
     } else {
-        for (int i = 0; i < nblocks; ++i)
-            if ((rc = bcuda(b, cudaGraphLaunch(b->graph, b->stream), "launching the sweep graph"))) return rc;
+        for (int i = 0; i < nblocks; ++i) {
+            const uint32_t sweep0 = b->sweeps + (uint32_t)i * (uint32_t)(n_hb * every);
+            double* row = meas ? b->d_trace + (size_t)i * b->n : nullptr;
+            if (replay) {
+                rc = bcuda(b, cudaGraphLaunch(b->graph, b->stream), "launching the sweep graph");
+            } else {
+                enqueue_block(b, n_hb, n_or, every, sweep0, row, nullptr);
+                rc = bcuda(b, cudaGetLastError(), "launching the sweeps");
+            }
+            if (rc) return rc;
+        }
     }
+    b->sweeps += (uint32_t)nblocks * (uint32_t)(n_hb * every);
     cudaEventRecord(b->ev1, b->stream);
     if ((rc = bcuda(b, cudaStreamSynchronize(b->stream), "running sweeps"))) return rc;
     if (ms) {
@@ -788,14 +925,13 @@ extern "C" int su2g_batch_autotune(su2g_batch* b, int32_t n_hb, int32_t n_or, in
 {
     if (!b) return set_error(nullptr, SU2G_EINVAL, "su2g_batch_autotune: null batch");
     cudaSetDevice(b->device);
-    // the trial sweeps must not move the chains: save and restore the pool and the counters
+    // the trial sweeps must not move the chains: save and restore the pool and the sweep counter
     const size_t pool_bytes = b->pool_bytes;
     void* save = nullptr;
-    uint32_t ctr[2];
+    const uint32_t sweeps = b->sweeps;
     int rc = bcuda(b, cudaMalloc(&save, pool_bytes), "allocating the autotune copy");
     if (!rc) rc = bcuda(b, cudaMemcpy(save, b->pool, pool_bytes, cudaMemcpyDeviceToDevice), "saving replicas");
-    if (!rc) rc = bcuda(b, cudaMemcpy(ctr, b->d_ctr, sizeof(ctr), cudaMemcpyDeviceToHost), "saving counters");
-    // the two forms (replayed graph of per-pass launches; one persistent launch) over CTA widths,
+    // the two forms (a launch per pass; one persistent launch) over CTA widths,
     // each timed on 4 sweeps with a plaquette after every sweep, after 2 warm-up sweeps
     const int candidates[][2] = {{SU2G_BATCH_GRAPH, 64},       {SU2G_BATCH_GRAPH, 128}, {SU2G_BATCH_GRAPH, 256},
                                  {SU2G_BATCH_PERSISTENT, 128}, {SU2G_BATCH_PERSISTENT, 256}};
@@ -806,7 +942,7 @@ extern "C" int su2g_batch_autotune(su2g_batch* b, int32_t n_hb, int32_t n_or, in
         if ((rc = build_maps(b, c[1]))) break;
         b->mode = c[0];
         double ms = 0;
-        if ((rc = su2g_batch_run(b, 2, n_hb, n_or, 1, nullptr, &ms))) break;   // warm-up + graph build
+        if ((rc = su2g_batch_run(b, 2, n_hb, n_or, 1, nullptr, &ms))) break;   // warm-up
         if ((rc = su2g_batch_run(b, 4, n_hb, n_or, 1, nullptr, &ms))) break;
         if (ms < best) {
             best = ms;
@@ -817,7 +953,7 @@ extern "C" int su2g_batch_autotune(su2g_batch* b, int32_t n_hb, int32_t n_or, in
     b->mode = best_mode;
     if (!rc) rc = build_maps(b, best_block);
     if (!rc) rc = bcuda(b, cudaMemcpy(b->pool, save, pool_bytes, cudaMemcpyDeviceToDevice), "restoring replicas");
-    if (!rc) rc = bcuda(b, cudaMemcpy(b->d_ctr, ctr, sizeof(ctr), cudaMemcpyHostToDevice), "restoring counters");
+    b->sweeps = sweeps;
     cudaFree(save);
     if (block_out) *block_out = b->block;
     return rc;
