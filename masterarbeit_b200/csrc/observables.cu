@@ -119,6 +119,16 @@ __global__ void __launch_bounds__(ape_block<R, MODE>(), ape_min_blocks<R, MODE>(
 constexpr int kWilsonTChunk = 32;   // T values one launch records
 constexpr int kWilsonWarps = kBlock / 32;
 
+// One launch's loops: RC spatial extents in ascending order, the temporal extents tlo ... thi, of which
+// those whose bit T - tlo is set in `want` are recorded.
+struct WilsonLoops {
+    int r[8];
+    int tlo, thi;
+    uint32_t want;
+    __host__ __device__ int nT() const { return thi - tlo + 1; }
+    __device__ bool records(int T) const { return T >= tlo && (want >> (T - tlo) & 1u); }
+};
+
 template <int K>
 __device__ __forceinline__ int shift_k(const Geom& g, int ck, int j)
 {
@@ -136,51 +146,47 @@ __device__ __forceinline__ int shift_t(const Geom& g, int ct, int T)
     return (c - ct) * g.S[0];
 }
 
-// For one site x and spatial direction K: all loops W(R, T) with R in [r0, r0+RC) and T in
-// [tlo, thi], by line products (compute_wloop, wilson.c:21-56, factored):
+// For one site x and spatial direction K: the launch's loops W(R, T), by line products (compute_wloop, wilson.c:21-56, factored):
 //   W = (1/2) Re tr [T_T(x) S_R(x+T t) T_T(x+R k)^dag S_R(x)^dag] = <T_T(x) S_R(x+T t), S_R(x) T_T(x+R k)>
 // with T_T(y) = U_0(y) U_0(y+t) ... (T links) and S_R(y) = U_K(y) ... U_K(y+(R-1)k) (R links).
 // Temporal lines grow by one link per T; spatial lines at x+T t are rebuilt per T.
 template <typename R, int K, int RC>
-__device__ __forceinline__ void wilson_site(const Field<R>& U, const Geom& g, const Site& s, int par, int r0, int tlo,
-                                            int thi, DD* __restrict__ wacc)
+__device__ __forceinline__ void wilson_site(const Field<R>& U, const Geom& g, const Site& s, int par, const WilsonLoops& l,
+                                            bool valid, DD* __restrict__ wacc)
 {
     const int lane = threadIdx.x & 31;
     Q<R> SX[RC], TR[RC];
-    int xr[RC];   // lexicographic index of x + (r0 + r) k
+    int xr[RC];   // lexicographic index of x + R k
     // spatial lines at x
     Q<R> S = q_one<R>();
-    for (int j = 0; j < r0 - 1; ++j) S = q_mul(S, U.ld(K, par ^ (j & 1), s.n + shift_k<K>(g, s.c[K], j)));
+    int j = 0;
 #pragma unroll
     for (int r = 0; r < RC; ++r) {
-        const int j = r0 - 1 + r;
-        S = q_mul(S, U.ld(K, par ^ (j & 1), s.n + shift_k<K>(g, s.c[K], j)));
+        for (; j < l.r[r]; ++j) S = q_mul(S, U.ld(K, par ^ (j & 1), s.n + shift_k<K>(g, s.c[K], j)));
         SX[r] = S;
-        xr[r] = s.n + shift_k<K>(g, s.c[K], j + 1);
+        xr[r] = s.n + shift_k<K>(g, s.c[K], l.r[r]);
         TR[r] = q_one<R>();
     }
     Q<R> TX = q_one<R>();
-    for (int T = 1; T <= thi; ++T) {
+    for (int T = 1; T <= l.thi; ++T) {
         const int tprev = shift_t(g, s.c[0], T - 1), tcur = shift_t(g, s.c[0], T);
         const int pprev = par ^ ((T - 1) & 1);
         TX = q_mul(TX, U.ld(0, pprev, s.n + tprev));
 #pragma unroll
-        for (int r = 0; r < RC; ++r) TR[r] = q_mul(TR[r], U.ld(0, pprev ^ ((r0 + r) & 1), xr[r] + tprev));
+        for (int r = 0; r < RC; ++r) TR[r] = q_mul(TR[r], U.ld(0, pprev ^ (l.r[r] & 1), xr[r] + tprev));
+        if (!l.records(T)) continue;
         // spatial lines at x + T t
         const int pT = par ^ (T & 1);
         Q<R> ST = q_one<R>();
-        for (int j = 0; j < r0 - 1; ++j)
-            ST = q_mul(ST, U.ld(K, pT ^ (j & 1), s.n + tcur + shift_k<K>(g, s.c[K], j)));
+        j = 0;
 #pragma unroll
         for (int r = 0; r < RC; ++r) {
-            const int j = r0 - 1 + r;
-            ST = q_mul(ST, U.ld(K, pT ^ (j & 1), s.n + tcur + shift_k<K>(g, s.c[K], j)));
-            double w = 0.0;
-            if (T >= tlo) w = (double)q_dot(q_mul(TX, ST), q_mul(SX[r], TR[r]));
+            for (; j < l.r[r]; ++j) ST = q_mul(ST, U.ld(K, pT ^ (j & 1), s.n + tcur + shift_k<K>(g, s.c[K], j)));
+            double w = valid ? (double)q_dot(q_mul(TX, ST), q_mul(SX[r], TR[r])) : 0.0;
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
-            if (T >= tlo && lane == 0) {
-                DD* slot = wacc + r * kWilsonTChunk + (T - tlo);
+            if (lane == 0) {
+                DD* slot = wacc + r * kWilsonTChunk + (T - l.tlo);
                 *slot = dd_add(*slot, w);
             }
         }
@@ -188,8 +194,7 @@ __device__ __forceinline__ void wilson_site(const Field<R>& U, const Geom& g, co
 }
 
 template <typename R, int RC>
-__global__ void __launch_bounds__(kBlock) k_wilson(Field<R> U, Geom g, int r0, int tlo, int thi,
-                                                   DD* __restrict__ partials)
+__global__ void __launch_bounds__(kBlock) k_wilson(Field<R> U, Geom g, WilsonLoops l, DD* __restrict__ partials)
 {
     __shared__ DD wacc[kWilsonWarps][RC * kWilsonTChunk];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -205,26 +210,24 @@ __global__ void __launch_bounds__(kBlock) k_wilson(Field<R> U, Geom g, int r0, i
         int par;
         const Site s = site_lex(g, ii, par);
         DD* acc = &wacc[warp][0];
-        // Lanes past the end recompute a valid site with an empty record window (tlo > thi).  Every
-        // lane makes the same calls, so each full-mask shuffle inside is one instruction executed
-        // by the whole warp.
-        const int tlo_lane = valid ? tlo : thi + 1;
-        wilson_site<R, 1, RC>(U, g, s, par, r0, tlo_lane, thi, acc);
-        wilson_site<R, 2, RC>(U, g, s, par, r0, tlo_lane, thi, acc);
-        wilson_site<R, 3, RC>(U, g, s, par, r0, tlo_lane, thi, acc);
+        // Lanes past the end recompute a valid site and add 0.  Every lane makes the same calls, so each
+        // full-mask shuffle inside is one instruction executed by the whole warp.
+        wilson_site<R, 1, RC>(U, g, s, par, l, valid, acc);
+        wilson_site<R, 2, RC>(U, g, s, par, l, valid, acc);
+        wilson_site<R, 3, RC>(U, g, s, par, l, valid, acc);
     }
     __syncthreads();
     // fixed-order sum over warps, one partial per slot
-    for (int j = threadIdx.x; j < RC * kWilsonTChunk; j += blockDim.x) {
+    for (int i = threadIdx.x; i < RC * l.nT(); i += blockDim.x) {
         DD v = {0.0, 0.0};
-        for (int w = 0; w < kWilsonWarps; ++w) v = dd_add(v, wacc[w][j]);
-        partials[(size_t)j * kMaxPartials + blockIdx.x] = v;
+        for (int w = 0; w < kWilsonWarps; ++w) v = dd_add(v, wacc[w][i / l.nT() * kWilsonTChunk + i % l.nT()]);
+        partials[(size_t)i * kMaxPartials + blockIdx.x] = v;
     }
 }
 
 // Column form of the same sums.  A CTA owns `sw` consecutive spatial sites s (the lexicographic
 // index within a time slice) in every time slice; thread t * sw + j takes site t S0 + s0 + j.  Per
-// spatial direction K each thread stores its spatial lines S_{r0+r}(x) in shared memory, so the
+// spatial direction K each thread stores its spatial lines S_R(x) in shared memory, so the
 // line at x + T t that the loop needs for every T is the one the thread of slice t + T stored:
 // it is read, not rebuilt, which removes the longest product chain of the per-site form.
 constexpr int kWilsonColMaxThreads = 512;
@@ -286,25 +289,37 @@ __device__ __forceinline__ void wilson_acc(double* __restrict__ wacc, R (&w)[RC]
 // U_t(x + R k) does not depend on T, so the T loop loads nothing from global memory: Y^{T-1}(x + t)
 // is the value the thread one time slice up (thread (t+1) sw + j, periodic) wrote into a
 // double-buffered shared array, one barrier per T; two products per (R, T) and site.
-template <typename R, int K, int RC>
+template <typename R, int K, int RC, bool DENSE>
 __device__ __forceinline__ void wilson_col_dir(const Field<R>& U, const Geom& g, Q<R>* __restrict__ ybuf,
                                                double* __restrict__ wacc, int sw, int t, int j, int s, bool valid,
-                                               int r0, int tlo, int thi)
+                                               const WilsonLoops& l)
 {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nT = thi - tlo + 1;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nT = l.nT();
     int par;
     const int n = t * g.S[0] + s;
     const Site st = site_lex(g, n, par);
-    Q<R> SX[RC], UR[RC], Y[RC];   // S_{r0+r}(x); U_t(x + (r0+r) k); the transported loop
+    Q<R> SX[RC], UR[RC], Y[RC];   // S_R(x); U_t(x + R k); the transported loop
     Q<R> S = q_one<R>();
-    for (int jj = 0; jj < r0 - 1; ++jj) S = q_mul(S, U.ld(K, par ^ (jj & 1), n + shift_k<K>(g, st.c[K], jj)));
+    if (DENSE) {   // consecutive extents: one link each after the first, loads free to run ahead
+        const int r0 = l.r[0];
+        for (int jj = 0; jj < r0 - 1; ++jj) S = q_mul(S, U.ld(K, par ^ (jj & 1), n + shift_k<K>(g, st.c[K], jj)));
 #pragma unroll
-    for (int r = 0; r < RC; ++r) {
-        const int jj = r0 - 1 + r;
-        S = q_mul(S, U.ld(K, par ^ (jj & 1), n + shift_k<K>(g, st.c[K], jj)));
-        SX[r] = S;
-        Y[r] = S;
-        UR[r] = U.ld(0, par ^ ((jj + 1) & 1), n + shift_k<K>(g, st.c[K], jj + 1));
+        for (int r = 0; r < RC; ++r) {
+            const int jj = r0 - 1 + r;
+            S = q_mul(S, U.ld(K, par ^ (jj & 1), n + shift_k<K>(g, st.c[K], jj)));
+            SX[r] = S;
+            Y[r] = S;
+            UR[r] = U.ld(0, par ^ ((jj + 1) & 1), n + shift_k<K>(g, st.c[K], jj + 1));
+        }
+    } else {
+        int jj = 0;
+#pragma unroll
+        for (int r = 0; r < RC; ++r) {
+            for (; jj < l.r[r]; ++jj) S = q_mul(S, U.ld(K, par ^ (jj & 1), n + shift_k<K>(g, st.c[K], jj)));
+            SX[r] = S;
+            Y[r] = S;
+            UR[r] = U.ld(0, par ^ (l.r[r] & 1), n + shift_k<K>(g, st.c[K], l.r[r]));
+        }
     }
     const Q<R> UT = U.ld(0, par, n);
     int tn = t + 1;
@@ -312,18 +327,18 @@ __device__ __forceinline__ void wilson_col_dir(const Field<R>& U, const Geom& g,
     // buffer layout [T & 1][r][thread]: a warp's 16-byte accesses to one r are consecutive, so they
     // are free of bank conflicts (a per-thread block of RC loops put lanes RC * 16 bytes apart)
     const int up = tn * sw + j, nt = blockDim.x;
-    for (int T = 1; T <= thi; ++T) {
+    for (int T = 1; T <= l.thi; ++T) {
         Q<R>* buf = ybuf + (size_t)(T & 1) * nt * RC;
 #pragma unroll
         for (int r = 0; r < RC; ++r) buf[(size_t)r * nt + threadIdx.x] = Y[r];
         __syncthreads();   // the other buffer was last read before the previous barrier
 #pragma unroll
         for (int r = 0; r < RC; ++r) Y[r] = q_mul_nd(q_mul(UT, buf[(size_t)r * nt + up]), UR[r]);
-        if (T < tlo) continue;
+        if (!l.records(T)) continue;
         R w[RC];
 #pragma unroll
         for (int r = 0; r < RC; ++r) w[r] = valid ? q_dot(Y[r], SX[r]) : R(0);
-        wilson_acc<R, RC>(wacc, w, T - tlo, nT, warp, lane);
+        wilson_acc<R, RC>(wacc, w, T - l.tlo, nT, warp, lane);
     }
     __syncthreads();   // the buffers are written again by the next direction
 }
@@ -332,13 +347,14 @@ __device__ __forceinline__ void wilson_col_dir(const Field<R>& U, const Geom& g,
 // kWilsonRc8MaxThreads threads (96-thread CTAs at 48^4) so that they need not spill: the R <= 9 set
 // took 3.95 ms against 4.25 ms with four loops (FP32) and 9.87 against 10.10 ms with two loops in
 // 288-thread CTAs (FP64).  These widths are chosen only where a column fits the cap.
-template <typename R, int RC>
-__global__ void __launch_bounds__((sizeof(R) == 4 && RC >= 8) || (sizeof(R) == 8 && RC >= 4) ? kWilsonRc8MaxThreads : kWilsonColMaxThreads, 1) k_wilson_col(Field<R> U, Geom g, int sw, int r0, int tlo,
-                                                                        int thi, DD* __restrict__ partials)
+// DENSE: the launch's extents are consecutive.
+template <typename R, int RC, bool DENSE>
+__global__ void __launch_bounds__((sizeof(R) == 4 && RC >= 8) || (sizeof(R) == 8 && RC >= 4) ? kWilsonRc8MaxThreads : kWilsonColMaxThreads, 1)
+    k_wilson_col(Field<R> U, Geom g, int sw, WilsonLoops l, DD* __restrict__ partials)
 {
     extern __shared__ __align__(16) unsigned char wsm[];
     Q<R>* ybuf = (Q<R>*)wsm;   // two buffers of RC loops per thread
-    const int nwarps = blockDim.x >> 5, nT = thi - tlo + 1;
+    const int nwarps = blockDim.x >> 5, nT = l.nT();
     double* wacc = (double*)(wsm + (size_t)2 * blockDim.x * RC * sizeof(Q<R>));
     const int owners = wilson_thread_slots<R>() ? (int)blockDim.x : nwarps;
     for (int i = threadIdx.x; i < owners * RC * nT; i += blockDim.x) wacc[i] = 0.0;
@@ -349,25 +365,24 @@ __global__ void __launch_bounds__((sizeof(R) == 4 && RC >= 8) || (sizeof(R) == 8
         const int s_req = tile * sw + j;
         const bool valid = s_req < stot;
         const int s = valid ? s_req : stot - 1;   // threads past the end read a valid site and add 0
-        wilson_col_dir<R, 1, RC>(U, g, ybuf, wacc, sw, t, j, s, valid, r0, tlo, thi);
-        wilson_col_dir<R, 2, RC>(U, g, ybuf, wacc, sw, t, j, s, valid, r0, tlo, thi);
-        wilson_col_dir<R, 3, RC>(U, g, ybuf, wacc, sw, t, j, s, valid, r0, tlo, thi);
+        wilson_col_dir<R, 1, RC, DENSE>(U, g, ybuf, wacc, sw, t, j, s, valid, l);
+        wilson_col_dir<R, 2, RC, DENSE>(U, g, ybuf, wacc, sw, t, j, s, valid, l);
+        wilson_col_dir<R, 3, RC, DENSE>(U, g, ybuf, wacc, sw, t, j, s, valid, l);
     }
-    // fixed-order sum over warps; slot r * kWilsonTChunk + (T - tlo) as in k_wilson
+    // fixed-order sum over warps; slot r nT + (T - tlo) as in k_wilson
     for (int i = threadIdx.x; i < RC * nT; i += blockDim.x) {
-        const int r = i / nT, ti = i % nT;
         DD v = {0.0, 0.0};
-        for (int w = 0; w < owners; ++w) v = dd_add(v, wacc[((size_t)r * nT + ti) * owners + w]);
-        partials[(size_t)(r * kWilsonTChunk + ti) * kMaxPartials + blockIdx.x] = v;
+        for (int w = 0; w < owners; ++w) v = dd_add(v, wacc[(size_t)i * owners + w]);
+        partials[(size_t)i * kMaxPartials + blockIdx.x] = v;
     }
 }
 
 // Spatial sites per CTA for the column kernel: the smallest sw with L_t sw a multiple of 32 and at
 // least `min_threads` threads; 0 if that exceeds kWilsonColMaxThreads (the per-site kernel then
 // runs).  Wide CTAs read longer runs of consecutive sites; small ones pack the SM's four schedulers
-// evenly.  Measured at 24^4 and 48^4 on B200: the FP32 R-chunk-4 kernel (106 registers, 4 warps per
-// scheduler) is fastest with ~96 threads (a 288-thread CTA left room for one CTA per SM), every
-// other instance with >= 256 threads (FP64 chunk 4: 23.4 ms against 26.7 ms at 96 threads).
+// evenly.  Measured at 24^4 and 48^4 on B200: chunks of four and eight loops are fastest with ~96 threads,
+// those of one and two with ~128 (W(1,1), W(1,5), W(5,1), W(5,5) at 48^4, ms, with 64, 128 and 256: FP64
+// 1.43, 1.15, 1.26, FP32 0.87, 0.61, 0.66).
 int wilson_col_width(const Geom& g, int min_threads = 256)
 {
     int a = g.L[0], b = 32;
@@ -562,50 +577,52 @@ void launch_ape(su2g_lattice* h, void* const in_dirs[4], void* const out_dirs[4]
 
 // Launch one chunk of loops; returns the number of CTAs (= partials per slot), 0 on a launch error.
 template <typename R, int RC>
-int launch_wilson_t(su2g_lattice* h, void* const dirs[4], int r0, int tlo, int thi)
+int launch_wilson_t(su2g_lattice* h, void* const dirs[4], const WilsonLoops& l, bool dense)
 {
     const Field<R> U = make_field<R>(dirs, h->g.Vh);
-    const int sw = wilson_col_width(h->g, (sizeof(R) == 4 && RC >= 4) || (sizeof(R) == 8 && RC >= 4) ? 64 : 256);
+    const int sw = wilson_col_width(h->g, RC >= 4 ? 64 : 128);
     if (sw > 0) {
         const int threads = sw * h->g.L[0];
-        const size_t smem = wilson_col_smem<R, RC>(threads, thi - tlo + 1);
+        const size_t smem = wilson_col_smem<R, RC>(threads, l.nT());
         int per_sm = 0;
+        auto* kernel = RC == 1 || dense ? k_wilson_col<R, RC, true> : k_wilson_col<R, RC, RC == 1>;
         if (smem <= (size_t)h->max_smem &&
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_wilson_col<R, RC>, threads, smem) == cudaSuccess &&
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) == cudaSuccess &&
             per_sm > 0) {
             const int ntiles = (h->g.S[0] + sw - 1) / sw;
             const int grid = std::max(1, std::min(std::min(ntiles, h->num_sms * per_sm), kMaxPartials));
-            k_wilson_col<R, RC><<<grid, threads, smem, h->stream>>>(U, h->g, sw, r0, tlo, thi, h->partials);
+            kernel<<<grid, threads, smem, h->stream>>>(U, h->g, sw, l, h->partials);
             return grid;
         }
         cudaGetLastError();
     }
     const int grid = resident_grid(h, (const void*)k_wilson<R, RC>, h->g.V);
-    k_wilson<R, RC><<<grid, kBlock, 0, h->stream>>>(U, h->g, r0, tlo, thi, h->partials);
+    k_wilson<R, RC><<<grid, kBlock, 0, h->stream>>>(U, h->g, l, h->partials);
     return grid;
 }
 
 template <typename R>
-int launch_wilson(su2g_lattice* h, void* const dirs[4], int rc, int r0, int tlo, int thi)
+int launch_wilson(su2g_lattice* h, void* const dirs[4], int rc, const WilsonLoops& l, bool dense)
 {
     switch (rc) {
-        case 1: return launch_wilson_t<R, 1>(h, dirs, r0, tlo, thi);
-        case 2: return launch_wilson_t<R, 2>(h, dirs, r0, tlo, thi);
-        case 4: return launch_wilson_t<R, 4>(h, dirs, r0, tlo, thi);
-        default: return launch_wilson_t<R, 8>(h, dirs, r0, tlo, thi);
+        case 1: return launch_wilson_t<R, 1>(h, dirs, l, dense);
+        case 2: return launch_wilson_t<R, 2>(h, dirs, l, dense);
+        case 4: return launch_wilson_t<R, 4>(h, dirs, l, dense);
+        default: return launch_wilson_t<R, 8>(h, dirs, l, dense);
     }
 }
 
-template <typename R, int RC>
+template <typename R, int RC, bool DENSE = true>
 void wilson_smem_attr(int bytes)
 {
-    cudaFuncSetAttribute(k_wilson_col<R, RC>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (DENSE && RC > 1) wilson_smem_attr<R, RC, RC == 1>(bytes);
+    cudaFuncSetAttribute(k_wilson_col<R, RC, DENSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     // the small FP32 CTAs (96 threads, two buffers of RC loops, ~13 KB) fit six per SM by their
     // registers and need ~80 KB of shared memory for that; without a preference the driver picked a
     // 32 KB carveout.  The FP64 instances keep the default, which leaves L1 its room (a maximal
     // carveout cost FP64 5 %).
     if (sizeof(R) == 4 && RC >= 4)
-        cudaFuncSetAttribute(k_wilson_col<R, RC>, cudaFuncAttributePreferredSharedMemoryCarveout, 50);
+        cudaFuncSetAttribute(k_wilson_col<R, RC, DENSE>, cudaFuncAttributePreferredSharedMemoryCarveout, 50);
 }
 
 }  // namespace
@@ -752,42 +769,55 @@ int su2g::wilson_check(su2g_lattice* h, const int32_t* R, const int32_t* T, int 
 int su2g::wilson_enqueue(su2g_lattice* h, void* const dirs[4], const int32_t* R, const int32_t* T, int n, int out_off,
                          int max_slots, int* slot)
 {
-    int rmax = 0, tmax = 0;
-    for (int i = 0; i < n; ++i) {
-        rmax = std::max(rmax, (int)R[i]);
-        tmax = std::max(tmax, (int)T[i]);
-    }
-    std::vector<char> want((size_t)rmax * tmax, 0);
-    for (int i = 0; i < n; ++i) want[(size_t)(R[i] - 1) * tmax + (T[i] - 1)] = 1;
-    // R in chunks of 8/4/2/1, T in chunks of kWilsonTChunk; a chunk with no wanted pair is skipped
+    int tmax = 0;
+    for (int i = 0; i < n; ++i) tmax = std::max(tmax, (int)T[i]);
+    std::vector<int> rs(R, R + n);   // the distinct spatial extents
+    std::sort(rs.begin(), rs.end());
+    rs.erase(std::unique(rs.begin(), rs.end()), rs.end());
+    const int nr = (int)rs.size();
+    std::vector<int> ri(n);          // each pair's index among them
+    for (int i = 0; i < n; ++i) ri[i] = (int)(std::lower_bound(rs.begin(), rs.end(), (int)R[i]) - rs.begin());
+    // The wanted R in chunks of 8/4/2/1, T in windows of at most kWilsonTChunk from the first to the last
+    // wanted one.  Lines and transported loops of extents nobody asked for are not formed: W(1,1), W(1,5),
+    // W(5,1), W(5,5) take one launch of two loops a thread instead of four (R <= 4) and one (R = 5), at
+    // 24^4 on B200 238 -> 103 us FP64, 139 -> 66 us FP32 a call.
     struct Chunk {
-        int rc_n, r0, tlo, thi, base;
+        int rc_n, base;
+        bool dense;
+        WilsonLoops l;
     };
     std::vector<Chunk> plan;
-    std::vector<int> slot_rt((size_t)rmax * tmax, -1);
     int used = 0;
     // the column kernel transports its loops in time, so a narrow R chunk costs it only the rebuild
-    // of its spatial lines: FP32 runs chunks of 4 loops per thread, FP64 of 2 (4 spills in FP64:
-    // 22.5 ms against 11.2 ms for W(R, T <= 9) at 48^4); the per-site kernel prefers 8
+    // of its spatial lines: at most 8 (FP32) or 4 (FP64) loops per thread where a column fits
+    // kWilsonRc8MaxThreads, 4 or 2 in wider columns (more spill); the per-site kernel prefers 8
     const int sw8 = wilson_col_width(h->g, 64);
     const bool rc8 = sw8 > 0 && sw8 * h->g.L[0] <= kWilsonRc8MaxThreads;
     const int rc_max = wilson_col_width(h->g) > 0 ? (h->prec == SU2G_FP32 ? (rc8 ? 8 : 4) : (rc8 ? 4 : 2)) : 8;
-    for (int r0 = 1; r0 <= rmax;) {
-        const int left = rmax - r0 + 1;
-        const int rc_n = left >= 8 && rc_max >= 8 ? 8 : (left >= 4 ? 4 : (left >= 2 ? 2 : 1));
-        for (int tlo = 1; tlo <= tmax; tlo += kWilsonTChunk) {
-            const int thi = std::min(tmax, tlo + kWilsonTChunk - 1);
-            bool any = false;
-            for (int r = r0; r < r0 + rc_n; ++r)
-                for (int t = tlo; t <= thi; ++t) any = any || want[(size_t)(r - 1) * tmax + (t - 1)];
-            if (!any) continue;
-            plan.push_back({rc_n, r0, tlo, thi, out_off + used});
-            for (int r = 0; r < rc_n; ++r)
-                for (int t = tlo; t <= thi; ++t)
-                    slot_rt[(size_t)(r0 + r - 1) * tmax + (t - 1)] = out_off + used + r * kWilsonTChunk + (t - tlo);
-            used += rc_n * kWilsonTChunk;
+    for (int i0 = 0; i0 < nr;) {
+        int rc_n = rc_max;
+        while (rc_n > nr - i0) rc_n >>= 1;
+        for (int t0 = 1; t0 <= tmax; t0 += kWilsonTChunk) {
+            uint32_t want = 0;
+            for (int i = 0; i < n; ++i)
+                if (ri[i] >= i0 && ri[i] < i0 + rc_n && T[i] >= t0 && T[i] < t0 + kWilsonTChunk) want |= 1u << (T[i] - t0);
+            if (!want) continue;
+            Chunk c{rc_n, out_off + used, false, {}};
+            int lo = 0, hi = kWilsonTChunk - 1;
+            while (!(want >> lo & 1u)) ++lo;
+            while (!(want >> hi & 1u)) --hi;
+            c.l.tlo = t0 + lo;
+            c.l.thi = t0 + hi;
+            c.l.want = want >> lo;
+            for (int r = 0; r < 8; ++r) c.l.r[r] = rs[std::min(i0 + r, nr - 1)];
+            c.dense = rs[i0 + rc_n - 1] - rs[i0] == rc_n - 1;
+            plan.push_back(c);
+            for (int i = 0; i < n; ++i)
+                if (ri[i] >= i0 && ri[i] < i0 + rc_n && T[i] >= c.l.tlo && T[i] <= c.l.thi)
+                    slot[i] = c.base + (ri[i] - i0) * c.l.nT() + (T[i] - c.l.tlo);
+            used += rc_n * c.l.nT();
         }
-        r0 += rc_n;
+        i0 += rc_n;
     }
     if (used > max_slots)
         return set_error(h, SU2G_EINVAL, "Wilson loops: %d result slots needed, %d available", used, max_slots);
@@ -795,14 +825,13 @@ int su2g::wilson_enqueue(su2g_lattice* h, void* const dirs[4], const int32_t* R,
     if (rc) return rc;
     for (const Chunk& c : plan) {
         launch_begin(h, SU2G_K_WILSON);
-        const int grid = h->prec == SU2G_FP32 ? launch_wilson<float>(h, dirs, c.rc_n, c.r0, c.tlo, c.thi)
-                                              : launch_wilson<double>(h, dirs, c.rc_n, c.r0, c.tlo, c.thi);
+        const int grid = h->prec == SU2G_FP32 ? launch_wilson<float>(h, dirs, c.rc_n, c.l, c.dense)
+                                              : launch_wilson<double>(h, dirs, c.rc_n, c.l, c.dense);
         if ((rc = launch_end(h, SU2G_K_WILSON, "Wilson loop kernel"))) return rc;
         // W = sum_x,k c0 / (3 V)  (wilson.c:322: sum of Re tr / (3 V 2))
-        if ((rc = finalize(h, h->partials, grid, c.rc_n * kWilsonTChunk, kMaxPartials, 1.0 / (3.0 * (double)h->g.V),
+        if ((rc = finalize(h, h->partials, grid, c.rc_n * c.l.nT(), kMaxPartials, 1.0 / (3.0 * (double)h->g.V),
                            h->d_out + c.base))) return rc;
     }
-    for (int i = 0; i < n; ++i) slot[i] = slot_rt[(size_t)(R[i] - 1) * tmax + (T[i] - 1)];
     return SU2G_OK;
 }
 
