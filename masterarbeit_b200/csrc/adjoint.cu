@@ -161,11 +161,16 @@ __global__ void __launch_bounds__(kBlock) k_line_chain(Field<R> Unc, Field<R> L2
 
 // ------------------------------------------------------ one APE step back ---
 
+// 128-thread CTAs for both kernels; per SM four (FP32) and three (FP64) for v-bar, five and four for the
+// gather, whose loads otherwise all run ahead (202 registers in FP64).  A VJP of five steps at 24^4, us:
+// FP64 1552 -> 1361, FP32 785 -> 740 against two 256-thread CTAs for v-bar and no bound for the gather.
+constexpr int kSmearAdjBlock = 128;
+
 // v-bar(x, mu) = (Gn - u' <u', Gn>) / |v|,  v = U + alpha S,  u' = v / |v|  (all four directions).
 // The staple sums are the forward step's own (ape_staples), so v is exactly the forward's
-// pre-projection link; same site order and occupancy as the forward kernel.
+// pre-projection link.
 template <typename R>
-__global__ void __launch_bounds__(kBlock, 2) k_ape_vbar(Field<R> U, Field<R> Gnc, Field<R> Vbar, Geom g, R alpha)
+__global__ void __launch_bounds__(kSmearAdjBlock, sizeof(R) == 4 ? 4 : 3) k_ape_vbar(Field<R> U, Field<R> Gnc, Field<R> Vbar, Geom g, R alpha)
 {
     pdl_trigger();
     Site s{};
@@ -233,7 +238,7 @@ __device__ __forceinline__ void gather_link(const FieldCA<R>& U, const FieldCA<R
 // of the same 32 half-volume indices (site_warp_pair): every warp reads consecutive links of one
 // parity array, and both parities of a region are loaded by the same SM.
 template <typename R>
-__global__ void __launch_bounds__(kBlock) k_ape_gather(Field<R> Unc, Field<R> Vbnc, Field<R> G, Geom g, R alpha)
+__global__ void __launch_bounds__(kSmearAdjBlock, sizeof(R) == 4 ? 5 : 4) k_ape_gather(Field<R> Unc, Field<R> Vbnc, Field<R> G, Geom g, R alpha)
 {
     pdl_trigger();
     Site s{};
@@ -385,9 +390,9 @@ int vjp_t(su2g_lattice* h, int n_ape, double alpha, int c, double* q_out, double
             Field<R> Gn = make_field<R>(G[gi].dirs, g.Vh), Gk = make_field<R>(G[gi ^ 1].dirs, g.Vh);
             Field<R> Vbf = make_field<R>(Vb.dirs, g.Vh);
             launch_begin(h, SU2G_K_OTHER);
-            const int blocks = 2 * (int)((g.Vh + kBlock - 1) / kBlock);
-            launch_pdl(k_ape_vbar<R>, blocks, kBlock, h->stream, Uk, Gn, Vbf, g, (R)alpha);
-            launch_pdl(k_ape_gather<R>, dim3(blocks, 4), kBlock, h->stream, Uk, Vbf, Gk, g, (R)alpha);
+            const int blocks = (g.V + kSmearAdjBlock - 1) / kSmearAdjBlock;
+            launch_pdl(k_ape_vbar<R>, blocks, kSmearAdjBlock, h->stream, Uk, Gn, Vbf, g, (R)alpha);
+            launch_pdl(k_ape_gather<R>, dim3(blocks, 4), kSmearAdjBlock, h->stream, Uk, Vbf, Gk, g, (R)alpha);
             if ((rc = launch_end(h, SU2G_K_OTHER, "smearing adjoint kernels"))) return rc;
             gi ^= 1;
         }
