@@ -64,9 +64,11 @@ struct AosField {
     __device__ __forceinline__ Q<double> ld(int mu, int, int n) const
     {
         const double2* a = p + 2 * ((size_t)n * 4 + mu);
-        if (A32) return ldnc_256(reinterpret_cast<const Vec4d*>(a));
-        const double2 x = __ldg(a), y = __ldg(a + 1);
-        return q_make<double>(x.x, x.y, y.x, y.y);
+        if (A32) return ld_256(reinterpret_cast<const Vec4d*>(a));
+        Q<double> q;
+        asm("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(q.c0), "=d"(q.c1) : "l"(a));
+        asm("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(q.c2), "=d"(q.c3) : "l"(a + 1));
+        return q;
     }
     __device__ __forceinline__ void st(int mu, int n, const Q<double>& q) const
     {
@@ -98,28 +100,35 @@ struct AtSite {
 
 // One Jacobi step from `in` into `out`: the links of the smeared directions become Proj(U + alpha S)
 // with the staples of smearing.c:42-71; with COPY the other directions are copied.  One site per thread, parities paired per warp as in the handle's kernel,
-// whose staple sums these are.
+// whose staple sums these are, and launched like it: a step starts in the tail of the one before.
 template <int MODE, bool COPY, typename In, typename Out>
-__global__ void __launch_bounds__(128) k_ape_any(In in, Out out, Geom g, double alpha)
+__global__ void __launch_bounds__(128, MODE == SU2G_APE_ALL ? 3 : (MODE == SU2G_APE_SPATIAL ? 4 : 8)) k_ape_any(In in, Out out, Geom g, double alpha)
 {
-    Site s;
+    pdl_trigger();
+    Site s{};
     int par, h;
-    if (!site_warp_pair(g, blockIdx.x, threadIdx.x, blockDim.x, s, par, h)) return;
+    const bool valid = site_warp_pair(g, blockIdx.x, threadIdx.x, blockDim.x, s, par, h);
+    pdl_wait(h, s.n);
+    if (!valid) return;
     const AtSite<In> at{in, s.n};
+    Q<double> res[4];
 #pragma unroll
     for (int mu = 0; mu < 4; ++mu)
-        if (COPY && !ape_updates(MODE, mu)) put(out, mu, par, h, s.n, in.ld(mu, par, s.n));
+        if (COPY && !ape_updates(MODE, mu)) res[mu] = in.ld(mu, par, s.n);
     ape_staples<double, MODE>(at, g, s, par, h, [&](int mu, const Q<double>& u, const Q<double>& S) {
-        put(out, mu, par, h, s.n, q_project(q_axpy(alpha, S, u)));
+        res[mu] = q_project(q_axpy(alpha, S, u));
     });
+#pragma unroll
+    for (int mu = 0; mu < 4; ++mu)
+        if (COPY || ape_updates(MODE, mu)) put(out, mu, par, h, s.n, res[mu]);
 }
 
 // Checkerboarded field with its smeared directions in one buffer and the others in another.
-Field<double> checkerboard(void* base, void* fixed, const Geom& g, int mode)
+FieldCA<double> checkerboard(void* base, void* fixed, const Geom& g, int mode)
 {
     void* dirs[4];
     for (int mu = 0; mu < 4; ++mu) dirs[mu] = (char*)(ape_updates(mode, mu) ? base : fixed) + (size_t)mu * g.V * 32;
-    return make_field<double>(dirs, g.Vh);
+    return field_ca(make_field<double>(dirs, g.Vh));
 }
 
 template <bool COPY, typename In, typename Out>
@@ -127,9 +136,9 @@ void step(const In& in, const Out& out, const Geom& g, int mode, double alpha, c
 {
     const int grid = (g.V + 127) / 128;
     switch (mode) {
-        case SU2G_APE_ALL: k_ape_any<SU2G_APE_ALL, COPY><<<grid, 128, 0, st>>>(in, out, g, alpha); break;
-        case SU2G_APE_SPATIAL: k_ape_any<SU2G_APE_SPATIAL, COPY><<<grid, 128, 0, st>>>(in, out, g, alpha); break;
-        default: k_ape_any<SU2G_APE_TEMPORAL, COPY><<<grid, 128, 0, st>>>(in, out, g, alpha); break;
+        case SU2G_APE_ALL: launch_pdl(k_ape_any<SU2G_APE_ALL, COPY, In, Out>, grid, 128, st, in, out, g, alpha); break;
+        case SU2G_APE_SPATIAL: launch_pdl(k_ape_any<SU2G_APE_SPATIAL, COPY, In, Out>, grid, 128, st, in, out, g, alpha); break;
+        default: launch_pdl(k_ape_any<SU2G_APE_TEMPORAL, COPY, In, Out>, grid, 128, st, in, out, g, alpha); break;
     }
 }
 
@@ -195,7 +204,7 @@ extern "C" int su2g_ape_inplace_noalloc(double* links, const int32_t dims[4], in
     // whose loads are contiguous over a warp (the site-major one touches a line per lane), and only in
     // the directions the mode changes: the others stay where the first step copied them, in the
     // scratch -- or, for a last step that reads the field and writes over the scratch, where the second
-    // step copied them again.  Twenty spatial steps at 20x16x18x14 on B200: 173 us, against 819 us
+    // step copied them again.  Twenty spatial steps at 20x16x18x14 on B200: 135 us (173 us without overlapping launches), against 819 us
     // with every level site-major, one direction after another and no shared products.  A field that is
     // not 32-byte aligned keeps its own layout throughout.
     const bool a32 = ((uintptr_t)links & 31u) == 0;
@@ -204,7 +213,7 @@ extern "C" int su2g_ape_inplace_noalloc(double* links, const int32_t dims[4], in
         void *src = base[i & 1], *dst = base[(i & 1) ^ 1];
         const bool first = i == 0, last = i + 1 == ns, again = i == 1 && (ns & 1);
         const AosField<true> asrc{(double2*)src, g.Vh}, adst{(double2*)dst, g.Vh};
-        const Field<double> csrc = checkerboard(src, last && (ns & 1) ? src : scratch, g, mode),
+        const FieldCA<double> csrc = checkerboard(src, last && (ns & 1) ? src : scratch, g, mode),
                             cdst = checkerboard(dst, dst, g, mode);
         if (!a32) step<true>(AosField<false>{(double2*)src, g.Vh}, AosField<false>{(double2*)dst, g.Vh}, g, mode, alpha, st);
         else if (first && last) step<true>(asrc, adst, g, mode, alpha, st);

@@ -466,7 +466,7 @@ struct FieldCA<double> : Field<double> {
 };
 
 template <typename R>
-__device__ __forceinline__ FieldCA<R> field_ca(const Field<R>& f)
+__host__ __device__ __forceinline__ FieldCA<R> field_ca(const Field<R>& f)
 {
     FieldCA<R> c;
     for (int mu = 0; mu < 4; ++mu) c.p[mu] = f.p[mu];
