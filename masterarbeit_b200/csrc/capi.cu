@@ -449,6 +449,7 @@ extern "C" int su2g_create(const su2g_params* p, su2g_lattice** out)
     if (!rc) rc = check_cuda(h, cudaMemsetAsync(h->fin_ticket, 0, kFinSlots * sizeof(unsigned), h->stream), "clearing reduction counter");
     if (!rc) rc = ensure_partials(h, 2);
     if (!rc) wilson_prepare(h);
+    if (!rc) chain_prepare(h);
     if (!rc) rc = check_cuda(h, cudaEventCreate(&h->ev_begin), "creating events");
     if (!rc) rc = check_cuda(h, cudaEventCreate(&h->ev_end), "creating events");
     if (!rc) rc = su2g_start(h, p->start, p->seed);

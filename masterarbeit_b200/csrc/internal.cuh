@@ -132,6 +132,7 @@ struct su2g_lattice {
     cudaEvent_t ev_begin = nullptr, ev_end = nullptr;
     int max_smem = 0;            // opt-in shared memory per CTA
     size_t l2_bytes = 0;
+    bool chain = false;          // sweeps in one launch (chain.cu)
     int ape_variant = 0;         // 0: per-site APE kernel, 1: TMA-tiled FP32 APE_all where it applies
     cudaMemPool_t pool = nullptr;      // scratch of the adjoint; keeps its memory until destroy
     void* lines = nullptr;             // 2- and 3-link line products of the field Q is measured on
@@ -251,9 +252,16 @@ int launch_update(su2g_lattice* h, int kind, int mu, int par, uint32_t sweep, DD
 int sweep_warps(const su2g_lattice* h);
 int sweep_plaq_finalize(su2g_lattice* h, const DD* parts, int nslots, size_t stride, double* out, int out_stride = 1);
 int sweep_acc_finalize(su2g_lattice* h, const DD* parts, int nslots, size_t stride, double* out, int out_stride = 1);
+// Small FP64 lattices (h->chain): whole blocks of sweeps in one launch.  chain_prepare decides (once
+// per handle, at creation).  chain_enqueue runs n_blocks blocks of `every` x (n_hb + n_or) sub-sweeps; block
+// b's plaquette partials (plaq) and acceptance entries (acc 1: set, 2: added to) go to parts + b stride and + 3 sweep_warps.
+void chain_prepare(su2g_lattice* h);
+int chain_enqueue(su2g_lattice* h, int n_blocks, int every, int n_hb, int n_or, uint32_t sweep0, DD* parts, size_t stride,
+                  bool plaq, int acc);
+constexpr int kChainSubSweeps = 1024;   // sub-sweeps one launch runs at most (some 20 ms)
 // Enqueue n_sweeps x (n_hb heatbath + n_or overrelaxation sweeps); heatbath sub-sweep j (counted
-// from 0 within the call) has index sweep0 + j.  acc_part (there must be a heatbath sub-sweep) receives
-// the acceptance of them all; with plaq_part (there must be a sub-sweep) the last sub-sweep also leaves
-// the three fused passes' plaquette partials there.
-int sweep_enqueue(su2g_lattice* h, int n_sweeps, int n_hb, int n_or, uint32_t sweep0, DD* acc_part, DD* plaq_part);
+// from 0 within the call) has index sweep0 + j.  With plaq (there must be a sub-sweep) the last one leaves
+// its three fused passes' plaquette partials at parts, with acc (there must be a heatbath sub-sweep) the
+// acceptance of them all goes to parts + 3 sweep_warps.
+int sweep_enqueue(su2g_lattice* h, int n_sweeps, int n_hb, int n_or, uint32_t sweep0, DD* parts, bool plaq, bool acc);
 }  // namespace su2g

@@ -36,6 +36,8 @@ extern "C" int su2g_graph_run(su2g_lattice* h, int32_t n_blocks, int32_t meas_ev
     const bool fused = n_hb + n_or > 0, with_acc = n_hb > 0;
     const size_t warps = sweep_warps(h), parts = 4 * warps;   // a block's: the plaquette's three passes, the acceptance
     const int group = std::max<int>(1, std::min<size_t>(kFinSlots, kPlaqScratchBytes / (parts * sizeof(DD))));
+    const bool grouped = h->chain && fused && !h->profiling &&
+                         (long long)group * meas_every * (n_hb + n_or) <= kChainSubSweeps;
     int rc = fused ? ensure_partial_entries(h, parts * std::min(group, (int)n_blocks)) : SU2G_OK;
     const double nupd = (double)meas_every * n_hb * 4.0 * (double)h->g.V;
     // as many blocks at a time as there are result slots: slot 2i takes block i's plaquette, 2i + 1 its acceptance
@@ -44,8 +46,9 @@ extern "C" int su2g_graph_run(su2g_lattice* h, int32_t n_blocks, int32_t meas_ev
         for (int i = 0; i < n && !rc; ++i) {
             const int j = i % group;
             DD* part = h->partials + j * parts;
-            rc = sweep_enqueue(h, meas_every, n_hb, n_or, h->hb_sweeps, with_acc ? part + 3 * warps : nullptr,
-                               fused ? part : nullptr);
+            if (!grouped) rc = sweep_enqueue(h, meas_every, n_hb, n_or, h->hb_sweeps, part, fused, with_acc);
+            else if (j == 0)   // the whole group in one launch
+                rc = chain_enqueue(h, std::min(group, n - i), meas_every, n_hb, n_or, h->hb_sweeps, part, parts, true, with_acc);
             h->hb_sweeps += (uint32_t)(meas_every * n_hb);
             if (rc) break;
             double* out = h->d_out + 2 * (i - j);

@@ -12,6 +12,7 @@
 // the sweep, update.c:166), except an FP64 heatbath draw, which is unit to rounding (hb_store).
 // Randoms come from Philox keyed by (seed, site, sweep, dir, draw,
 // replica), so the result does not depend on grid shape or on which thread takes which link.
+#include <algorithm>
 #include <cfloat>
 #include <cmath>
 
@@ -340,10 +341,22 @@ extern "C" int su2g_update_pass(su2g_lattice* h, int32_t kind, int32_t mu, int32
     return launch_update(h, kind, mu, parity, sweep, nullptr, false, nullptr);
 }
 
-int su2g::sweep_enqueue(su2g_lattice* h, int n_sweeps, int n_hb, int n_or, uint32_t sweep0, DD* acc_part, DD* plaq_part)
+int su2g::sweep_enqueue(su2g_lattice* h, int n_sweeps, int n_hb, int n_or, uint32_t sweep0, DD* part0, bool with_plaq, bool with_acc)
 {
     const int parts = sweep_warps(h);   // per fused pass
+    DD *plaq_part = with_plaq ? part0 : nullptr, *acc_part = with_acc ? part0 + 3 * parts : nullptr;
     const int subs = n_sweeps * (n_hb + n_or);
+    if (h->chain && !h->profiling && n_hb + n_or > 0) {   // (profiling times every pass)
+        const int most = std::max(1, kChainSubSweeps / (n_hb + n_or));
+        for (int s = 0; s < n_sweeps; s += most) {
+            const int n = std::min(most, n_sweeps - s);
+            const bool plaq = plaq_part && s + n == n_sweeps;
+            const int rc = chain_enqueue(h, 1, n, n_hb, n_or, sweep0 + (uint32_t)(s * n_hb), part0, 0, plaq,
+                                         acc_part ? (s == 0 ? 1 : 2) : 0);
+            if (rc) return rc;
+        }
+        return SU2G_OK;
+    }
     int sub = 0;
     for (int s = 0; s < n_sweeps; ++s)
         for (int i = 0; i < n_hb + n_or; ++i) {
@@ -376,11 +389,10 @@ int sweep_call(su2g_lattice* h, int32_t n_sweeps, int32_t n_hb, int32_t n_or, do
     int rc = fused || acc ? ensure_partial_entries(h, 4 * warps) : SU2G_OK;
     if (rc) return rc;
     // partials: three passes of the plaquette, then the acceptance
-    DD *part = fused ? h->partials : nullptr, *acc_part = acc ? h->partials + 3 * warps : nullptr;
-    if ((rc = sweep_enqueue(h, n_sweeps, n_hb, n_or, h->hb_sweeps, acc_part, part))) return rc;
-    if (fused) rc = sweep_plaq_finalize(h, part, 1, 0, h->d_out + slot_plaq);
+    if ((rc = sweep_enqueue(h, n_sweeps, n_hb, n_or, h->hb_sweeps, h->partials, fused, acc))) return rc;
+    if (fused) rc = sweep_plaq_finalize(h, h->partials, 1, 0, h->d_out + slot_plaq);
     else if (plaq_out) rc = plaquette_enqueue(h, h->d_out + slot_plaq);
-    if (!rc && acc) rc = sweep_acc_finalize(h, acc_part, 1, 0, h->d_out + slot_acc);
+    if (!rc && acc) rc = sweep_acc_finalize(h, h->partials + 3 * warps, 1, 0, h->d_out + slot_acc);
     if (rc) return rc;
     h->hb_sweeps += (uint32_t)(n_sweeps * n_hb);
     if (acc_out || plaq_out) {
