@@ -62,17 +62,16 @@ __global__ void __launch_bounds__(128, 8) k_plaquette(Field<R> Unc, Geom g, DD* 
 
 // One Jacobi step U'_mu(x) = Proj(U_mu(x) + alpha S_mu(x)) (smearing.c:74-168) with the staple
 // sums of ape_staples (ape.cuh).  Reads `in`, writes only the updated directions of `out`.
-// 128-thread CTAs; resident CTAs per SM, measured at 48^4 on B200: FP32 APE_all four (at most 128
-// registers; 235.5 us against 238.8 us with five, 243 us with six, 254 us with two 256-thread
-// CTAs); FP32 spatial and temporal eight (131.4 us spatial against 132.6 us with four of 256, 136 us
-// with six, 164 us with two). FP64
-// APE_all three (619 us against 626 us with four, 655 us with two of 256), spatial four (337 us
-// against 359 us with three, 357 us with two of 256), temporal eight (212 against 216 us with four
-// of 256).
+// 128-thread CTAs; resident CTAs per SM, measured on B200: FP32 APE_all five (96 registers; ten steps at
+// 24^4 / 40x30x36x34 / 48^4: 153 / 658 / 2440 us against 158 / 699 / 2550 with four and 163 / 670 / 2490
+// with six); FP32 spatial and temporal eight (131.4 us spatial at 48^4 against 132.6 us with four of 256, 136 us
+// with six, 164 us with two).  FP64 APE_all three (24^4: 284 us ten steps against 295 with four, 324 with two),
+// spatial four (48^4: 337 us against 359 us with three, 357 us with two of 256, before 256-bit
+// loads), temporal eight (212 against 216 us with four of 256).
 template <typename R, int MODE>
 constexpr int ape_min_blocks()
 {
-    return MODE == SU2G_APE_ALL ? (sizeof(R) == 4 ? 4 : 3) : (sizeof(R) == 4 || MODE == SU2G_APE_TEMPORAL ? 8 : 4);
+    return MODE == SU2G_APE_ALL ? (sizeof(R) == 4 ? 5 : 3) : (sizeof(R) == 4 || MODE == SU2G_APE_TEMPORAL ? 8 : 4);
 }
 template <typename R, int MODE>
 constexpr int ape_block()
@@ -80,13 +79,13 @@ constexpr int ape_block()
     return 128;
 }
 
-// With PDL a step is a programmatic dependent launch (pdl_wait): the CTAs of the next step take the slots
-// that the tail of this one frees (ten steps, us, 24x14x18x22: FP64 all 166 -> 141, spatial 105 -> 84; FP32
-// 24^4 all 185 -> 162, spatial 116 -> 94; 48^4 within 2 %).  Its links are stored together at the end: with
-// plain loads, a store between them keeps the later ones behind it (FP32 all at 24^4 190 -> 169 us).  Only
-// FP32 APE_all at sizes whose two fields exceed L2 is faster without, its loads through the read-only
-// path (48^4 264 against 276 us a step; equal at 36^4).
-template <typename R, int MODE, bool PDL>
+// A step is a programmatic dependent launch (pdl_wait): the CTAs of the next step take the slots that the
+// tail of this one frees (ten steps, us, 24x14x18x22: FP64 all 166 -> 141, spatial 105 -> 84; FP32 24^4 all 185 -> 162,
+// spatial 116 -> 94; FP32 all at 40x30x36x34 658 -> 637, 48^4 within 2 %).  Its links are stored together at the
+// end: with plain loads, a store between them keeps the later ones behind it (FP32 all at 24^4 190 -> 169 us).
+// A step is bound by latency between the L1's and the issue slots' limits (FP32 spatial: 55-67 % and 68 %); tiles
+// of two, four or eight x planes a CTA, for more hits in L1, were 2 to 30 % slower.
+template <typename R, int MODE>
 __global__ void __launch_bounds__(ape_block<R, MODE>(), ape_min_blocks<R, MODE>()) k_ape(Field<R> in, Field<R> out,
                                                                                         Geom g, R alpha)
 {
@@ -95,23 +94,17 @@ __global__ void __launch_bounds__(ape_block<R, MODE>(), ape_min_blocks<R, MODE>(
     // 129.1 against 131.6 us, FP64 spatial 355 against 367 us with parity-alternating CTAs)
     Site s{};
     int par, h;
-    if (PDL) pdl_trigger();
+    pdl_trigger();
     const bool valid = site_warp_pair(g, blockIdx.x, threadIdx.x, blockDim.x, s, par, h);
-    if (PDL) pdl_wait(h, s.n);
+    pdl_wait(h, s.n);
     if (!valid) return;
-    if (PDL) {
-        Q<R> res[4];
-        ape_staples<R, MODE>(field_ca(in), g, s, par, h, [&](int mu, const Q<R>& u, const Q<R>& S) {
-            res[mu] = q_project(q_axpy(alpha, S, u));
-        });
+    Q<R> res[4];
+    ape_staples<R, MODE>(field_ca(in), g, s, par, h, [&](int mu, const Q<R>& u, const Q<R>& S) {
+        res[mu] = q_project(q_axpy(alpha, S, u));
+    });
 #pragma unroll
-        for (int mu = 0; mu < 4; ++mu)
-            if (ape_updates(MODE, mu)) out.sth(mu, par, h, res[mu]);
-    } else {
-        ape_staples<R, MODE>(in, g, s, par, h, [&](int mu, const Q<R>& u, const Q<R>& S) {
-            out.sth(mu, par, h, q_project(q_axpy(alpha, S, u)));
-        });
-    }
+    for (int mu = 0; mu < 4; ++mu)
+        if (ape_updates(MODE, mu)) out.sth(mu, par, h, res[mu]);
 }
 
 // ---------------------------------------------------------- Wilson loops ---
@@ -556,14 +549,7 @@ void launch_ape_t(su2g_lattice* h, const Field<R>& in, const Field<R>& out, R al
 {
     constexpr int block = ape_block<R, MODE>();
     const int grid = (int)((2 * (long long)h->g.Vh + block - 1) / block);   // warp pairs over the same h run
-    // FP32 APE_all on fields beyond L2: in order, through the read-only path (below)
-    if constexpr (MODE == SU2G_APE_ALL && sizeof(R) == 4) {
-        if (8ull * h->g.V * h->link_bytes > h->l2_bytes) {
-            k_ape<R, MODE, false><<<grid, block, 0, h->stream>>>(in, out, h->g, alpha);
-            return;
-        }
-    }
-    launch_pdl(k_ape<R, MODE, true>, grid, block, h->stream, in, out, h->g, alpha);
+    launch_pdl(k_ape<R, MODE>, grid, block, h->stream, in, out, h->g, alpha);
 }
 
 template <typename R>
