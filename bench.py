@@ -367,8 +367,8 @@ def time_steps(lat, K, fn):
 def batch_figures(dist, sweeps=1000, seq_sweeps=20):
     """Batched replicas: (a) 64 lattices 16 x 8^4, 16 x 10^4, 16 x 12^4, 16 x 16^4, beta ~ U[2.2, 3.2],
     distinct seeds, alternating hot/cold, `sweeps` sweeps of 1 HB + 4 OR with the plaquette of every
-    replica every sweep, one CUDA-graph replay per sweep; (b) the same for 64 x 12^4 against 64 single
-    handles swept one after another (no graph)."""
+    replica every sweep; (b) the same for 64 x 12^4 against 64 single
+    handles swept one after another."""
     import random
     from masterarbeit_b200.su2g import Batch, Lattice
 
@@ -419,7 +419,7 @@ def batch_figures(dist, sweeps=1000, seq_sweeps=20):
 def graph_figures(dist, sweeps=200):
     """The small-lattice chain of the reference's own test run (8^4, beta 3.09, cold start, seed 1,
     `sweeps` x (1 HB + N_OR OR) with the plaquette after every sweep), issued call by call against
-    one replayed CUDA graph per sweep (su2g_graph_run)."""
+    one su2g_graph_run call."""
     from masterarbeit_b200.su2g import Lattice
 
     out = {}
@@ -674,7 +674,7 @@ def run_ours(args, dist, dims):
         extras["batch"] = batch_figures(dist)
         extras["graph_loop"] = graph_figures(dist)
         # one configuration's measurement (the 48^4 flows of the thesis: 400 spatial APE steps then
-        # W(R<=9, T<=9); Q after 30 APE_all steps), one CUDA graph per configuration
+        # W(R<=9, T<=9); Q after 30 APE_all steps), one su2g_measure call per configuration
         L = Lattice(dims, precision="fp32", beta=BETA, seed=1000 + rank, start="haar", replica=rank, device=dist.local)
         L.sweep(2, 1, N_OR)
         R9 = [r for r in range(1, 10) for t in range(1, 10)]

@@ -147,14 +147,13 @@ int su2g_write_config(su2g_lattice *h, const char *path, double *plaq);
 int su2g_read_config_reflect(su2g_lattice *h, const char *path, double *plaq_file, double *plaq);
 
 /* ---- one configuration's measurement in the meas and qtop drivers
- * (LGT_Code/main_meas/meas.c:93-126, LGT_Code/main_qtop/qtop.c:76-91) as one replayed CUDA graph.
- * Both branches start from a device copy of the handle's field, which is left unchanged:
+ * (LGT_Code/main_meas/meas.c:93-126, LGT_Code/main_qtop/qtop.c:76-91) in one call: one sequence of
+ * launches and one copy of the results.  Both branches smear away from the handle's field, which is left unchanged:
  *  - charges: q[i] = Q after q_ape[i] APE_all steps of parameter alpha_q (cumulative counts,
  *    ascending; meas.c records one charge after smear_tc steps, qtop.c one per step count);
  *  - loops: w[i] = W(R[i], T[i]) after ns_t temporal steps (alpha_t) and then ns_s spatial steps
  *    (alpha_s), the tSmear / rSmear order of meas.c:106-109.
- * The graph is captured on the first call with a given spec and replayed by later calls with the
- * same spec (a new field read into the handle needs no new capture). */
+ * The first call allocates two field buffers, which later calls use again. */
 typedef struct su2g_meas_spec {
     int32_t n_q;            /* charges to record (0: none) */
     const int32_t *q_ape;   /* APE_all step count before each charge */
@@ -168,7 +167,7 @@ typedef struct su2g_meas_spec {
     double alpha_s;         /* measParams.smpars */
 } su2g_meas_spec;
 int su2g_measure(su2g_lattice *h, const su2g_meas_spec *spec, double *q, double *w);
-/* Free the measurement graph and its two field copies (also freed by su2g_destroy). */
+/* Free the measurement's two field buffers (also freed by su2g_destroy). */
 int su2g_measure_release(su2g_lattice *h);
 
 /* ---- the reference's analysis tools on the device.  Inputs may be host or device memory;
@@ -192,14 +191,13 @@ int su2g_stats_veff(const double *w, int32_t n_conf, int32_t n_r, int32_t n_t, i
                     double *veff_err, double *v, double *v_err);
 
 /* ---- the driver loop of LGT_Code/main/qcd.c:55-60 (gaugefieldUpdate, then plaquette) as one
- * replayed CUDA graph.  Runs n_blocks blocks of [meas_every x (n_hb heatbath + n_or overrelaxation
- * sweeps), plaquette].  The block is captured on first use and replayed; it is captured again
- * when the block shape, beta, the seed or the field's buffers have changed.  The results equal
+ * call: n_blocks blocks of [meas_every x (n_hb heatbath + n_or overrelaxation sweeps), plaquette],
+ * enqueued one after another, the host waiting once per group of blocks.  The results equal
  * those of the same su2g_sweep_plaquette sequence bit for bit.  plaq[b] and acc[b] (either
  * may be NULL) receive the plaquette after block b and block b's mean heatbath acceptance. */
 int su2g_graph_run(su2g_lattice *h, int32_t n_blocks, int32_t meas_every, int32_t n_hb, int32_t n_or,
                    double *plaq, double *acc);
-/* Free the captured block (it is also freed by su2g_destroy). */
+/* Kept for callers of earlier versions, whose loop held a captured block; there is nothing to free. */
 int su2g_graph_release(su2g_lattice *h);
 
 /* ---- observables */
@@ -250,13 +248,13 @@ int su2g_batch_destroy(su2g_batch *b);
 const char *su2g_batch_last_error(const su2g_batch *b);
 /* n_sweeps sweeps of (n_hb heatbath + n_or overrelaxation); every meas_every sweeps the plaquette
  * of every replica goes to plaq_trace[k * n + r] (k-th measurement; may be NULL; 0 = no
- * measurement).  The block of meas_every sweeps plus measurement is one CUDA graph, replayed.
- * ms (may be NULL) receives the device time of the replays. */
+ * measurement).  ms (may be NULL) receives the device time of the run. */
 int su2g_batch_run(su2g_batch *b, int32_t n_sweeps, int32_t n_hb, int32_t n_or, int32_t meas_every,
                    double *plaq_trace, double *ms);
 /* How a batch runs its sweeps.  SU2G_BATCH_GRAPH: one launch per checkerboard pass for all replicas
  * (CTAs mapped to replicas by the replica-offset table), a measurement block captured once in a CUDA
- * graph and replayed.  SU2G_BATCH_PERSISTENT: the whole su2g_batch_run as one cooperative launch
+ * graph and replayed (larger batches: launched directly, each pass starting in the tail of the one before).
+ * SU2G_BATCH_PERSISTENT: the whole su2g_batch_run as one cooperative launch
  * whose resident CTAs walk every pass as one global link index over all replicas (small replicas
  * share a CTA) and meet at a bounded grid-wide barrier between passes; a barrier that waits too
  * long makes the run return SU2G_EDEVICE.  Both draw the same Philox streams; the persistent

@@ -1,7 +1,7 @@
 // su2meas -- native measurement driver over libsu2g: the flows of the reference's meas and qtop
 // programs (LGT_Code/main_meas/meas.c:38-133, LGT_Code/main_qtop/qtop.c:17-99) with every
 // configuration read straight into device memory (su2g_read_config) and each configuration's
-// smearing + charge + Wilson-loop sequence replayed from one CUDA graph (su2g_measure).
+// smearing + charge + Wilson-loop sequence run by one call (su2g_measure).
 //
 //   su2meas -i meas.in -d TxXxYxZ [-p fp64|fp32] [--device N]
 //       reads the reference's meas input file (keys of readInputFileForMeas, inp_IO.c:250-360) and

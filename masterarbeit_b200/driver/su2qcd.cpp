@@ -1,6 +1,6 @@
 // su2qcd -- native thermalisation/production driver over libsu2g: the flow of the reference's qcd
-// program (LGT_Code/main/qcd.c:26-79) with the sweeps between two configuration writes replayed
-// from one CUDA graph (su2g_graph_run) and configurations written from device memory
+// program (LGT_Code/main/qcd.c:26-79) with the sweeps between two configuration writes run
+// by one call (su2g_graph_run) and configurations written from device memory
 // (su2g_write_config).
 //
 //   su2qcd -i qcd.in -d TxXxYxZ [-c cfg | -t cfg] [-p fp64|fp32] [--or N] [--utype 0|1] [--stype 0|1]
@@ -17,7 +17,7 @@
 // Differences: the extents are a command-line argument (the reference compiles them in); --or N adds
 // N overrelaxation sweeps after every heatbath sweep (the reference has none; default 0); the
 // random numbers are Philox keyed by `seed`, not RANLUX, so chains agree with the reference's
-// statistically; the update record's time is the mean over a graph block.
+// statistically; the update record's time is the mean over a call.
 #include <chrono>
 #include <cstdarg>
 #include <cstdio>

@@ -288,8 +288,8 @@ class Lattice:
         self._check(self.lib.su2g_update_pass(self.h, int(kind), int(mu), int(parity), int(sweep)))
 
     def graph_run(self, n_blocks, meas_every=1, n_hb=1, n_or=0):
-        """n_blocks x [meas_every x (n_hb HB + n_or OR sweeps), plaquette] from one replayed CUDA
-        graph; returns (plaquette trace, acceptance trace), one entry per block."""
+        """n_blocks x [meas_every x (n_hb HB + n_or OR sweeps), plaquette] in one call;
+        returns (plaquette trace, acceptance trace), one entry per block."""
         plaq = np.zeros(int(n_blocks))
         acc = np.zeros(int(n_blocks))
         self._check(self.lib.su2g_graph_run(self.h, int(n_blocks), int(meas_every), int(n_hb), int(n_or),
@@ -320,7 +320,7 @@ class Lattice:
         return a.value, b.value
 
     def measure(self, q_ape=(), alpha_q=0.0, R=(), T=(), ns_t=0, alpha_t=0.0, ns_s=0, alpha_s=0.0):
-        """One measurement of the meas / qtop drivers on a copy of the field (one CUDA graph):
+        """One measurement of the meas / qtop drivers in one call, away from the field:
         Q after each cumulative APE_all step count in q_ape, and W(R[i], T[i]) after ns_t temporal
         and ns_s spatial steps.  Returns (q array, w array); the field is left unchanged."""
         qa = (ctypes.c_int32 * max(1, len(q_ape)))(*[int(x) for x in q_ape])
@@ -521,7 +521,7 @@ class Batch:
     MODES = {"graph": 0, "persistent": 1}
 
     def configure(self, mode="graph", block=256):
-        """Run the sweeps as a replayed graph of per-pass launches or as one persistent launch."""
+        """Run the sweeps as per-pass launches (a replayed graph for small batches) or as one persistent launch."""
         self._check(self.lib.su2g_batch_configure(self.h, self.MODES[mode], int(block)))
 
     def selftest_grid_barrier(self, missing=1, wait_cycles=100_000_000):
