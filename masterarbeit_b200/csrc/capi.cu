@@ -476,6 +476,7 @@ extern "C" int su2g_destroy(su2g_lattice* h)
     if (h->ev_begin) cudaEventDestroy(h->ev_begin);
     if (h->ev_end) cudaEventDestroy(h->ev_end);
     if (h->pool) cudaMemPoolDestroy(h->pool);
+    release_meas_graph(h);
     cudaFree(h->lines);
     cudaFree(h->meas_work);
     cudaFree(h->meas_alt);

@@ -138,6 +138,7 @@ struct su2g_lattice {
     void* lines = nullptr;             // 2- and 3-link line products of the field Q is measured on
     void* meas_work = nullptr;         // the measurement's smeared field and its ping-pong partner
     void* meas_alt = nullptr;
+    struct su2g_meas_graph* meas = nullptr;   // the last measurement, or null
     bool profiling = false;
     struct Prof {
         cudaEvent_t a, b;
@@ -203,6 +204,7 @@ int fetch_results(su2g_lattice* h, int off, int n);
 
 namespace su2g {
 // Enqueue `ns` smearing steps on the handle's stream (no synchronisation).
+void release_meas_graph(su2g_lattice* h);
 int ape_enqueue(su2g_lattice* h, int ns, double alpha, int mode);
 // One smearing step from the field at in_dirs into out_dirs (only the smeared directions are written).
 int ape_step(su2g_lattice* h, void* const in_dirs[4], void* const out_dirs[4], int mode, double alpha);
