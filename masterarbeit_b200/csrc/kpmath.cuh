@@ -12,7 +12,7 @@
 //  - cosines and sines: the angle is reduced exactly in integers, then near-minimax polynomials (Chebyshev
 //    fits computed from sin and cos in 60 digits) of relative error below 2^-57.
 // Against 80-bit arithmetic over 8 x 10^7 words, largest error in ulp of the value: log 1.2, cos^2 5.3, sine and
-// cosine 1.5.  On B200, with beta entering as its reciprocal and sqrt(x) as x rsqrt(x): FP64 heatbath pass at
+// cosine 1.5.  On B200, with beta entering as its reciprocal: FP64 heatbath pass at
 // 24^4 16.4 -> 14.6 us, at 24x14x18x22 9.0 -> 8.5 us, at 48^4 164 -> 156 us.
 #pragma once
 #include <cstdint>

@@ -38,15 +38,15 @@ __device__ __forceinline__ float kp_cos2pi_sq(uint32_t w, float)
     return c * c;
 }
 __device__ __forceinline__ double kp_cos2pi_sq(uint32_t w, double) { return kp_cos2pi_sq_word(w); }
-// Square root of x > 0: FP32 uses the hardware approximation (sqrt.approx.f32, relative error
-// ~2^-23), FP64 the reciprocal square root.
+// Square root of x >= 0 (delta is 0 at an infinite beta): FP32 uses the hardware approximation (sqrt.approx.f32,
+// relative error ~2^-23), FP64 the correctly rounded one.
 __device__ __forceinline__ float kp_sqrt(float x)
 {
     float r;
     asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
-__device__ __forceinline__ double kp_sqrt(double x) { return x * rsqrt(x); }
+__device__ __forceinline__ double kp_sqrt(double x) { return sqrt(x); }
 // What the sampler takes for beta: FP32 beta itself, FP64 its reciprocal (a division a link less).
 template <typename R>
 __host__ __device__ __forceinline__ R kp_beta(double beta)
