@@ -31,7 +31,8 @@ namespace {
 
 struct Replica {
     Geom g;
-    double beta, kb;   // kb: kp_beta of the batch's precision
+    double beta;
+    KpBeta<double> kb;   // of beta
     uint64_t seed;
     uint32_t id;
     int start;
@@ -91,6 +92,9 @@ int bcuda(su2g_batch* b, cudaError_t e, const char* what)
     if (e == cudaSuccess) return SU2G_OK;
     return berr(b, e == cudaErrorMemoryAllocation ? SU2G_ENOMEM : SU2G_ECUDA, "%s: %s", what, cudaGetErrorString(e));
 }
+
+__device__ __forceinline__ KpBeta<float> rep_beta(const Replica& r, float) { return {(float)r.beta}; }
+__device__ __forceinline__ KpBeta<double> rep_beta(const Replica& r, double) { return r.kb; }
 
 template <typename R>
 __device__ __forceinline__ Field<R> rep_field(const Replica& r)
@@ -184,7 +188,7 @@ __global__ void __launch_bounds__(256, 4) k_batch_update(BatchGrid a, int par, u
     if (KIND == SU2G_HEATBATH) {
         Q<R> out;
         uint32_t trials = 0;
-        if (heatbath_link<R, EARLY>(A, (R)rp.kb, rp.seed, (uint32_t)s.n, sweep, (uint32_t)MU, rp.id, trials, out, status, 0u,
+        if (heatbath_link<R, EARLY>(A, rep_beta(rp, R(0)), rp.seed, (uint32_t)s.n, sweep, (uint32_t)MU, rp.id, trials, out, status, 0u,
                                     early, angles))
             U.sth(MU, par, h, hb_store(out));
     } else {
@@ -409,7 +413,7 @@ __device__ __forceinline__ void persist_pass(const PersistArgs& a, const int* __
         if (KIND == SU2G_HEATBATH) {
             Q<R> out;
             uint32_t trials = 0;
-            if (heatbath_link<R>(A, (R)rp.kb, rp.seed, (uint32_t)s.n, sweep, (uint32_t)MU, rp.id, trials, out,
+            if (heatbath_link<R>(A, rep_beta(rp, R(0)), rp.seed, (uint32_t)s.n, sweep, (uint32_t)MU, rp.id, trials, out,
                                  a.status))
                 U.sth(MU, par, h, hb_store(out));
         } else {
@@ -773,7 +777,7 @@ extern "C" int su2g_batch_create(const su2g_replica* reps, int32_t n, int32_t pr
         Replica rp;
         rp.g = make_geom(reps[r].dims);
         rp.beta = reps[r].beta;
-        rp.kb = precision == SU2G_FP32 ? rp.beta : kp_beta<double>(rp.beta);
+        rp.kb = kp_beta<double>(rp.beta);
         rp.seed = reps[r].seed;
         rp.id = reps[r].replica;
         rp.start = reps[r].start;

@@ -68,7 +68,7 @@ __device__ __forceinline__ double warp_acceptance(uint32_t trials)
 }
 
 template <int MU, int KIND, bool PLQ>
-__device__ __forceinline__ void chain_pass(const ChainLink& l, int par, double kb, const PhiloxKeys& keys, uint32_t sweep,
+__device__ __forceinline__ void chain_pass(const ChainLink& l, int par, const KpBeta<double>& kb, const PhiloxKeys& keys, uint32_t sweep,
                                            uint32_t replica, unsigned* status, double* acc, DD* plaq)
 {
     Site s = l.s[0];
@@ -108,7 +108,7 @@ __device__ __forceinline__ void chain_pass(const ChainLink& l, int par, double k
 // One sub-sweep; `last`: its passes (1, 1), (2, 1), (3, 1) also leave their plaquette partials, at plaq and
 // `warps` entries on each.
 template <int KIND>
-__device__ __forceinline__ void chain_sweep(const ChainLink& l, double kb, const PhiloxKeys& keys, uint32_t sweep,
+__device__ __forceinline__ void chain_sweep(const ChainLink& l, const KpBeta<double>& kb, const PhiloxKeys& keys, uint32_t sweep,
                                             uint32_t replica, unsigned* status, double* acc, bool last, DD* plaq, int warps)
 {
 #pragma unroll 1
@@ -125,7 +125,7 @@ __device__ __forceinline__ void chain_sweep(const ChainLink& l, double kb, const
     if (last) chain_pass<3, KIND, true>(l, 1, kb, keys, sweep, replica, status, acc, plaq ? plaq + 2 * warps : nullptr);
 }
 
-__global__ void __launch_bounds__(kChainThreads, 1) k_chain(Field<double> U0, Geom g, double kb, PhiloxKeys keys,
+__global__ void __launch_bounds__(kChainThreads, 1) k_chain(Field<double> U0, Geom g, KpBeta<double> kb, PhiloxKeys keys,
                                                             uint32_t sweep, uint32_t replica, ChainArgs a,
                                                             unsigned* __restrict__ status)
 {

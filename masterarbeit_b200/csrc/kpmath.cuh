@@ -1,5 +1,5 @@
-// kpmath.cuh -- the FP64 logarithm, squared cosine and sine/cosine pair of the Kennedy-Pendleton sampler, for
-// the uniforms u = (w + 1/2) / 2^32 of a 32-bit random word.
+// kpmath.cuh -- the Kennedy-Pendleton sampler's division by beta, and the FP64 logarithm, squared cosine and
+// sine/cosine pair of its uniforms u = (w + 1/2) / 2^32 of a 32-bit random word.
 //
 // The general library functions spend most of their instructions on arguments that cannot occur here
 // (negative, zero, denormal, infinite, any size) and fetch each coefficient with two moves.  These use what
@@ -12,12 +12,43 @@
 //  - cosines and sines: the angle is reduced exactly in integers, then near-minimax polynomials (Chebyshev
 //    fits computed from sin and cos in 60 digits) of relative error below 2^-57.
 // Against 80-bit arithmetic over 8 x 10^7 words, largest error in ulp of the value: log 1.2, cos^2 5.3, sine and
-// cosine 1.5.  On B200, with beta entering as its reciprocal: FP64 heatbath pass at
+// cosine 1.5.  On B200, with beta entering as its reciprocal (KpBeta): FP64 heatbath pass at
 // 24^4 16.4 -> 14.6 us, at 24x14x18x22 9.0 -> 8.5 us, at 48^4 164 -> 156 us.
 #pragma once
+#include <cmath>
 #include <cstdint>
 
 namespace su2g {
+
+// What the sampler takes for beta: FP32 beta itself, FP64 its reciprocal as hi + lo, so that a product with
+// it is as accurate as the division it stands for (two multiply-adds a link instead).  lo is 0 where the
+// reciprocal is 0 or infinite.
+template <typename R>
+struct KpBeta;
+template <>
+struct KpBeta<float> {
+    float beta;
+};
+template <>
+struct KpBeta<double> {
+    double hi, lo;
+};
+template <typename R>
+inline KpBeta<R> kp_beta(double beta);
+template <>
+inline KpBeta<float> kp_beta<float>(double beta)
+{
+    return {(float)beta};
+}
+template <>
+inline KpBeta<double> kp_beta<double>(double beta)
+{
+    const double hi = 1.0 / beta;
+    return {hi, std::isfinite(beta) && std::isfinite(hi) ? std::fma(-beta, hi, 1.0) / beta : 0.0};
+}
+// x / beta
+__device__ __forceinline__ float kp_over_beta(float x, const KpBeta<float>& b) { return __fdividef(x, b.beta); }
+__device__ __forceinline__ double kp_over_beta(double x, const KpBeta<double>& b) { return fma(x, b.hi, x * b.lo); }
 
 // (2^52 + w) as a double: a 32-bit word enters FP64 arithmetic without a conversion instruction
 __device__ __forceinline__ double kp_magic(uint32_t w) { return __hiloint2double(0x43300000, (int)w); }

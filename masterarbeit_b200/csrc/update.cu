@@ -83,7 +83,7 @@ int update_shape(const su2g_lattice* h, int grid)
 // again (20 FP64 sweeps at 10x12x14x12: 0.81, 0.72, 0.59 ms with one, two, three; 0.82 with none).
 template <typename R, int MU, int KIND, bool PLQ, int CTAS, int EARLY>
 __global__ void __launch_bounds__(kUpdateBlock, CTAS)
-    k_update(Field<R> Unc, Geom g, int par, R kb, PhiloxKeys seed, uint32_t sweep, uint32_t replica,
+    k_update(Field<R> Unc, Geom g, int par, KpBeta<R> kb, PhiloxKeys seed, uint32_t sweep, uint32_t replica,
              DD* acc_part, int acc_first, unsigned* __restrict__ status, DD* __restrict__ plaq_part)
 {
     // one link per thread; CTAs are dispatched in index order, so the CTAs in flight cover a
@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(kUpdateBlock, CTAS)
 //    count for the site's four links), heatbath or Metropolis once per visit.
 // The acceptance sum counts 1/trials per heatbath visit and accepted/hits per Metropolis visit.
 struct VisitArgs {
-    double beta, kb, eps;   // kb: kp_beta of the handle's precision
+    double beta, eps;
     int hits;
     double p0;   // (1 - 1/V)^V
     uint64_t seed;
@@ -161,7 +161,7 @@ struct VisitArgs {
 
 // Two resident CTAs per SM: the visit loop and the Metropolis state spill at 64 registers.
 template <typename R, int MU, int KIND, int ORDER>
-__global__ void __launch_bounds__(kBlock, 2) k_visit(Field<R> U, Geom g, int par, VisitArgs a,
+__global__ void __launch_bounds__(kBlock, 2) k_visit(Field<R> U, Geom g, int par, VisitArgs a, KpBeta<R> kb,
                                                   double* __restrict__ acc_sum, unsigned* __restrict__ status)
 {
     double acc_thread = 0.0;
@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_visit(Field<R> U, Geom g, int par
                 bool changed = false;
                 for (int v = 0; v < visits; ++v) {
                     uint32_t trials = 0;
-                    if (heatbath_link<R>(A, (R)a.kb, a.seed, (uint32_t)s.n, a.sweep, (uint32_t)MU, a.replica, trials,
+                    if (heatbath_link<R>(A, kb, a.seed, (uint32_t)s.n, a.sweep, (uint32_t)MU, a.replica, trials,
                                          out, status, (uint32_t)v << kVisitShift)) {
                         cur = out;
                         changed = true;
@@ -207,11 +207,12 @@ template <typename R, int KIND, int ORDER>
 void launch_visit_t(su2g_lattice* h, int mu, int par, const VisitArgs& a, double* acc_sum, int grid)
 {
     Field<R> U = make_field<R>(h->dirp, h->g.Vh);
+    const KpBeta<R> kb = kp_beta<R>(h->beta);
     switch (mu) {
-        case 0: k_visit<R, 0, KIND, ORDER><<<grid, kBlock, 0, h->stream>>>(U, h->g, par, a, acc_sum, h->d_status); break;
-        case 1: k_visit<R, 1, KIND, ORDER><<<grid, kBlock, 0, h->stream>>>(U, h->g, par, a, acc_sum, h->d_status); break;
-        case 2: k_visit<R, 2, KIND, ORDER><<<grid, kBlock, 0, h->stream>>>(U, h->g, par, a, acc_sum, h->d_status); break;
-        default: k_visit<R, 3, KIND, ORDER><<<grid, kBlock, 0, h->stream>>>(U, h->g, par, a, acc_sum, h->d_status); break;
+        case 0: k_visit<R, 0, KIND, ORDER><<<grid, kBlock, 0, h->stream>>>(U, h->g, par, a, kb, acc_sum, h->d_status); break;
+        case 1: k_visit<R, 1, KIND, ORDER><<<grid, kBlock, 0, h->stream>>>(U, h->g, par, a, kb, acc_sum, h->d_status); break;
+        case 2: k_visit<R, 2, KIND, ORDER><<<grid, kBlock, 0, h->stream>>>(U, h->g, par, a, kb, acc_sum, h->d_status); break;
+        default: k_visit<R, 3, KIND, ORDER><<<grid, kBlock, 0, h->stream>>>(U, h->g, par, a, kb, acc_sum, h->d_status); break;
     }
 }
 
@@ -308,7 +309,7 @@ namespace {
 // the FP32 histogram exercises the FP32 sampler's fast logarithm, sine/cosine, approximate square
 // roots and delta clamp.  Draw i uses the Philox stream of site i (sweep i >> 32, direction 0).
 template <typename R>
-__global__ void __launch_bounds__(kBlock) k_kp_histogram(double kb, uint64_t seed, long long n, int nbins,
+__global__ void __launch_bounds__(kBlock) k_kp_histogram(KpBeta<R> kb, uint64_t seed, long long n, int nbins,
                                                          unsigned long long* __restrict__ counts,
                                                          unsigned* __restrict__ status)
 {
@@ -319,7 +320,7 @@ __global__ void __launch_bounds__(kBlock) k_kp_histogram(double kb, uint64_t see
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         Q<R> X;
         uint32_t trials = 0;
-        if (!heatbath_link<R>(A, (R)kb, seed, (uint32_t)i, (uint32_t)(i >> 32), 0u, 0u, trials, X, status))
+        if (!heatbath_link<R>(A, kb, seed, (uint32_t)i, (uint32_t)(i >> 32), 0u, 0u, trials, X, status))
             continue;   // trial bound hit: the status word tells the host
         int b = (int)(((double)X.c0 + 1.0) * 0.5 * nbins);   // bin of x0 on [-1, 1]
         b = b < 0 ? 0 : (b >= nbins ? nbins - 1 : b);
@@ -441,7 +442,6 @@ extern "C" int su2g_gauge_update(su2g_lattice* h, int32_t nup, int32_t utype, in
     }
     VisitArgs a;
     a.beta = h->beta;
-    a.kb = h->prec == SU2G_FP32 ? h->beta : kp_beta<double>(h->beta);
     a.eps = eps;
     a.hits = utype == 0 ? hits : 1;
     a.p0 = std::exp((double)h->g.V * std::log1p(-1.0 / (double)h->g.V));

@@ -47,27 +47,21 @@ __device__ __forceinline__ float kp_sqrt(float x)
     return r;
 }
 __device__ __forceinline__ double kp_sqrt(double x) { return sqrt(x); }
-// What the sampler takes for beta: FP32 beta itself, FP64 its reciprocal (a division a link less).
-template <typename R>
-__host__ __device__ __forceinline__ R kp_beta(double beta)
-{
-    return sizeof(R) == 8 ? R(1.0 / beta) : R(beta);
-}
 // 1/|A| and 1/(beta |A|) from |A|^2, from one reciprocal square root (FP32: the hardware
 // approximation; FP64: rsqrt, within an ulp, in place of a square root and two divisions: the FP64
 // heatbath pass 152.9 -> 152.1 us at 48^4).  |A| = 0 gives k = NaN (0 * inf), which fails the
 // k > eps test like k = 0 does.
-__device__ __forceinline__ void kp_norms(float n2, float beta, float& k, float& ik, float& ia)
+__device__ __forceinline__ void kp_norms(float n2, const KpBeta<float>& b, float& k, float& ik, float& ia)
 {
     ik = rsqrtf(n2);
     k = n2 * ik;
-    ia = __fdividef(ik, beta);
+    ia = kp_over_beta(ik, b);
 }
-__device__ __forceinline__ void kp_norms(double n2, double ibeta, double& k, double& ik, double& ia)
+__device__ __forceinline__ void kp_norms(double n2, const KpBeta<double>& b, double& k, double& ik, double& ia)
 {
     ik = rsqrt(n2);
     k = n2 * ik;
-    ia = ik * ibeta;
+    ia = kp_over_beta(ik, b);
 }
 // The FP32 logs of uniforms just below 1 may come out positive by their absolute error (~2^-21);
 // delta is clamped at 0 so that sqrt(delta (2 - delta)) stays real.  FP64 logs are exact in sign.
@@ -176,7 +170,7 @@ __device__ __forceinline__ KpAngles<R> kp_angles(const Seed& seed, uint32_t site
 // kb is kp_beta<R>(beta).  With EARLY > 0 that many first trials and the angles were drawn by the caller
 // (draw_base 0), which needs no staple for them.
 template <typename R, int EARLY = 0, typename Seed>
-__device__ __forceinline__ bool heatbath_link(const Q<R>& A, R kb, const Seed& seed, uint32_t site, uint32_t sweep,
+__device__ __forceinline__ bool heatbath_link(const Q<R>& A, const KpBeta<R>& kb, const Seed& seed, uint32_t site, uint32_t sweep,
                                               uint32_t mu, uint32_t replica, uint32_t& trials, Q<R>& out,
                                               unsigned* status, uint32_t draw_base = 0u,
                                               const KpTrial<R>* early = nullptr, const KpAngles<R>& angles = {})
