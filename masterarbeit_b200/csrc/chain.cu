@@ -78,6 +78,7 @@ __device__ __forceinline__ void chain_pass(const ChainLink& l, int par, const Kp
     if (KIND == SU2G_HEATBATH) {
         early[0] = kp_trial<double>(keys, (uint32_t)s.n, sweep, (uint32_t)MU, replica, 0u);
         angles = kp_angles<double>(keys, (uint32_t)s.n, sweep, (uint32_t)MU, replica, 0u);
+        kp_pin(early, angles);
     }
     cluster_wait();
     uint32_t trials = 0;

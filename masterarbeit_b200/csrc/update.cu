@@ -102,6 +102,7 @@ __global__ void __launch_bounds__(kUpdateBlock, CTAS)
         for (int i = 0; i < EARLY; ++i)
             early[i] = kp_trial<R>(seed, (uint32_t)s.n, sweep, (uint32_t)MU, replica, (uint32_t)i);
         angles = kp_angles<R>(seed, (uint32_t)s.n, sweep, (uint32_t)MU, replica, 0u);
+        kp_pin(early, angles);
     }
     pdl_wait(h, s.n);
     if (KIND == SU2G_HEATBATH && acc_part && !acc_first) acc_warp = acc_part[warp].s;   // of the passes before

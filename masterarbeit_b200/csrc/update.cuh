@@ -167,6 +167,23 @@ __device__ __forceinline__ KpAngles<R> kp_angles(const Seed& seed, uint32_t site
     return a;
 }
 
+// Keeps what was drawn early ahead of the wait.
+__device__ __forceinline__ void kp_pin(float& x) { asm volatile("" : "+f"(x)); }
+__device__ __forceinline__ void kp_pin(double& x) { asm volatile("" : "+d"(x)); }
+template <typename R, int N>
+__device__ __forceinline__ void kp_pin(KpTrial<R> (&t)[N], KpAngles<R>& a)
+{
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        kp_pin(t[i].lc);
+        kp_pin(t[i].u3);
+    }
+    kp_pin(a.sth);
+    kp_pin(a.cth);
+    kp_pin(a.sph);
+    kp_pin(a.cph);
+}
+
 // kb is kp_beta<R>(beta).  With EARLY > 0 that many first trials and the angles were drawn by the caller
 // (draw_base 0), which needs no staple for them.
 template <typename R, int EARLY = 0, typename Seed>
