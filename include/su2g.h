@@ -258,9 +258,9 @@ int su2g_batch_run(su2g_batch *b, int32_t n_sweeps, int32_t n_hb, int32_t n_or, 
  * SU2G_BATCH_PERSISTENT: the whole su2g_batch_run as one cooperative launch
  * whose resident CTAs walk every pass as one global link index over all replicas (small replicas
  * share a CTA) and meet at a bounded grid-wide barrier between passes; a barrier that waits too
- * long makes the run return SU2G_EDEVICE.  Both draw the same Philox streams; the persistent
- * kernel's multiply-adds may round differently in the last bit, so its fields agree with the
- * graph form's to rounding, not bit for bit. */
+ * long makes the run return SU2G_EDEVICE.  Both draw the same Philox streams; FP64 fields are the same to the
+ * bit, while the persistent kernel's FP32 multiply-adds may round differently in the last bit, so that its FP32 fields
+ * agree with the graph form's to rounding. */
 enum su2g_batch_mode { SU2G_BATCH_GRAPH = 0, SU2G_BATCH_PERSISTENT = 1 };
 /* Choose the form and the CTA width (64, 128 or 256 threads; 128 or 256 for the persistent form). */
 int su2g_batch_configure(su2g_batch *b, int32_t mode, int32_t block);
@@ -318,7 +318,8 @@ int su2g_synchronize(su2g_lattice *h);
 int su2g_timer_begin(su2g_lattice *h);
 int su2g_timer_end(su2g_lattice *h, double *ms);
 /* When enabled, every kernel launch is bracketed by events; su2g_profile_read returns, for a
- * kernel class, the launch count and summed device time since the last reset. */
+ * kernel class, the launch count and summed device time since the last reset.  The fields and results are the
+ * same either way; FP64 sweeps of up to 4096 sites, otherwise one launch, run as passes while it is enabled. */
 enum su2g_kernel_class {
     SU2G_K_HEATBATH = 0, SU2G_K_OVERRELAX = 1, SU2G_K_PLAQUETTE = 2, SU2G_K_APE = 3,
     SU2G_K_WILSON = 4, SU2G_K_QTOP = 5, SU2G_K_REDUCE = 6, SU2G_K_OTHER = 7, SU2G_K_METROPOLIS = 8,

@@ -7,9 +7,9 @@
 // and its hardware barrier separates them.
 //
 // The links, draws and order of operations are k_update's, and so is the assignment of links to warps, whose
-// plaquette and acceptance sums go to the same entries; compiled as a separate kernel, its multiply-adds
-// may round differently in the last bit (as the batch's do).  FP32 fields are the same to the bit in a
-// batch and in a handle, so FP32 keeps to the passes.
+// plaquette and acceptance sums go to the same entries: the fields are the same to the bit (update.cuh spells the
+// multiply-adds out in FP64).  FP32 leaves them to the compiler, which starts a refused link's sums elsewhere here than in
+// the passes; FP32 fields being the same in a batch and in a handle, FP32 keeps to the passes.
 //
 // Measured, FP64, call by call (passes -> here): 20 heatbath sweeps 525 -> 430 us (8^4), 509 -> 369 us (4^4);
 // the loop of 10 sweeps, plaquette and acceptance 360 -> 252 us (8^4).  The line lies at one link per thread

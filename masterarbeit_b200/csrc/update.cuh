@@ -63,10 +63,12 @@ __device__ __forceinline__ void kp_norms(double n2, const KpBeta<double>& b, dou
     k = n2 * ik;
     ia = kp_over_beta(ik, b);
 }
-// The FP32 logs of uniforms just below 1 may come out positive by their absolute error (~2^-21);
-// delta is clamped at 0 so that sqrt(delta (2 - delta)) stays real.  FP64 logs are exact in sign.
-__device__ __forceinline__ float kp_clamp(float d) { return fmaxf(d, 0.0f); }
-__device__ __forceinline__ double kp_clamp(double d) { return d; }
+// delta = -lc / alpha.  The FP32 logs of uniforms just below 1 may come out positive by their absolute error
+// (~2^-21); delta is clamped at 0 so that sqrt(delta (2 - delta)) stays real.  FP64 logs are exact in sign; the product is
+// rounded by itself, since the compiler would fuse it into 1 - delta in some of the kernels and not in others, and one
+// chain would differ in the last bit from kernel to kernel.
+__device__ __forceinline__ float kp_delta(float lc, float ia) { return fmaxf(-lc * ia, 0.0f); }
+__device__ __forceinline__ double kp_delta(double lc, double ia) { return __dmul_rn(-lc, ia); }
 
 // Staple sum A with U_mu(x) A = sum of the six plaquettes containing U_mu(x)  (metro.c:34-63):
 //   A = sum_{nu != mu} U_nu(x+mu) U_mu(x+nu)^dag U_nu(x)^dag + U_nu(x-nu+mu)^dag U_mu(x-nu)^dag U_nu(x-nu)
@@ -184,6 +186,23 @@ __device__ __forceinline__ void kp_pin(KpTrial<R> (&t)[N], KpAngles<R>& a)
     kp_pin(a.cph);
 }
 
+// X (s A)^dag and |A|^2.  FP64 spells the multiply-adds out, for the reason given at kp_delta: which product of a sum
+// the compiler starts from depends on the code around it.
+__device__ __forceinline__ Q<float> kp_link(const Q<float>& X, const Q<float>& A, float s) { return q_mul_nd(X, q_scale(A, s)); }
+__device__ __forceinline__ Q<double> kp_link(const Q<double>& X, const Q<double>& A, double s)
+{
+    const Q<double> b = q_scale(A, s);
+    return q_make<double>(fma(X.c3, b.c3, fma(X.c2, b.c2, fma(X.c1, b.c1, X.c0 * b.c0))),
+                          fma(-X.c3, b.c2, fma(X.c2, b.c3, fma(-X.c0, b.c1, X.c1 * b.c0))),
+                          fma(X.c3, b.c1, fma(-X.c1, b.c3, fma(-X.c0, b.c2, X.c2 * b.c0))),
+                          fma(-X.c2, b.c1, fma(X.c1, b.c2, fma(-X.c0, b.c3, X.c3 * b.c0))));
+}
+__device__ __forceinline__ float kp_norm2(const Q<float>& A) { return q_norm2(A); }
+__device__ __forceinline__ double kp_norm2(const Q<double>& A)
+{
+    return fma(A.c3, A.c3, fma(A.c2, A.c2, fma(A.c1, A.c1, A.c0 * A.c0)));
+}
+
 // kb is kp_beta<R>(beta).  With EARLY > 0 that many first trials and the angles were drawn by the caller
 // (draw_base 0), which needs no staple for them.
 template <typename R, int EARLY = 0, typename Seed>
@@ -193,7 +212,7 @@ __device__ __forceinline__ bool heatbath_link(const Q<R>& A, const KpBeta<R>& kb
                                               const KpTrial<R>* early = nullptr, const KpAngles<R>& angles = {})
 {
     R k, ik, ia;   // |A|, 1/|A|, 1/alpha with alpha = |A| beta (heatbath.c:142)
-    kp_norms(q_norm2(A), kb, k, ik, ia);
+    kp_norms(kp_norm2(A), kb, k, ik, ia);
     if (!(k > eps_r<R>())) {
         U4 w = link_random(seed, site, sweep, mu, draw_base | 1u, 1u, kStreamUpdate, replica);
         trials = 0;
@@ -207,14 +226,14 @@ __device__ __forceinline__ bool heatbath_link(const Q<R>& A, const KpBeta<R>& kb
     for (int i = 0; i < EARLY; ++i)
         if (!taken) {
             ++trial;
-            delta = kp_clamp(-early[i].lc * ia);
+            delta = kp_delta(early[i].lc, ia);
             taken = early[i].u3 * early[i].u3 <= R(1) - R(0.5) * delta;
         }
     if (EARLY == 0 || !taken) {
         for (;;) {
             const KpTrial<R> t = kp_trial<R>(seed, site, sweep, mu, replica, draw_base | trial);
             ++trial;
-            delta = kp_clamp(-t.lc * ia);
+            delta = kp_delta(t.lc, ia);
             if (t.u3 * t.u3 <= R(1) - R(0.5) * delta) break;   // heatbath.c:94
             if (trial >= kMaxTrials) {   // the link keeps its value and the host sees the status bit
                 atomicOr(status, kStatusKpTrials);
@@ -229,7 +248,7 @@ __device__ __forceinline__ bool heatbath_link(const Q<R>& A, const KpBeta<R>& kb
     const R len = kp_sqrt(delta * (R(2) - delta));          // sqrt(1 - (1-delta)^2)
     Q<R> X = q_make<R>(R(1) - delta, len * a.sth * a.cph, len * a.sth * a.sph, len * a.cth);
     // U = X V^dag, V = A/k  (heatbath.c:140-146)
-    out = q_mul_nd(X, q_scale(A, ik));
+    out = kp_link(X, A, ik);
     return true;
 }
 
