@@ -348,8 +348,9 @@ int su2g::sweep_enqueue(su2g_lattice* h, int n_sweeps, int n_hb, int n_or, uint3
     const int parts = sweep_warps(h);   // per fused pass
     DD *plaq_part = with_plaq ? part0 : nullptr, *acc_part = with_acc ? part0 + 3 * parts : nullptr;
     const int subs = n_sweeps * (n_hb + n_or);
-    if (h->chain && !h->profiling && n_hb + n_or > 0) {   // (profiling times every pass)
-        const int most = std::max(1, kChainSubSweeps / (n_hb + n_or));
+    // (profiling times every pass; a sweep of more sub-sweeps than a launch may run goes pass by pass)
+    if (h->chain && !h->profiling && n_hb + n_or > 0 && n_hb + n_or <= kChainSubSweeps) {
+        const int most = kChainSubSweeps / (n_hb + n_or);
         for (int s = 0; s < n_sweeps; s += most) {
             const int n = std::min(most, n_sweeps - s);
             const bool plaq = plaq_part && s + n == n_sweeps;

@@ -56,3 +56,17 @@ def test_heatbath_with_and_without_the_plaquette(dims):
     a = _handle(dims, "fp64", lambda L: L.sweep(2, 1, 0))
     assert np.array_equal(a, _handle(dims, "fp64", lambda L: L.sweep_plaquette(2, 1, 0)))
     assert np.array_equal(a, _handle(dims, "fp64", lambda L: [L.sweep_plaquette(1, 1, 0) for _ in range(2)]))
+
+
+@pytest.mark.parametrize("n_hb,n_or", [(1024, 0), (24, 1000), (1024, 1), (25, 1000)])
+def test_long_sweeps(n_hb, n_or):
+    """A sweep of as many sub-sweeps as one cluster launch may run, and one more, which goes pass by pass."""
+    def run(L):
+        run.out = L.sweep_plaquette(1, n_hb, n_or, acc=True)
+
+    a = _handle((4, 2, 4, 4), "fp64", run)
+    pa = run.out
+    b = _handle((4, 2, 4, 4), "fp64", run, profile=True)
+    assert np.array_equal(a, b)
+    # the same terms in the same order: at most the last bit of a warp's sum
+    assert abs(pa[0] - run.out[0]) <= 1e-14 and abs(pa[1] - run.out[1]) <= 1e-14
