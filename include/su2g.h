@@ -153,8 +153,8 @@ int su2g_read_config_reflect(su2g_lattice *h, const char *path, double *plaq_fil
  *    ascending; meas.c records one charge after smear_tc steps, qtop.c one per step count);
  *  - loops: w[i] = W(R[i], T[i]) after ns_t temporal steps (alpha_t) and then ns_s spatial steps
  *    (alpha_s), the tSmear / rSmear order of meas.c:106-109.
- * The first call allocates two field buffers, which later calls use again; a small field's launches are captured
- * as a CUDA graph when the same measurement is asked for again. */
+ * The first call allocates two field buffers, which later calls use again; a small field's launches are replayed
+ * from a CUDA graph once the same measurement has been asked for a dozen times in a row. */
 typedef struct su2g_meas_spec {
     int32_t n_q;            /* charges to record (0: none) */
     const int32_t *q_ape;   /* APE_all step count before each charge */

@@ -9,11 +9,12 @@
 // Everything is enqueued at once and the results come back with one copy.
 //
 // A step of a small field is shorter than its launch takes on the host.  Fields up to kMeasGraphBytes are
-// therefore captured as a graph when a handle asks for the same measurement again (the first call runs as it is:
-// a program that measures once pays for no capture), and later calls replay it; the smearing steps stay programmatic
-// launches in it.  Q after 24 steps, 35 loops after 50 steps, direct -> replayed, us: FP32 8^4 257 -> 236, 20x14x16x16
-// 449 -> 409, 24^4 1056 -> 1027; FP64 8^4 311 -> 290, 12^4 489 -> 460, 24^4 1886 -> 1861.  The gain is what the launches cost,
-// some 25 us; beyond the limit it is less than the runs of one side differ by.
+// therefore replayed from a captured graph once a handle has asked for the same measurement kMeasGraphCalls times in a
+// row; the smearing steps stay programmatic launches in it.  Q after 24 steps, 35 loops after 50 steps on B200, us a call,
+// direct and replayed: FP32 8^4 320, 295; 20x14x16x16 457, 416; FP64 8^4 325, 312; 24^4 1936, 1903.  The call that captures,
+// instantiates and first launches the graph takes 360 to 430 us more (24^4: 2340; 20x14x16x16: 790), what some 11 replays
+// save: a program that stops before the limit has paid nothing, any other at most twice what the calls could have cost.
+// The saving being the launches' and so the same for any field, it is under 2 % from 24^4 FP64 (42 MB) on, hence the limit.
 #include <algorithm>
 #include <array>
 #include <cmath>
@@ -29,9 +30,10 @@ using namespace su2g;
 using MeasKey = std::tuple<std::vector<int32_t>, std::vector<int32_t>, std::vector<int32_t>, std::array<double, 3>,
                            std::array<int, 3>, std::array<void*, 6>, const void*>;
 
-// The last measurement and, from its second call on, its graph.
+// The last measurement, how often it was asked for in a row, and its graph.
 struct su2g_meas_graph {
     MeasKey key;
+    int calls = 1;
     std::vector<int> slot;   // d_out slot of each loop
     int nres = 0;            // d_out slots to fetch
     cudaGraphExec_t exec = nullptr;
@@ -84,6 +86,7 @@ struct Smeared {
 };
 
 constexpr size_t kMeasGraphBytes = 64ull << 20;
+constexpr int kMeasGraphCalls = 12;
 
 int enqueue(su2g_lattice* h, const su2g_meas_spec* sp, std::vector<int>& slot, int& nres)
 {
@@ -166,7 +169,8 @@ extern "C" int su2g_measure(su2g_lattice* h, const su2g_meas_spec* sp, double* q
     int nres = 0;
     const bool again = !h->profiling && 4ull * h->g.V * h->link_bytes <= kMeasGraphBytes && h->meas &&
                        h->meas->key == key_of(h, sp);
-    if (again) {
+    if (again && h->meas->calls < kMeasGraphCalls) ++h->meas->calls;
+    if (again && h->meas->calls == kMeasGraphCalls) {
         if (!h->meas->exec && (rc = capture(h, sp, h->meas))) {
             release_meas_graph(h);
             return rc;
@@ -175,9 +179,9 @@ extern "C" int su2g_measure(su2g_lattice* h, const su2g_meas_spec* sp, double* q
         nres = h->meas->nres;
         if ((rc = check_cuda(h, cudaGraphLaunch(h->meas->exec, h->stream), "replaying the measurement graph"))) return rc;
     } else {
-        release_meas_graph(h);
+        if (!again) release_meas_graph(h);
         if ((rc = enqueue(h, sp, slot, nres))) return rc;
-        h->meas = new su2g_meas_graph{key_of(h, sp), {}, 0, nullptr};
+        if (!again) h->meas = new su2g_meas_graph{key_of(h, sp)};
     }
     if ((rc = fetch_results(h, 0, nres))) return rc;
     for (int i = 0; i < sp->n_q; ++i) q[i] = h->h_out[2 * i];

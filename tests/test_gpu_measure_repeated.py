@@ -1,0 +1,71 @@
+"""su2g_measure called again and again on one handle: every call gives what the same steps give one by one, whatever
+happened to the handle's buffers in between, and the second call costs what the later ones do."""
+import time
+
+import numpy as np
+import pytest
+
+import _oracle as O
+from masterarbeit_b200 import Lattice
+
+pytestmark = pytest.mark.gpu
+
+A = dict(q_ape=[1, 3], alpha_q=0.5, R=[1, 2], T=[1, 2], ns_t=1, alpha_t=0.3, ns_s=2, alpha_s=0.5)
+B = dict(q_ape=[2], alpha_q=0.4, R=[1, 3, 3], T=[3, 1, 2], ns_t=0, alpha_t=0.0, ns_s=1, alpha_s=0.25)
+
+
+def _steps(L, U, R, T, q_ape, alpha_q, ns_t, alpha_t, ns_s, alpha_s):
+    L.upload(U)
+    q, done = [], 0
+    for n in q_ape:
+        L.ape(n - done, alpha_q, "all")
+        done = n
+        q.append(L.qtop())
+    L.upload(U)
+    L.ape(ns_t, alpha_t, "temporal")
+    L.ape(ns_s, alpha_s, "spatial")
+    return np.array(q), np.array(L.wilson(R, T))
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("dims", [(6, 4, 4, 8), (8, 6, 10, 4)])
+def test_each_call_equals_its_steps(dims, precision):
+    L, step = Lattice(dims, precision=precision), Lattice(dims, precision=precision)
+
+    def check(spec, seed):
+        U = O.start(dims, "haar", seed)
+        L.upload(U)
+        qs, ws = _steps(step, U, **spec)
+        for _ in range(5):
+            q, w = L.measure(**spec)
+            assert np.array_equal(q, qs) and np.array_equal(w, ws), seed
+
+    for seed in range(1, 5):          # the same measurement of new configurations, replayed in the end
+        check(A, seed)
+    L.ape(1, 0.2, "all")              # the field's links move to the other buffer
+    check(A, 5)
+    L.wilson([1] * 5 + [2] * 5, [1, 2, 3, 4, 5] * 2)
+    check(B, 6)                       # A, B, A, A, A
+    for seed in range(7, 10):
+        check(A, seed)
+    L.profile(True)
+    check(A, 10)
+    L.profile(False)
+    check(A, 11)
+    L.measure_release()
+    check(B, 12)
+
+
+def test_the_second_call_is_as_fast_as_the_later_ones():
+    spec = dict(q_ape=[12, 24], alpha_q=0.5, R=[1, 2, 3], T=[1, 2, 3], ns_s=50, alpha_s=0.5)
+    ratios = []
+    for seed in range(3):             # a stalled host must not decide: the best of three handles
+        L = Lattice((20, 14, 16, 16), precision="fp64", start="haar", seed=seed)
+        t = []
+        for _ in range(12):
+            t0 = time.perf_counter()
+            L.measure(**spec)
+            t.append(time.perf_counter() - t0)
+        ratios.append(t[1] / np.median(t[2:]))   # the first call allocates
+        L.close()
+    assert min(ratios) < 1.5, ratios
