@@ -28,8 +28,9 @@ __host__ __device__ constexpr bool ape_staple(int mode, int mu, int nu)
 // loads (7) do not wait for a link's end.  Against link by link, where one link's state at a time is live but
 // U_nu(x-nu) stays in registers or is read again: FP64 24^4 30.2 -> 28.4 us a step, 48^4 512 -> 487; FP32 24^4 16.2 -> 15.3,
 // 40x30x36x34 72 -> 64, 48^4 250 -> 235.  The spatial and temporal steps have no more than two links a plane and
-// keep the order by links (spatial by planes: FP64 0 to 2 %, FP32 spills at eight CTAs per SM).
-template <typename R, int MODE, typename F, typename Emit>
+// keep the order by links (spatial by planes: FP64 0 to 2 %, FP32 spills at eight CTAs per SM); so does the FP32 step on
+// fields of large time slices (PLANES false, k_ape).
+template <typename R, int MODE, bool PLANES = true, typename F, typename Emit>
 __device__ __forceinline__ void ape_staples(const F& in, const Geom& g, const Site& s, int par, int h, Emit&& emit)
 {
     const int q = par ^ 1;
@@ -56,7 +57,7 @@ __device__ __forceinline__ void ape_staples(const F& in, const Geom& g, const Si
             if (a) S[mu] = q_mul_add(S[mu], u[nu], P);      // U_nu(x) U_mu(x+nu) U_nu(x+mu)^dag
             if (b) S[nu] = q_mul_nd_add(S[nu], u[mu], P);   // U_mu(x) U_nu(x+mu) U_mu(x+nu)^dag
         }
-    if (MODE == SU2G_APE_ALL) {   // plane by plane
+    if (MODE == SU2G_APE_ALL && PLANES) {   // plane by plane
 #pragma unroll
         for (int nu = 0; nu < 4; ++nu) {
             const Q<R> a = in.ld(nu, q, xm[nu]);   // U_nu(x-nu), of all three links

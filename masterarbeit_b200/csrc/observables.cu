@@ -68,15 +68,12 @@ __global__ void __launch_bounds__(128, 8) k_plaquette(Field<R> Unc, Geom g, DD* 
 // with six, 164 us with two).  FP64 APE_all three (24^4: 284 us ten steps against 295 with four, 324 with two),
 // spatial four (48^4: 337 us against 359 us with three, 357 us with two of 256, before 256-bit
 // loads), temporal eight (212 against 216 us with four of 256).
-template <typename R, int MODE>
+constexpr int kApeBlock = 128;
+
+template <typename R, int MODE, bool WIDE>
 constexpr int ape_min_blocks()
 {
-    return MODE == SU2G_APE_ALL ? (sizeof(R) == 4 ? 5 : 3) : (sizeof(R) == 4 || MODE == SU2G_APE_TEMPORAL ? 8 : 4);
-}
-template <typename R, int MODE>
-constexpr int ape_block()
-{
-    return 128;
+    return MODE == SU2G_APE_ALL ? (sizeof(R) == 4 ? (WIDE ? 4 : 5) : 3) : (sizeof(R) == 4 || MODE == SU2G_APE_TEMPORAL ? 8 : 4);
 }
 
 // A step is a programmatic dependent launch (pdl_wait): the CTAs of the next step take the slots that the
@@ -85,19 +82,31 @@ constexpr int ape_block()
 // end: with plain loads, a store between them keeps the later ones behind it (FP32 all at 24^4 190 -> 169 us).
 // A step is bound by latency between the L1's and the issue slots' limits (FP32 spatial: 55-67 % and 68 %); tiles
 // of two, four or eight x planes a CTA, for more hits in L1, were 2 to 30 % slower.
-template <typename R, int MODE>
-__global__ void __launch_bounds__(ape_block<R, MODE>(), ape_min_blocks<R, MODE>()) k_ape(Field<R> in, Field<R> out,
-                                                                                        Geom g, R alpha)
+//
+// WIDE: launched in order, read-only loads, links stored as they come, the order by links in four CTAs per SM.  It is
+// the FP32 step of fields whose t-1, t and t+1 slices and the slice written exceed L2 together, where fewer sites in flight
+// keep more neighbours there.  A step, us, overlapped / overlapped with four CTAs / WIDE: all 48^4 235 / 258 / 252, 64^4 797 /
+// 835 / 833, 72^4 1443 / 1446 / 1438, 76^4 1910 / - / 1830, 80^4 2379 / 2294 / 2252, 96^4 5012 / 4836 / 4693, 12x96^3 628 / - / 590;
+// spatial 64^4 447 / - / 442, 76^4 933 / - / 908, 80^4 1119 / - / 1097, 96^4 2366 / - / 2290; temporal 64^4 339 / - / 337, 96^4 2057 /
+// - / 1990.  (Below that line the order of launches alone makes 1 to 2 %.)
+template <typename R, int MODE, bool WIDE>
+__global__ void __launch_bounds__(kApeBlock, ape_min_blocks<R, MODE, WIDE>()) k_ape(Field<R> in, Field<R> out, Geom g, R alpha)
 {
     // one site per thread; CTAs dispatched in order, warps alternating parity over the same h run
     // (so that both parities of a region share an L1: FP32 APE_all 237.8 against 240.7 us, spatial
     // 129.1 against 131.6 us, FP64 spatial 355 against 367 us with parity-alternating CTAs)
     Site s{};
     int par, h;
-    pdl_trigger();
+    if (!WIDE) pdl_trigger();
     const bool valid = site_warp_pair(g, blockIdx.x, threadIdx.x, blockDim.x, s, par, h);
-    pdl_wait(h, s.n);
+    if (!WIDE) pdl_wait(h, s.n);
     if (!valid) return;
+    if (WIDE) {
+        ape_staples<R, MODE, false>(in, g, s, par, h, [&](int mu, const Q<R>& u, const Q<R>& S) {
+            out.sth(mu, par, h, q_project(q_axpy(alpha, S, u)));
+        });
+        return;
+    }
     Q<R> res[4];
     ape_staples<R, MODE>(field_ca(in), g, s, par, h, [&](int mu, const Q<R>& u, const Q<R>& S) {
         res[mu] = q_project(q_axpy(alpha, S, u));
@@ -547,9 +556,14 @@ int ensure_alt(su2g_lattice* h)
 template <typename R, int MODE>
 void launch_ape_t(su2g_lattice* h, const Field<R>& in, const Field<R>& out, R alpha)
 {
-    constexpr int block = ape_block<R, MODE>();
-    const int grid = (int)((2 * (long long)h->g.Vh + block - 1) / block);   // warp pairs over the same h run
-    launch_pdl(k_ape<R, MODE>, grid, block, h->stream, in, out, h->g, alpha);
+    const int grid = (int)((2 * (long long)h->g.Vh + kApeBlock - 1) / kApeBlock);   // warp pairs over the same h run
+    if constexpr (sizeof(R) == 4) {
+        if (4 * 4ull * h->g.S[0] * h->link_bytes > h->l2_bytes) {   // four time slices
+            k_ape<R, MODE, true><<<grid, kApeBlock, 0, h->stream>>>(in, out, h->g, alpha);
+            return;
+        }
+    }
+    launch_pdl(k_ape<R, MODE, false>, grid, kApeBlock, h->stream, in, out, h->g, alpha);
 }
 
 template <typename R>
