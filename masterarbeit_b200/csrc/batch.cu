@@ -196,8 +196,7 @@ __global__ void __launch_bounds__(256, 4) k_batch_update(BatchGrid a, int par, u
     }
 }
 
-// One site per thread, parities paired per warp; one partial per CTA (plain FP64 within a warp,
-// compensated across its warps), 256 threads at most.
+// One site per thread, parities paired per warp; one compensated partial per CTA, 256 threads at most.
 template <typename R, bool UNI>
 __global__ void __launch_bounds__(256) k_batch_plaquette(BatchGrid a, DD* __restrict__ partials)
 {
@@ -228,14 +227,12 @@ __global__ void __launch_bounds__(256) k_batch_plaquette(BatchGrid a, DD* __rest
                 site += (double)q_dot(x, y);
             }
     }
-    __shared__ double part[8];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) site += __shfl_xor_sync(0xffffffffu, site, o);
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = site;
+    __shared__ DD part[8];
+    DD v = dd_warp_sum(DD{site, 0.0});
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
     __syncthreads();
     if (threadIdx.x == 0) {
-        DD v = {0.0, 0.0};
-        for (int w = 0; w < (int)blockDim.x >> 5; ++w) v = dd_add(v, part[w]);
+        for (int w = 1; w < (int)blockDim.x >> 5; ++w) v = dd_add(v, part[w]);
         partials[UNI ? blockIdx.y * gridDim.x + blockIdx.x : blockIdx.x] = v;
     }
 }
