@@ -29,8 +29,8 @@ constexpr int kCluster = 16;        // CTAs (non-portable size, asked for at cre
 constexpr int kChainThreads = 128;   // per CTA
 
 // `n_blocks` blocks of `every` sweeps of n_hb heatbath and n_or overrelaxation sub-sweeps.  Block b's sums go
-// to parts + b stride: three fused passes of `warps` plaquette partials (with plaq), then the acceptance's
-// (acc 1: set, 2: added to what is there).
+// to parts + b stride: `warps` entries of the acceptance (acc 1: set, 2: added to what is there), then three fused passes of
+// as many plaquette partials (with plaq).
 struct ChainArgs {
     int n_blocks, every, n_hb, n_or;
     DD* parts;
@@ -143,19 +143,19 @@ __global__ void __launch_bounds__(kChainThreads, 1) k_chain(Field<double> U0, Ge
     for (int b = 0; b < a.n_blocks; ++b) {
         DD* part = a.parts + b * a.stride + warp;
         const bool sums = warp < a.warps;
-        double acc = a.acc == 2 && sums ? part[3 * a.warps].s : 0.0;
+        double acc = a.acc == 2 && sums ? part->s : 0.0;
         int left = a.every * (a.n_hb + a.n_or);
         for (int s = 0; s < a.every; ++s) {
 #pragma unroll 1
             for (int i = 0; i < a.n_hb; ++i, ++sweep)
                 chain_sweep<SU2G_HEATBATH>(l, kb, keys, sweep, replica, status, a.acc ? &acc : nullptr,
-                                              --left == 0 && a.plaq, sums ? part : nullptr, a.warps);
+                                              --left == 0 && a.plaq, sums ? part + a.warps : nullptr, a.warps);
 #pragma unroll 1
             for (int i = 0; i < a.n_or; ++i)
                 chain_sweep<SU2G_OVERRELAX>(l, kb, keys, sweep, replica, status, nullptr,
-                                               --left == 0 && a.plaq, sums ? part : nullptr, a.warps);
+                                               --left == 0 && a.plaq, sums ? part + a.warps : nullptr, a.warps);
         }
-        if (a.acc && sums && (threadIdx.x & 31) == 0) part[3 * a.warps] = DD{acc, 0.0};
+        if (a.acc && sums && (threadIdx.x & 31) == 0) *part = DD{acc, 0.0};
     }
     cluster_wait();
 }

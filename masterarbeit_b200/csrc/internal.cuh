@@ -256,14 +256,14 @@ int sweep_plaq_finalize(su2g_lattice* h, const DD* parts, int nslots, size_t str
 int sweep_acc_finalize(su2g_lattice* h, const DD* parts, int nslots, size_t stride, double* out, int out_stride = 1);
 // Small FP64 lattices (h->chain): whole blocks of sweeps in one launch.  chain_prepare decides (once
 // per handle, at creation).  chain_enqueue runs n_blocks blocks of `every` x (n_hb + n_or) sub-sweeps; block
-// b's plaquette partials (plaq) and acceptance entries (acc 1: set, 2: added to) go to parts + b stride and + 3 sweep_warps.
+// b's acceptance entries (acc 1: set, 2: added to) and plaquette partials (plaq) go to parts + b stride and + sweep_warps.
 void chain_prepare(su2g_lattice* h);
 int chain_enqueue(su2g_lattice* h, int n_blocks, int every, int n_hb, int n_or, uint32_t sweep0, DD* parts, size_t stride,
                   bool plaq, int acc);
 constexpr int kChainSubSweeps = 1024;   // sub-sweeps one launch runs at most (some 20 ms)
 // Enqueue n_sweeps x (n_hb heatbath + n_or overrelaxation sweeps); heatbath sub-sweep j (counted
-// from 0 within the call) has index sweep0 + j.  With plaq (there must be a sub-sweep) the last one leaves
-// its three fused passes' plaquette partials at parts, with acc (there must be a heatbath sub-sweep) the
-// acceptance of them all goes to parts + 3 sweep_warps.
+// from 0 within the call) has index sweep0 + j.  With acc (there must be a heatbath sub-sweep) the
+// acceptance of them all goes to parts, with plaq (there must be a sub-sweep) the last one leaves its three fused
+// passes' plaquette partials at parts + sweep_warps.
 int sweep_enqueue(su2g_lattice* h, int n_sweeps, int n_hb, int n_or, uint32_t sweep0, DD* parts, bool plaq, bool acc);
 }  // namespace su2g

@@ -35,7 +35,7 @@ extern "C" int su2g_graph_run(su2g_lattice* h, int32_t n_blocks, int32_t meas_ev
     if (n_blocks == 0) return SU2G_OK;
     cudaSetDevice(h->device);
     const bool fused = n_hb + n_or > 0, with_acc = n_hb > 0;
-    const size_t warps = sweep_warps(h), parts = 4 * warps;   // a block's: the plaquette's three passes, the acceptance
+    const size_t warps = sweep_warps(h), parts = 4 * warps;   // a block's: the acceptance, the plaquette's three passes
     const int group = std::max<int>(1, std::min<size_t>(kFinSlots, kPlaqScratchBytes / (parts * sizeof(DD))));
     const bool grouped = h->chain && fused && !h->profiling &&
                          (long long)group * meas_every * (n_hb + n_or) <= kChainSubSweeps;
@@ -56,8 +56,8 @@ extern "C" int su2g_graph_run(su2g_lattice* h, int32_t n_blocks, int32_t meas_ev
             if (!fused) {
                 rc = plaquette_enqueue(h, h->d_out + 2 * i);
             } else if (j == group - 1 || i == n - 1) {
-                rc = sweep_plaq_finalize(h, h->partials, j + 1, parts, out, 2);
-                if (!rc && with_acc) rc = sweep_acc_finalize(h, h->partials + 3 * warps, j + 1, parts, out + 1, 2);
+                rc = sweep_plaq_finalize(h, h->partials + warps, j + 1, parts, out, 2);
+                if (!rc && with_acc) rc = sweep_acc_finalize(h, h->partials, j + 1, parts, out + 1, 2);
             }
         }
         if (!rc) rc = fetch_results(h, 0, 2 * n);

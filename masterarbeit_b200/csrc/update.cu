@@ -346,7 +346,7 @@ extern "C" int su2g_update_pass(su2g_lattice* h, int32_t kind, int32_t mu, int32
 int su2g::sweep_enqueue(su2g_lattice* h, int n_sweeps, int n_hb, int n_or, uint32_t sweep0, DD* part0, bool with_plaq, bool with_acc)
 {
     const int parts = sweep_warps(h);   // per fused pass
-    DD *plaq_part = with_plaq ? part0 : nullptr, *acc_part = with_acc ? part0 + 3 * parts : nullptr;
+    DD *acc_part = with_acc ? part0 : nullptr, *plaq_part = with_plaq ? part0 + parts : nullptr;
     const int subs = n_sweeps * (n_hb + n_or);
     // (profiling times every pass; a sweep of more sub-sweeps than a launch may run goes pass by pass)
     if (h->chain && !h->profiling && n_hb + n_or > 0 && n_hb + n_or <= kChainSubSweeps) {
@@ -389,13 +389,13 @@ int sweep_call(su2g_lattice* h, int32_t n_sweeps, int32_t n_hb, int32_t n_or, do
     const int slot_acc = 0, slot_plaq = 1;
     const size_t warps = sweep_warps(h);
     const bool fused = plaq_out && n_sweeps * (n_hb + n_or) > 0, acc = acc_out && n_sweeps * n_hb > 0;
-    int rc = fused || acc ? ensure_partial_entries(h, 4 * warps) : SU2G_OK;
+    // partials: the acceptance, then three passes of the plaquette (none for a sweep that returns the acceptance alone)
+    int rc = fused || acc ? ensure_partial_entries(h, fused ? 4 * warps : warps) : SU2G_OK;
     if (rc) return rc;
-    // partials: three passes of the plaquette, then the acceptance
     if ((rc = sweep_enqueue(h, n_sweeps, n_hb, n_or, h->hb_sweeps, h->partials, fused, acc))) return rc;
-    if (fused) rc = sweep_plaq_finalize(h, h->partials, 1, 0, h->d_out + slot_plaq);
+    if (fused) rc = sweep_plaq_finalize(h, h->partials + warps, 1, 0, h->d_out + slot_plaq);
     else if (plaq_out) rc = plaquette_enqueue(h, h->d_out + slot_plaq);
-    if (!rc && acc) rc = sweep_acc_finalize(h, h->partials + 3 * warps, 1, 0, h->d_out + slot_acc);
+    if (!rc && acc) rc = sweep_acc_finalize(h, h->partials, 1, 0, h->d_out + slot_acc);
     if (rc) return rc;
     h->hb_sweeps += (uint32_t)(n_sweeps * n_hb);
     if (acc_out || plaq_out) {
