@@ -199,6 +199,8 @@ __global__ void __launch_bounds__(kFinWideThreads) k_finalize_wide(const DD* par
 int finalize(su2g_lattice* h, const DD* parts, int nparts, int nslots, size_t stride, double scale, double* out,
              int out_stride)
 {
+    if (out < h->d_out || (out - h->d_out) + (nslots - 1) * (ptrdiff_t)out_stride >= kOutSlots)
+        return set_error(h, SU2G_EINVAL, "too many result slots");
     launch_begin(h, SU2G_K_REDUCE);
     if (nslots <= kFinSlots && nparts > 4 * kFinalizeBlock) {
         const int nb = std::min(kFinBlocks, (nparts + 2 * kFinWideThreads - 1) / (2 * kFinWideThreads));
