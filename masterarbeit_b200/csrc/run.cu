@@ -50,8 +50,8 @@ extern "C" int su2g_graph_run(su2g_lattice* h, int32_t n_blocks, int32_t meas_ev
             if (!grouped) rc = sweep_enqueue(h, meas_every, n_hb, n_or, h->hb_sweeps, part, fused, with_acc);
             else if (j == 0)   // the whole group in one launch
                 rc = chain_enqueue(h, std::min(group, n - i), meas_every, n_hb, n_or, h->hb_sweeps, part, parts, true, with_acc);
-            h->hb_sweeps += (uint32_t)(meas_every * n_hb);
             if (rc) break;
+            h->hb_sweeps += (uint32_t)(meas_every * n_hb);
             double* out = h->d_out + 2 * (i - j);
             if (!fused) {
                 rc = plaquette_enqueue(h, h->d_out + 2 * i);
