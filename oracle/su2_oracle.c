@@ -523,7 +523,7 @@ int su2o_sweep(const int dims[4], double *U, int kind, double beta, uint64_t see
 {
     lat_t g;
     if (lat_init(&g, dims)) return -1;
-    double a = 0.0;
+    long double a = 0.0;   /* 20 million terms at 48^4: a double's own rounding would be 1e-13 of the mean */
     for (int mu = 0; mu < 4; ++mu)
         for (int p = 0; p < 2; ++p)
             for (uint64_t n = 0; n < g.V; ++n) {
@@ -533,7 +533,7 @@ int su2o_sweep(const int dims[4], double *U, int kind, double beta, uint64_t see
                 else
                     or_link(&g, U, n, mu);
             }
-    if (acc) *acc = a / (4.0 * (double)g.V);
+    if (acc) *acc = (double)(a / (4.0 * (double)g.V));
     return 0;
 }
 
