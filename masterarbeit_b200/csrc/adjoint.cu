@@ -98,8 +98,9 @@ __device__ __forceinline__ Q<R> line_gradient(const FieldCA<R>& L, const R* fbar
 // walk over every leaf that added each link's term with an atomic (1728 products and 576 atomics a site;
 // here 36 line gradients of about 15 products and 36 loads each): a whole VJP of five steps without the
 // gradient's copy at 24^4 on B200 1580 -> 825 us (FP32) and 5290 -> 1510 us (FP64), at 8^4 605 -> 200 us
-// (FP64).  Two to five CTAs per SM asked for in FP64 and four to eight in FP32 measured the same within
-// 3 %, so the compiler's own register count stands.
+// (FP64).  Asking for two to six CTAs per SM changed a VJP of ten steps by less than 3 % from 8^4 to 32^4 (32^4: FP64 7.80
+// ms as it is, 7.78, 7.64, 7.61, 7.61 with two, three, four, six; FP32 4.29, 4.29, 4.28, 4.29, 4.14), so the compiler's own
+// register count (86 in FP64) stands.  FP64 at 32^4: 54 % of the FP64 pipe, L1 and L2 at 52 and 54 %.
 constexpr int kLineBlock = 128;
 
 template <typename R>
@@ -164,6 +165,10 @@ __global__ void __launch_bounds__(kBlock) k_line_chain(Field<R> Unc, Field<R> L2
 // 128-thread CTAs for both kernels; per SM four (FP32) and three (FP64) for v-bar, five and four for the
 // gather, whose loads otherwise all run ahead (202 registers in FP64).  A VJP of five steps at 24^4, us:
 // FP64 1552 -> 1361, FP32 785 -> 740 against two 256-thread CTAs for v-bar and no bound for the gather.
+// One shape serves all grids: a VJP of ten steps, us, with 2, 3, 4 and 6 CTAs for v-bar: FP64 8^4 236, 235, 240, 256;
+// 16x12x16x20 566, 562, 563, 638; 24^4 2559, 2454, 2460, 2688; 32^4 8161, 7794, 7695, 8381; FP32 16x12x16x20 390, 387, 381, 398,
+// 32^4 4249, 4263, 4186, 4148; with 3, 4, 5, 6 for the gather: FP64 8^4 228, 237, 238, 237; 16x12x16x20 560, 563, 563, 587; 24^4 2525,
+// 2442, 2469, 2503; 32^4 8088, 7760, 7744, 7845; FP32 all within 2 %.
 constexpr int kSmearAdjBlock = 128;
 
 // v-bar(x, mu) = (Gn - u' <u', Gn>) / |v|,  v = U + alpha S,  u' = v / |v|  (all four directions).

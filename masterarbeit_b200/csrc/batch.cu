@@ -4,10 +4,10 @@
 // hot/cold start and id).  Here a batch holds R replicas of possibly different extents, beta,
 // seed and start in one device pool.  A replica-offset table maps every CTA of a launch to its
 // replica, so one launch per checkerboard pass (mu, parity) updates all replicas, and one launch
-// measures every replica's plaquette.  The launches of a run are enqueued at once, as programmatic
-// dependent ones (pdl_wait): each starts in the tail of the one before.  Each replica draws the same Philox
-// streams as a single-lattice handle with the same (seed, replica id), so a batch and a set of single
-// handles give identical fields.
+// measures every replica's plaquette.  Large batches enqueue the launches of a run at once, as programmatic
+// dependent ones (pdl_wait): each starts in the tail of the one before; small ones replay a captured block of
+// ordinary launches (small_batch).  Each replica draws the same Philox streams as a single-lattice handle with the
+// same (seed, replica id), so a batch and a set of single handles give identical fields.
 //
 // Persistent form.  Alternatively one cooperative launch runs every measurement block of a
 // su2g_batch_run: its CTAs (all resident) walk the links of each pass as one global index over all
@@ -548,10 +548,12 @@ BatchGrid batch_grid(const su2g_batch* b, bool sites)
 
 // A batch is small when a pass has fewer links than fill the SMs about twice over at 256 threads a CTA.
 // A pass of a small batch is as short as a launch takes the host, and the CTAs of an overlapping launch
-// crowd on the SMs the running one leaves idle (16 x 8^4, 1 HB + 4 OR, us a sweep: 115 FP32, 184 FP64
-// one after another; 143, 234 overlapping).  Small batches therefore replay a captured block of ordinary
-// launches; the others launch pass by pass, programmatically, FP32 with two trials drawn early (64 x 8^4:
-// 193 -> 172 FP32, 377 -> 282 FP64).
+// crowd on the SMs the running one leaves idle.  Small batches therefore replay a captured block of ordinary
+// launches; the others launch pass by pass, programmatically, FP32 with two trials drawn early.  1 HB + 4 OR and the
+// plaquette on B200, us a sweep, replayed / pass by pass, FP32 and FP64:
+//    4 x 6^4    103 / 101   144 / 144       46 x 8^4   154 / 171   238 / 277   (94208 links, the line is at 94720)
+//    16 x 8^4   107 / 161   148 / 242       64 x 8^4   195 / 175   290 / 288
+//    32 x 8^4   129 / 164   184 / 261       64 x 12^4  685 / 648   1600 / 1586
 bool small_batch(const su2g_batch* b) { return b->links <= 640ll * b->num_sms; }
 
 template <typename R, int MU, int KIND>

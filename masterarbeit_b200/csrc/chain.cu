@@ -11,10 +11,12 @@
 // multiply-adds out in FP64).  FP32 leaves them to the compiler, which starts a refused link's sums elsewhere here than in
 // the passes; FP32 fields being the same in a batch and in a handle, FP32 keeps to the passes.
 //
-// Measured, FP64, call by call (passes -> here): 20 heatbath sweeps 525 -> 430 us (8^4), 509 -> 369 us (4^4);
-// the loop of 10 sweeps, plaquette and acceptance 360 -> 252 us (8^4).  The line lies at one link per thread
-// of 128-thread CTAs: with 256 threads the heatbath's registers leave one warp per scheduler waiting for two,
-// and the one SM's load queue takes the links of both (10^4: 661 us against the passes' 580).
+// Measured, FP64, passes -> here: 20 heatbath sweeps 427-530 -> 387-409 us (8^4), 390 -> 363 us (4^4); the loop of 10 sweeps,
+// plaquette and acceptance 291 -> 237 us (8^4), 243 -> 225 us (4^4); four times 1 heatbath and 4 overrelaxation sweeps 384 -> 326
+// us (8^4).  The line lies at one link per thread of 128-thread CTAs: with 256 threads the heatbath's registers leave one
+// warp per scheduler waiting for two, and the one SM's load queue takes the links of both (8^4 455 against 387 us; 10^4 514 us,
+// as long as the passes).  A sweep at 8^4 issues in 12 % of its SMs' cycles, the FP64 pipes 10 % busy; a warp waits 2.7
+// cycles per instruction for instructions, 1.5 for fixed latencies, 1.1 for loads and 1.0 for the barrier's fence.
 #include <algorithm>
 
 #include "internal.cuh"
@@ -57,15 +59,6 @@ struct ChainLink {
     bool active;
     Site s[2];
 };
-
-// What the thread keeps of a heatbath pass for its warp's acceptance.
-__device__ __forceinline__ double warp_acceptance(uint32_t trials)
-{
-    double a = (double)__popc(__ballot_sync(0xffffffffu, trials == 1u));
-    for (unsigned more = __ballot_sync(0xffffffffu, trials > 1u); more; more &= more - 1u)
-        a += 1.0 / (double)__shfl_sync(0xffffffffu, trials, __ffs(more) - 1);
-    return a;
-}
 
 template <int MU, int KIND, bool PLQ>
 __device__ __forceinline__ void chain_pass(const ChainLink& l, int par, const KpBeta<double>& kb, const PhiloxKeys& keys, uint32_t sweep,

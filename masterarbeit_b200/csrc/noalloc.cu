@@ -175,8 +175,8 @@ extern "C" int su2g_ape_inplace_noalloc(double* links, const int32_t dims[4], in
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess)
         return set_error(nullptr, SU2G_ECUDA, "su2g_ape_inplace_noalloc: %s", cudaGetErrorString(e));
-    // The kernels read and write the field as double2, so it must be 16-byte aligned device (or
-    // managed) memory of the current device.  Callers hand in sub-allocations of their own pools,
+    // The kernels access the field 16 bytes at a time (32 where its alignment allows), so it must be 16-byte
+    // aligned device (or managed) memory of the current device.  Callers hand in sub-allocations of their own pools,
     // so a bad pointer is refused here instead of faulting on the GPU.  Neither check allocates.
     if (((uintptr_t)links & 15u) != 0)
         return set_error(nullptr, SU2G_EINVAL,

@@ -11,7 +11,7 @@
 // The launches are programmatic dependent ones (k_update), each starting in the tail of the one before.
 // A captured graph of a block, replayed, ran slower on B200: its nodes did not overlap in that way and
 // each replay began with a full dependency (FP64 heatbath with the plaquette every sweep, us a sweep:
-// 8^4 51.2 as a graph, 37.8 as passes and 25.2 as one cluster launch, chain.cu; 24^4 140 and 92; 48^4 1520 and 1290
+// 8^4 51.2 as a graph, 29.1 as passes and 23.7 as one cluster launch, chain.cu; 24^4 140 and 92; 48^4 1520 and 1290
 // -- with the faster passes).
 #include <algorithm>
 

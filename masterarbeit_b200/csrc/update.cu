@@ -35,13 +35,28 @@ constexpr int kUpdateBlock = 128;
 //  - Larger grids: six CTAs per SM while the FP64 field stays in L2, or while a FP32 grid is at most
 //    one wave of eight; else eight (32 warps per SM; against 8, 16, 24 and 48 the fastest at 48^4), where
 //    FP64 draws nothing early (no registers left).
-// Twenty FP64 / FP32 heatbath sweeps on B200, ms, with the kernel for 2, 3, 4, 6, 8 CTAs (FP64: eight without
-// early draws):
-//    16^4           0.69 0.81 0.85 1.01 0.95      0.57 0.63 0.63 0.72 0.85
-//    24x14x18x22    1.11 1.05 0.92 1.21 1.04      0.59 0.60 0.60 0.77 0.82
-//    24^4           2.10 1.72 1.67 1.64 1.90      1.10 1.10 1.10 0.94 0.97
-//    28^4           3.80 3.08 2.88 2.65 2.82      1.74 1.74 1.74 1.48 1.47
-//    48^4                          24.6 23.5                     12.8 12.7
+// Twenty sweeps at beta = 3.09 on B200, ms, with the kernel for 2, 3, 4, 6, 8 CTAs (FP64 heatbath: eight without early draws).
+//                    heatbath FP64                   FP32
+//    10x12x14x12     0.48  0.42  0.46  0.59  0.77    0.41  0.41  0.40  0.44  0.47
+//    16^4            0.53  0.59  0.67  0.84  1.38    0.57  0.57  0.57  0.68  0.79
+//    24x14x18x22     0.97  0.98  0.72  1.03  1.59    0.59  0.59  0.59  0.73  0.82
+//    24^4            2.07  1.63  1.54  1.66  1.96    1.12  1.12  1.12  0.95  1.00
+//    28^4            3.91  3.03  2.74  2.60  2.88    1.76  1.76  1.76  1.51  1.50
+//    40^4                        13.3  12.9  12.9
+//    48^4            35.4  26.3  24.4  24.8  24.5    15.1  15.0  14.9  12.6  12.2
+//    64^4                        86.3  80.9  78.4
+//                    overrelaxation FP64             FP32
+//    14x10x12x18     0.40  0.40  0.39  0.54  0.54    0.42  0.54  0.57  0.51  0.53
+//    16^4            0.58  0.57  0.63  0.72  0.80    0.64  0.64  0.64  0.68  0.78
+//    18x14x18x22     0.60  0.59  0.68  0.78  0.87    0.48  0.48  0.50  0.52  0.56
+//    24x14x18x22     0.70  0.69  0.68  0.85  0.99    0.50  0.49  0.49  0.55  0.61
+//    20^4            0.77  0.76  0.78  0.84  1.07    0.50  0.50  0.50  0.54  0.63
+//    24^4            1.18  1.16  1.18  1.20  1.27    0.74  0.74  0.74  0.76  0.76
+//    28^4            2.25  2.22  2.14  2.03  2.04    1.17  1.17  1.17  1.11  1.06
+//    40x30x36x34     6.81  6.88  6.86  6.61  6.35    3.44  3.43  3.44  3.25  3.05
+//    48^4            23.4  23.2  23.2  22.9  23.0    12.3  12.4  12.3  12.4  11.3
+// Overrelaxation has the kernels for two (FP64), four and eight only: between 592 CTAs and a few waves (20^4) the one
+// for three or four would be the faster.
 struct UpdateShape {
     int ctas, early;
 };
@@ -80,7 +95,7 @@ int update_shape(const su2g_lattice* h, int grid)
 // frees, find their sites, and wait there.  EARLY > 0: they also draw that many trials and the angles
 // before the wait (they need no links), which leaves loads, staple and the end of the draw behind it.
 // One trial is refused in 30, so with one drawn early most passes still end with a warp that draws
-// again (20 FP64 sweeps at 10x12x14x12: 0.81, 0.72, 0.59 ms with one, two, three; 0.82 with none).
+// again (20 FP64 sweeps at 10x12x14x12: 0.63, 0.56, 0.48 ms with one, two, three; 0.79 with none).
 template <typename R, int MU, int KIND, bool PLQ, int CTAS, int EARLY>
 __global__ void __launch_bounds__(kUpdateBlock, CTAS)
     k_update(Field<R> Unc, Geom g, int par, KpBeta<R> kb, PhiloxKeys seed, uint32_t sweep, uint32_t replica,
@@ -132,10 +147,7 @@ __global__ void __launch_bounds__(kUpdateBlock, CTAS)
     // an atomic: the loop of sweeps with plaquette and
     // acceptance at 24^4 94.5 us a sweep, 91.3 us this way; FP32 61.2 and 58.1.)
     if (KIND == SU2G_HEATBATH && acc_part) {
-        // the sum of 1 / trials: nearly every lane needed one
-        double a = (double)__popc(__ballot_sync(0xffffffffu, trials == 1u));
-        for (unsigned more = __ballot_sync(0xffffffffu, trials > 1u); more; more &= more - 1u)
-            a += 1.0 / (double)__shfl_sync(0xffffffffu, trials, __ffs(more) - 1);
+        const double a = warp_acceptance(trials);
         if ((threadIdx.x & 31) == 0) acc_part[warp] = DD{acc_warp + a, 0.0};
     }
     if (PLQ) {

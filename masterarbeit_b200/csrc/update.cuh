@@ -186,6 +186,15 @@ __device__ __forceinline__ void kp_pin(KpTrial<R> (&t)[N], KpAngles<R>& a)
     kp_pin(a.cph);
 }
 
+// A warp's sum of 1 / trials (0: no draw, counted as 0): nearly every lane needed one.
+__device__ __forceinline__ double warp_acceptance(uint32_t trials)
+{
+    double a = (double)__popc(__ballot_sync(0xffffffffu, trials == 1u));
+    for (unsigned more = __ballot_sync(0xffffffffu, trials > 1u); more; more &= more - 1u)
+        a += 1.0 / (double)__shfl_sync(0xffffffffu, trials, __ffs(more) - 1);
+    return a;
+}
+
 // X (s A)^dag and |A|^2.  FP64 spells the multiply-adds out, for the reason given at kp_delta: which product of a sum
 // the compiler starts from depends on the code around it.
 __device__ __forceinline__ Q<float> kp_link(const Q<float>& X, const Q<float>& A, float s) { return q_mul_nd(X, q_scale(A, s)); }
