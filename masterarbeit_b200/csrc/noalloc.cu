@@ -100,7 +100,8 @@ struct AtSite {
 
 // One Jacobi step from `in` into `out`: the links of the smeared directions become Proj(U + alpha S)
 // with the staples of smearing.c:42-71; with COPY the other directions are copied.  One site per thread, parities paired per warp as in the handle's kernel,
-// whose staple sums these are, and launched like it: a step starts in the tail of the one before.
+// whose staple sums these are, but for the rounding of each staple by itself (ape_staples), and launched like it: a step starts
+// in the tail of the one before.
 template <int MODE, bool COPY, typename In, typename Out>
 __global__ void __launch_bounds__(128, MODE == SU2G_APE_ALL ? 3 : (MODE == SU2G_APE_SPATIAL ? 4 : 8)) k_ape_any(In in, Out out, Geom g, double alpha)
 {
@@ -115,7 +116,7 @@ __global__ void __launch_bounds__(128, MODE == SU2G_APE_ALL ? 3 : (MODE == SU2G_
 #pragma unroll
     for (int mu = 0; mu < 4; ++mu)
         if (COPY && !ape_updates(MODE, mu)) res[mu] = in.ld(mu, par, s.n);
-    ape_staples<double, MODE>(at, g, s, par, h, [&](int mu, const Q<double>& u, const Q<double>& S) {
+    ape_staples<double, MODE, true, false>(at, g, s, par, h, [&](int mu, const Q<double>& u, const Q<double>& S) {
         res[mu] = q_project(q_axpy(alpha, S, u));
     });
 #pragma unroll
@@ -204,7 +205,7 @@ extern "C" int su2g_ape_inplace_noalloc(double* links, const int32_t dims[4], in
     // whose loads are contiguous over a warp (the site-major one touches a line per lane), and only in
     // the directions the mode changes: the others stay where the first step copied them, in the
     // scratch -- or, for a last step that reads the field and writes over the scratch, where the second
-    // step copied them again.  Twenty spatial steps at 20x16x18x14 on B200: 135 us (173 us without overlapping launches), against 819 us
+    // step copied them again.  Twenty spatial steps at 20x16x18x14 on B200: 136 us (173 us without overlapping launches), against 819 us
     // with every level site-major, one direction after another and no shared products.  A field that is
     // not 32-byte aligned keeps its own layout throughout.
     const bool a32 = ((uintptr_t)links & 31u) == 0;
