@@ -31,18 +31,18 @@ namespace {
 
 // ----------------------------------------------------------- dQ / dU_N ---
 
-// r + a b for a pure quaternion a (a.c0 is not read), and for a pure b.
+// a b for a pure quaternion a (a.c0 is not read), and for a pure b.
 template <typename R>
-__device__ __forceinline__ Q<R> q_pure_mul_add(const Q<R>& r, const Q<R>& a, const Q<R>& b)
+__device__ __forceinline__ Q<R> q_pure_mul(const Q<R>& a, const Q<R>& b)
 {
-    return q_make<R>(r.c0 - a.c1 * b.c1 - a.c2 * b.c2 - a.c3 * b.c3, r.c1 + a.c1 * b.c0 - a.c2 * b.c3 + a.c3 * b.c2,
-                     r.c2 + a.c1 * b.c3 + a.c2 * b.c0 - a.c3 * b.c1, r.c3 - a.c1 * b.c2 + a.c2 * b.c1 + a.c3 * b.c0);
+    return q_make<R>(-a.c1 * b.c1 - a.c2 * b.c2 - a.c3 * b.c3, a.c1 * b.c0 - a.c2 * b.c3 + a.c3 * b.c2,
+                     a.c1 * b.c3 + a.c2 * b.c0 - a.c3 * b.c1, -a.c1 * b.c2 + a.c2 * b.c1 + a.c3 * b.c0);
 }
 template <typename R>
-__device__ __forceinline__ Q<R> q_mul_pure_add(const Q<R>& r, const Q<R>& a, const Q<R>& b)
+__device__ __forceinline__ Q<R> q_mul_pure(const Q<R>& a, const Q<R>& b)
 {
-    return q_make<R>(r.c0 - a.c1 * b.c1 - a.c2 * b.c2 - a.c3 * b.c3, r.c1 + a.c0 * b.c1 - a.c2 * b.c3 + a.c3 * b.c2,
-                     r.c2 + a.c0 * b.c2 + a.c1 * b.c3 - a.c3 * b.c1, r.c3 + a.c0 * b.c3 - a.c1 * b.c2 + a.c2 * b.c1);
+    return q_make<R>(-a.c1 * b.c1 - a.c2 * b.c2 - a.c3 * b.c3, a.c0 * b.c1 - a.c2 * b.c3 + a.c3 * b.c2,
+                     a.c0 * b.c2 + a.c1 * b.c3 - a.c3 * b.c1, a.c0 * b.c3 - a.c1 * b.c2 + a.c2 * b.c1);
 }
 
 // The plane of directions (d, v) among clover_plane's six, and whether d is its first direction.
@@ -58,9 +58,14 @@ __host__ __device__ constexpr bool plane_first(int d, int v) { return clover_pla
 // the e x e loop above it in each plane (D, v) and of the one below, and each loop enters F at its four
 // corners.  With F-bar = dQ/dF (pure) and the path x -> x+v -> x+v+D -> x+D of lines B, A, B' (each e
 // links) around the loop above, those four terms are the path with F-bar inserted at each corner:
-//   F(x) M + M F(x+D) + B [F(x+v) A + A F(x+v+D)] B'^dag,  M = B A B'^dag;
+//   F(x) M + M F(x+D) + [B F(x+v)] [A B'^dag] + [B A] [F(x+v+D) B'^dag],  M = B A B'^dag;
 // the loop below runs the other way round and enters with the opposite sign, as does every loop of a
-// plane whose first direction is v.
+// plane whose first direction is v.  The charge's gradient after n smearing steps is what little of these terms varies slowly
+// over the lattice, so that their rounding decides its accuracy.  Each term is therefore rounded at its own size and loops above
+// and below are subtracted term by term: rms against 80-bit
+// arithmetic after ten steps at 8x6x8x10 1.80e-14, where B [F(x+v) A + A F(x+v+D)] B'^dag with sums folded into multiply-adds has
+// 2.11e-14 and a walk over every leaf 1.77e-14 (without smearing 4.2e-16, 4.3e-16 and 6.2e-16), for one product more a loop: a VJP
+// of ten FP64 steps at 16x12x16x20 on B200 654 -> 664 us.
 template <typename R, int D>
 __device__ __forceinline__ Q<R> line_gradient(const FieldCA<R>& L, const R* fbar, const Geom& g,
                                               const Site& s, int par, int h, int e)
@@ -77,16 +82,12 @@ __device__ __forceinline__ Q<R> line_gradient(const FieldCA<R>& L, const R* fbar
         const int p = plane_of(D, v);
         const int up = s.n + shift_by(g, v, s.c[v], e), dn = s.n + shift_by(g, v, s.c[v], -e);
         const Q<R> A = L.ld(D, q1, up), B = L.ldh(v, par, h), B2 = L.ld(v, q1, s.n + upD);
-        Q<R> m = q_pure_mul_add(q_zero<R>(), F(p, q1, up), A);
-        m = q_mul_pure_add(m, A, F(p, par, up + upD));
-        Q<R> M = q_mul_nd(q_mul(B, A), B2), N = q_mul_nd(q_mul(B, m), B2);
-        const Q<R> a = L.ld(D, q1, dn), b = L.ld(v, q1, dn), b2 = L.ld(v, par, dn + upD);
-        m = q_pure_mul_add(q_zero<R>(), F(p, q1, dn), a);
-        m = q_mul_pure_add(m, a, F(p, par, dn + upD));
-        M = q_sub(M, q_mul(q_mul_dn(b, a), b2));
-        N = q_sub(N, q_mul(q_mul_dn(b, m), b2));
-        N = q_pure_mul_add(N, F(p, par, s.n), M);
-        N = q_mul_pure_add(N, M, F(p, q1, s.n + upD));
+        const Q<R> a = L.ld(D, q1, dn), b = q_dag(L.ld(v, q1, dn)), b2 = L.ld(v, par, dn + upD);
+        const Q<R> BA = q_mul(B, A), ba = q_mul(b, a);
+        const Q<R> M = q_sub(q_mul_nd(BA, B2), q_mul(ba, b2));
+        Q<R> N = q_sub(q_mul(q_mul_pure(B, F(p, q1, up)), q_mul_nd(A, B2)), q_mul(q_mul_pure(b, F(p, q1, dn)), q_mul(a, b2)));
+        N = q_add(N, q_sub(q_mul(BA, q_pure_mul(F(p, par, up + upD), q_dag(B2))), q_mul(ba, q_pure_mul(F(p, par, dn + upD), b2))));
+        N = q_add(N, q_add(q_pure_mul(F(p, par, s.n), M), q_mul_pure(M, F(p, q1, s.n + upD))));
         acc = plane_first(D, v) ? q_add(acc, N) : q_sub(acc, N);
     }
     return acc;
@@ -96,7 +97,7 @@ __device__ __forceinline__ Q<R> line_gradient(const FieldCA<R>& L, const R* fbar
 // b mod 12 of site block b / 12 (parities paired per warp), so that the twelve share their loads in L2.
 // A gather: every result is written once, no atomics, and the sums run in a fixed order.  It replaced a
 // walk over every leaf that added each link's term with an atomic (1728 products and 576 atomics a site;
-// here 36 line gradients of about 15 products and 36 loads each): a whole VJP of five steps without the
+// here 36 line gradients of about 17 products and 36 loads each): a whole VJP of five steps without the
 // gradient's copy at 24^4 on B200 1580 -> 825 us (FP32) and 5290 -> 1510 us (FP64), at 8^4 605 -> 200 us
 // (FP64).  Asking for two to six CTAs per SM changed a VJP of ten steps by less than 3 % from 8^4 to 32^4 (32^4: FP64 7.80
 // ms as it is, 7.78, 7.64, 7.61, 7.61 with two, three, four, six; FP32 4.29, 4.29, 4.28, 4.29, 4.14), so the compiler's own

@@ -1,5 +1,5 @@
 """FP64 results are no less accurate than the same operations in plain 64-bit numpy, both against 80-bit arithmetic:
-in-place smearing."""
+in-place smearing, and the gradient of the charge, whose terms cancel the more the field was smeared."""
 import ctypes
 
 import numpy as np
@@ -7,7 +7,7 @@ import pytest
 
 import _oracle as O
 import _reverse as X
-from masterarbeit_b200 import su2g
+from masterarbeit_b200 import Lattice, su2g
 from test_zz_no_alloc import DeviceBuffer
 
 pytestmark = pytest.mark.gpu
@@ -57,3 +57,14 @@ def test_in_place_smearing(mode):
     # 61 thousand numbers: two such rms differ by a percent by chance; the projection takes the reciprocal of a root instead
     # of a division (one rounding more of some fifteen)
     assert _rms(got, exact) <= 1.08 * plain, plain
+
+
+@pytest.mark.parametrize("seed", [1, 2, 3])
+@pytest.mark.parametrize("n_ape", [0, 1, 10])
+def test_gradient_of_the_charge(n_ape, seed):
+    U = _field(seed)
+    exact = X.charge_gradient(U, DIMS, n_ape, 0.5, np.longdouble)
+    plain = _rms(X.charge_gradient(U, DIMS, n_ape, 0.5, np.float64), exact)
+    L = Lattice(DIMS, precision="fp64", start="cold")
+    L.upload(U)
+    assert _rms(L.ape_qtop_vjp(n_ape, 0.5)[1], exact) <= plain, plain
