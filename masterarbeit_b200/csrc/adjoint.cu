@@ -99,13 +99,14 @@ __device__ __forceinline__ Q<R> line_gradient(const FieldCA<R>& L, const R* fbar
 // walk over every leaf that added each link's term with an atomic (1728 products and 576 atomics a site;
 // here 36 line gradients of about 17 products and 36 loads each): a whole VJP of five steps without the
 // gradient's copy at 24^4 on B200 1580 -> 825 us (FP32) and 5290 -> 1510 us (FP64), at 8^4 605 -> 200 us
-// (FP64).  Asking for two to six CTAs per SM changed a VJP of ten steps by less than 3 % from 8^4 to 32^4 (32^4: FP64 7.80
-// ms as it is, 7.78, 7.64, 7.61, 7.61 with two, three, four, six; FP32 4.29, 4.29, 4.28, 4.29, 4.14), so the compiler's own
-// register count (86 in FP64) stands.  FP64 at 32^4: 54 % of the FP64 pipe, L1 and L2 at 52 and 54 %.
+// (FP64).  Four CTAs per SM (FP64) and six (FP32): a VJP of ten steps, us, unbounded (104 registers in FP64) and with 3, 4, 5, 6:
+// FP64 16x12x16x20 571, 561, 560, 561, 562; 24^4 2446, 2423, 2396, 2415, 2415; 32^4 7658, 7585, 7462, 7475, 7512; FP32 402, 404, 401, 392,
+// 389; 1318, 1316, 1319, 1283, 1268; 4111, 4109, 4110, 3995, 3945; 8^4 all within 2 %.  FP64 at 32^4: 54 % of the FP64 pipe, L1 and
+// L2 at 42 %; FP32: 64 % of the issue slots, waiting for instructions most.
 constexpr int kLineBlock = 128;
 
 template <typename R>
-__global__ void __launch_bounds__(kLineBlock) k_line_gradient(Field<R> U, Field<R> L2, Field<R> L3, Field<R> T1, Field<R> T2,
+__global__ void __launch_bounds__(kLineBlock, sizeof(R) == 4 ? 6 : 4) k_line_gradient(Field<R> U, Field<R> L2, Field<R> L3, Field<R> T1, Field<R> T2,
                                                               Field<R> T3, Geom g, const R* fbar)
 {
     pdl_trigger();
