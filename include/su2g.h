@@ -104,8 +104,8 @@ int su2g_sweep(su2g_lattice *h, int32_t n_sweeps, int32_t n_hb, int32_t n_or, do
  * (mu, nu < mu), covers all 6V plaquettes of the final field once (each holds one odd-site link of
  * its higher direction, and the plaquette's other links are final by then).  *plaq equals
  * su2g_plaquette of the resulting field to rounding (the terms are summed in another order).  The
- * field and the acceptance equal su2g_sweep's to rounding: the fused passes are separately compiled
- * kernels whose multiply-adds may round differently in the last bit.  Synchronises.  With no
+ * field equals su2g_sweep's, in FP64 to the bit (in FP32 the fused passes' multiply-adds are the compiler's, who may
+ * round the last bit differently).  Synchronises.  With no
  * sub-sweep, *plaq is su2g_plaquette. */
 int su2g_sweep_plaquette(su2g_lattice *h, int32_t n_sweeps, int32_t n_hb, int32_t n_or, double *plaq,
                          double *acc_out);

@@ -56,6 +56,17 @@ def test_each_call_equals_its_steps(dims, precision):
     check(B, 12)
 
 
+def test_a_field_beyond_the_limit_of_replays():
+    dims = (32, 32, 32, 34)           # 71 MB of FP32 links, replays up to 64
+    U = O.start(dims, "haar", 3)
+    L, step = Lattice(dims, precision="fp32"), Lattice(dims, precision="fp32")
+    L.upload(U)
+    qs, ws = _steps(step, U, **A)
+    for _ in range(14):
+        q, w = L.measure(**A)
+        assert np.array_equal(q, qs) and np.array_equal(w, ws)
+
+
 def test_the_second_call_is_as_fast_as_the_later_ones():
     spec = dict(q_ape=[12, 24], alpha_q=0.5, R=[1, 2, 3], T=[1, 2, 3], ns_s=50, alpha_s=0.5)
     ratios = []
