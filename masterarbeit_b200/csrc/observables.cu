@@ -80,7 +80,8 @@ constexpr int ape_min_blocks()
 // tail of this one frees (ten steps, us, 24x14x18x22: FP64 all 166 -> 141, spatial 105 -> 84; FP32 24^4 all 185 -> 162,
 // spatial 116 -> 94; FP32 all at 40x30x36x34 658 -> 637, 48^4 within 2 %).  Its links are stored together at the
 // end: with plain loads, a store between them keeps the later ones behind it (FP32 all at 24^4 190 -> 169 us).
-// A step is bound by latency between the L1's and the issue slots' limits (FP32 spatial: 55-67 % and 68 %); tiles
+// A step is bound by latency between the limits of L1, issue slots and FMA (FP32: 58, 67 and 58 % for all links, 58, 68 and 55 %
+// spatial; FP64: L1 63 and 61 %, FP64 pipe 51 and 46 %); tiles
 // of two, four or eight x planes a CTA, for more hits in L1, were 2 to 30 % slower.
 //
 // WIDE: launched in order, read-only loads, links stored as they come, the order by links in four CTAs per SM.  It is
@@ -508,8 +509,8 @@ __device__ __forceinline__ double qtop_product(const FieldCA<R>& U, const FieldC
 }
 
 // One site per thread, parities paired per warp (site_warp_pair); CTA partials of q and |q| at
-// partials[b] and partials[gridDim.x + b].  FMA-bound: 2736 multiply-adds a site, 0.39 ms (FP32) and
-// 1.53 ms (FP64) at 48^4 on B200.  128-thread CTAs, five per SM in FP32 (96 registers) and three in FP64
+// partials[b] and partials[gridDim.x + b].  2736 multiply-adds a site, 0.39 ms (FP32) and 1.53 ms
+// (FP64) at 48^4 on B200; it takes 0.99 and 1.80: issue 70 % (FP32), L1 60, L2 56 and FP64 pipe 47 % (FP64).  128-thread CTAs, five per SM in FP32 (96 registers) and three in FP64
 // (168).  Measured, a whole Q at 24^4 / 48^4 with k_lines: FP32 104 us / 1.19 ms (six CTAs 105 / 1.24,
 // seven 114 / 1.26, three of 256 threads 109 / 1.26; the twelve-product form with offsets per plane
 // 118 / 1.40), FP64 167 us / 2.2-2.4 ms (four CTAs 169 / 2.4, five 183 / 2.7).  Slower: all six planes in one
